@@ -179,6 +179,9 @@ struct nmlmc_ctx {
     std::vector<GraphSlot> graphs;    // executable graphs of recent submissions, by topology
     uint64_t graph_clock = 0;
     uint64_t graph_instantiations = 0, graph_updates = 0, graph_launches = 0;
+    // device block of nmlmc_path_adjoint calls
+    unsigned char* adj_mem = nullptr;
+    size_t adj_bytes = 0;
     // trace
     nmlmc_trace_rec* trace_host = nullptr;
     uint64_t trace_cap = 0;
@@ -1049,6 +1052,7 @@ int nmlmc_destroy(nmlmc_ctx* c) {
     free_dev_portfolio(c->dpf64);
     dfree(c->d_states); dfree(c->d_part_sums); dfree(c->d_part_stats);
     dfree(c->d_out_sums); dfree(c->d_out_stats); dfree(c->d_trace);
+    dfree(c->adj_mem);
     free_outer(c);
     for (cudaEvent_t e : c->pev) cudaEventDestroy(e);
     dfree(c->d_stamps);
@@ -1215,22 +1219,31 @@ int nmlmc_set_portfolio_methods(nmlmc_ctx* c, const nmlmc_portfolio* p, const nm
 
 namespace {
 
-struct DevAlloc {                       // device buffers of one nmlmc_path_adjoint call
-    std::vector<void*> ptrs;
-    ~DevAlloc() { for (void* p : ptrs) cudaFree(p); }
-    template <class T>
-    T* get(size_t n) {
-        void* p = nullptr;
-        if (dev_malloc(&p, (n ? n : 1) * sizeof(T)) != cudaSuccess) return nullptr;
-        ptrs.push_back(p);
-        return static_cast<T*>(p);
+// Device memory of nmlmc_path_adjoint calls: one block per context, kept between calls up to
+// kAdjKeepBytes (allocating and freeing two dozen buffers took 2 ms of each call) and released
+// with the context.  The derivatives kept between the two passes take at most kAdjStoreBytes of it.
+constexpr size_t kAdjKeepBytes = 5ull << 28, kAdjStoreBytes = 1ull << 30;
+
+int adj_reserve(nmlmc_ctx* c, size_t bytes) {
+    if (c->adj_bytes >= bytes) return NMLMC_OK;
+    dfree(c->adj_mem);
+    c->adj_bytes = 0;
+    if (dev_malloc(&c->adj_mem, bytes) != cudaSuccess) {
+        cudaGetLastError();
+        c->adj_mem = nullptr;
+        return NMLMC_ERR_NOMEM;
     }
-    template <class T>
-    T* put(const std::vector<T>& h) {
-        T* d = get<T>(h.size());
-        if (d && !h.empty() && cudaMemcpy(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice) != cudaSuccess)
-            return nullptr;
-        return d;
+    c->adj_bytes = bytes;
+    return NMLMC_OK;
+}
+
+// Offsets of buffers laid end to end on 256-byte boundaries.
+struct Layout {
+    size_t size = 0;
+    size_t add(size_t bytes) {
+        const size_t at = size;
+        size += (bytes + 255) & ~(size_t)255;
+        return at;
     }
 };
 
@@ -1240,67 +1253,87 @@ int path_adjoint_t(nmlmc_ctx* c, const nmlmc_portfolio_batch* b, const nmlmc_adj
                    double* loss, double* seconds) {
     const uint32_t n = b->n, NS = b->stock_off[n], NO = b->option_off[n];
     const bool grad = gwE || gwP || gsE || gsP;
-    DevAlloc D;
     AdjLaunch<RT> A{};
-    A.n = n; A.ell = a->ell; A.pairs = a->inner_pairs; A.M = a->M; A.seed = a->seed;
+    A.n = n; A.n_options = NO; A.ell = a->ell; A.pairs = a->inner_pairs; A.M = a->M; A.seed = a->seed;
     A.milstein = a->milstein ? 1 : 0;
-    A.tile = 0;
     A.r = (RT)b->r; A.rho = (RT)b->rho; A.tau = (RT)b->tau;
     A.s1_rho2 = (RT)sqrt(1 - b->rho * b->rho); A.stau = (RT)sqrt(b->tau); A.disc_tau = (RT)exp(-b->r * b->tau);
-    std::vector<uint32_t> so(b->stock_off, b->stock_off + n + 1), oo(b->option_off, b->option_off + n + 1);
-    std::vector<uint32_t> co(n + 1, 0);
-    uint32_t qmax = 0;
+    // the small per-portfolio and per-stock arrays travel as one copy
+    Layout in;
+    const size_t so = in.add((n + 1) * 4ull), oo = in.add((n + 1) * 4ull), co = in.add((n + 1) * 4ull),
+                 kk = in.add(n * 8ull), dl = in.add(n * 8ull), s0 = in.add(NS * 8ull), mu = in.add(NS * 8ull),
+                 sg = in.add(NS * 8ull);
+    std::vector<unsigned char> small(in.size);
+    memcpy(small.data() + so, b->stock_off, (n + 1) * 4ull);
+    memcpy(small.data() + oo, b->option_off, (n + 1) * 4ull);
+    memcpy(small.data() + kk, b->K, n * 8ull);
+    memcpy(small.data() + s0, b->S0, NS * 8ull);
+    memcpy(small.data() + mu, b->mu, NS * 8ull);
+    memcpy(small.data() + sg, b->sigma, NS * 8ull);
+    uint32_t* chunks = reinterpret_cast<uint32_t*>(small.data() + co);
+    double* delta = reinterpret_cast<double*>(small.data() + dl);
+    chunks[0] = 0;
     for (uint32_t p = 0; p < n; p++) {
-        co[p + 1] = co[p] + (oo[p + 1] - oo[p] + 127) / 128;
-        qmax = std::max(qmax, so[p + 1] - so[p]);
+        chunks[p + 1] = chunks[p] + (b->option_off[p + 1] - b->option_off[p] + 127) / 128;
+        A.q_max = std::max(A.q_max, b->stock_off[p + 1] - b->stock_off[p]);
+        delta[p] = b->K[p] != 0 ? a->delta_rel * fabs(b->K[p]) : a->delta_rel;
     }
-    A.n_chunks = co[n];
-    A.q_max = qmax;
-    // outer samples per CTA: at most kAdjMaxTile, and small enough for about 32 CTAs of four
-    // warps per SM (two waves at full occupancy) when the option chunks alone are too few
-    {
-        const uint64_t want = 148ull * 32;
-        const uint64_t rows = (want + A.n_chunks - 1) / A.n_chunks;
-        const uint64_t t = (a->M + rows - 1) / rows;
-        A.tile = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>({kAdjMaxTile, a->M, t}));
+    A.n_chunks = chunks[n];
+    // one device block: inputs as given, the kernels' arrays, results (zeroed), kept derivatives
+    Layout lay;
+    const size_t dsm = lay.add(in.size), dK = lay.add(NO * 8ull), dT = lay.add(NO * 8ull), dw = lay.add(NO * 8ull),
+                 dty = lay.add(NO * 4ull), dsi = lay.add(NO * 4ull);
+    const size_t rS0 = lay.add(NS * sizeof(RT)), rmu = lay.add(NS * sizeof(RT)), rsg = lay.add(NS * sizeof(RT)),
+                 rK = lay.add(NO * sizeof(RT)), rT = lay.add(NO * sizeof(RT)), rw = lay.add(NO * sizeof(RT)),
+                 rV0 = lay.add(NO * sizeof(RT)), rvg = lay.add(NO * sizeof(RT)), rty = lay.add(NO);
+    const size_t oR = lay.add((size_t)NS * a->M * sizeof(RT)), odR = lay.add((size_t)NS * a->M * sizeof(RT)),
+                 oom = lay.add((size_t)n * a->M * 8), oest = lay.add(3ull * n * 8), owE = lay.add(n * 8ull);
+    const size_t zero = lay.size;
+    const size_t oL = lay.add((size_t)n * a->M * 8), ogwE = lay.add(NO * 8ull), ogwP = lay.add(NO * 8ull),
+                 ogsE = lay.add(NS * 8ull), ogsP = lay.add(NS * 8ull);
+    const size_t zeroed = lay.size - zero;
+    const size_t per_m = (size_t)NO * 2 * sizeof(RT);
+    A.m_store = grad ? std::min<uint64_t>(a->M, kAdjStoreBytes / per_m) : 0;
+    const size_t fixed = lay.size;
+    int rc = adj_reserve(c, fixed + A.m_store * per_m);
+    if (rc && A.m_store) {                       // no room for the kept derivatives: recompute all of them
+        A.m_store = 0;
+        rc = adj_reserve(c, fixed);
     }
-    std::vector<RT> S0(NS), mu(NS), sg(NS), K(NO), T(NO), w(NO), V0(NO), vega(NO);
-    std::vector<int8_t> ty(NO);
-    std::vector<uint32_t> si(b->stock_ind, b->stock_ind + NO);
-    for (uint32_t j = 0; j < NS; j++) { S0[j] = (RT)b->S0[j]; mu[j] = (RT)b->mu[j]; sg[j] = (RT)b->sigma[j]; }
-    for (uint32_t p = 0; p < n; p++)
-        for (uint32_t i = oo[p]; i < oo[p + 1]; i++) {
-            const uint32_t s = so[p] + si[i];
-            const double Sd = b->S0[s], sd = b->sigma[s], Kd = b->strike[i], Td = b->maturity[i];
-            K[i] = (RT)Kd; T[i] = (RT)Td; w[i] = (RT)b->w[i]; ty[i] = (int8_t)b->type[i];
-            V0[i] = (RT)h_calc_bs<double>(b->type[i], Sd, Kd, b->r, Td, sd);
-            const double d1 = h_d1<double>(Sd, Kd, b->r, Td, sd);
-            vega[i] = (RT)(Sd * exp(-0.5 * d1 * d1) * 0.39894228040143268 * sqrt(Td));   // S0 phi(d1) sqrt(T)
-        }
-    std::vector<double> Kp(n), dl(n);
-    for (uint32_t p = 0; p < n; p++) {
-        Kp[p] = b->K[p];
-        dl[p] = b->K[p] != 0 ? a->delta_rel * fabs(b->K[p]) : a->delta_rel;
-    }
-    A.stock_off = D.put(so); A.option_off = D.put(oo); A.chunk_off = D.put(co);
-    A.S0 = D.put(S0); A.mu = D.put(mu); A.sigma = D.put(sg);
-    A.strike = D.put(K); A.maturity = D.put(T); A.w = D.put(w); A.V0 = D.put(V0); A.vega = D.put(vega);
-    A.stock_ind = D.put(si); A.type = D.put(ty); A.K = D.put(Kp); A.delta = D.put(dl);
-    A.R = D.get<RT>((size_t)NS * a->M); A.dR = D.get<RT>((size_t)NS * a->M);
-    A.L = D.get<double>((size_t)n * a->M); A.omega = D.get<double>((size_t)n * a->M);
-    A.est = D.get<double>(3 * n); A.wE = D.get<double>(n);
-    A.gw_E = D.get<double>(NO); A.gw_P = D.get<double>(NO); A.gs_E = D.get<double>(NS); A.gs_P = D.get<double>(NS);
-    if (!A.stock_off || !A.option_off || !A.chunk_off || !A.S0 || !A.mu || !A.sigma || !A.strike || !A.maturity ||
-        !A.w || !A.V0 || !A.vega || !A.stock_ind || !A.type || !A.K || !A.delta || !A.R || !A.dR || !A.L ||
-        !A.omega || !A.est || !A.wE || !A.gw_E || !A.gw_P || !A.gs_E || !A.gs_P)
-        return set_err(NMLMC_ERR_NOMEM);
-    NM_CUDA(cudaMemsetAsync(A.L, 0, (size_t)n * a->M * sizeof(double), c->stream), "memset");
-    NM_CUDA(cudaMemsetAsync(A.gw_E, 0, NO * sizeof(double), c->stream), "memset");
-    NM_CUDA(cudaMemsetAsync(A.gw_P, 0, NO * sizeof(double), c->stream), "memset");
-    NM_CUDA(cudaMemsetAsync(A.gs_E, 0, NS * sizeof(double), c->stream), "memset");
-    NM_CUDA(cudaMemsetAsync(A.gs_P, 0, NS * sizeof(double), c->stream), "memset");
+    if (rc) return set_err(rc);
+    struct Trim {                                // a block above the limit goes back when the call ends
+        nmlmc_ctx* c;
+        ~Trim() { if (c->adj_bytes > kAdjKeepBytes) { dfree(c->adj_mem); c->adj_bytes = 0; } }
+    } trim{c};
+    unsigned char* base = c->adj_mem;
+    AdjInputs I;
+    I.S0 = reinterpret_cast<double*>(base + dsm + s0); I.mu = reinterpret_cast<double*>(base + dsm + mu);
+    I.sigma = reinterpret_cast<double*>(base + dsm + sg);
+    I.strike = reinterpret_cast<double*>(base + dK); I.maturity = reinterpret_cast<double*>(base + dT);
+    I.w = reinterpret_cast<double*>(base + dw); I.type = reinterpret_cast<int32_t*>(base + dty);
+    I.r = b->r;
+    A.stock_off = reinterpret_cast<uint32_t*>(base + dsm + so); A.option_off = reinterpret_cast<uint32_t*>(base + dsm + oo);
+    A.chunk_off = reinterpret_cast<uint32_t*>(base + dsm + co);
+    A.K = reinterpret_cast<double*>(base + dsm + kk); A.delta = reinterpret_cast<double*>(base + dsm + dl);
+    A.stock_ind = reinterpret_cast<uint32_t*>(base + dsi);
+    auto rt = [&](size_t at) { return reinterpret_cast<RT*>(base + at); };
+    auto db = [&](size_t at) { return reinterpret_cast<double*>(base + at); };
+    A.S0 = rt(rS0); A.mu = rt(rmu); A.sigma = rt(rsg);
+    A.strike = rt(rK); A.maturity = rt(rT); A.w = rt(rw); A.V0 = rt(rV0); A.vega = rt(rvg);
+    A.type = reinterpret_cast<int8_t*>(base + rty);
+    A.R = rt(oR); A.dR = rt(odR);
+    A.L = db(oL); A.omega = db(oom); A.est = db(oest); A.wE = db(owE);
+    A.gw_E = db(ogwE); A.gw_P = db(ogwP); A.gs_E = db(ogsE); A.gs_P = db(ogsP);
+    A.store = reinterpret_cast<typename Pair2<RT>::type*>(base + fixed);
+    NM_CUDA(cudaMemcpyAsync(base + dsm, small.data(), in.size, cudaMemcpyHostToDevice, c->stream), "h2d");
+    NM_CUDA(cudaMemcpyAsync(base + dK, b->strike, NO * 8ull, cudaMemcpyHostToDevice, c->stream), "h2d");
+    NM_CUDA(cudaMemcpyAsync(base + dT, b->maturity, NO * 8ull, cudaMemcpyHostToDevice, c->stream), "h2d");
+    NM_CUDA(cudaMemcpyAsync(base + dw, b->w, NO * 8ull, cudaMemcpyHostToDevice, c->stream), "h2d");
+    NM_CUDA(cudaMemcpyAsync(base + dty, b->type, NO * 4ull, cudaMemcpyHostToDevice, c->stream), "h2d");
+    NM_CUDA(cudaMemcpyAsync(base + dsi, b->stock_ind, NO * 4ull, cudaMemcpyHostToDevice, c->stream), "h2d");
+    NM_CUDA(cudaMemsetAsync(base + zero, 0, zeroed, c->stream), "memset");
     NM_CUDA(cudaEventRecord(c->ev0, c->stream), "event");
-    NM_CUDA(launch_adjoint(A, grad, c->stream), "adjoint kernels");
+    NM_CUDA(launch_adjoint(A, I, grad, c->stream), "adjoint kernels");
     NM_CUDA(cudaEventRecord(c->ev1, c->stream), "event");
     std::vector<double> est(3 * n);
     NM_CUDA(cudaMemcpyAsync(est.data(), A.est, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "d2h");
