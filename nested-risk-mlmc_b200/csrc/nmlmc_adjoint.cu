@@ -39,8 +39,7 @@ __device__ __forceinline__ uint64_t adj_stream_id(uint32_t ell, uint32_t p, uint
 template <class RT>
 __device__ __forceinline__ void normals4(uint64_t v0, uint64_t v1, RT* z) {
     if constexpr (sizeof(RT) == 4) {
-        boxmuller32_f((uint32_t)v0, (uint32_t)(v0 >> 32), z[0], z[1]);
-        boxmuller32_f((uint32_t)v1, (uint32_t)(v1 >> 32), z[2], z[3]);
+        boxmuller32_f4(v0, v1, z);
     } else {
         boxmuller32_d((uint32_t)v0, (uint32_t)(v0 >> 32), z[0], z[1]);
         boxmuller32_d((uint32_t)v1, (uint32_t)(v1 >> 32), z[2], z[3]);

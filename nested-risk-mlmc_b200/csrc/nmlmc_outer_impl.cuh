@@ -154,6 +154,17 @@ __device__ __forceinline__ void bm_pair(uint32_t u0, uint32_t u1, RT& x, RT& y) 
     }
 }
 
+// The four normals of a block at the context precision.
+template <int PREC, class RT>
+__device__ __forceinline__ void bm_block(uint64_t v0, uint64_t v1, RT* z) {
+    if constexpr (PREC == PREC_FP32) {
+        boxmuller32_f4(v0, v1, z);
+    } else {
+        bm_pair<PREC, RT>((uint32_t)v0, (uint32_t)(v0 >> 32), z[0], z[1]);
+        bm_pair<PREC, RT>((uint32_t)v1, (uint32_t)(v1 >> 32), z[2], z[3]);
+    }
+}
+
 template <int PREC, class RT>
 __device__ __forceinline__ RT u01_word(uint32_t w) {
     if (PREC == PREC_FP64) return (RT)__dadd_rn(__dmul_rn((double)w, 0x1p-32), 0x1p-33);
@@ -761,11 +772,19 @@ __device__ __forceinline__ void eval_chunk_c(const DevLevel<RT>& D, uint32_t ite
             uint64_t v0, v1;
             threefry2x64((s0 >> 2) + b, tag, key, v0, v1);
             RT z[4];
-            bm_pair<PREC, RT>((uint32_t)v0, (uint32_t)(v0 >> 32), z[0], z[1]);
-            bm_pair<PREC, RT>((uint32_t)v1, (uint32_t)(v1 >> 32), z[2], z[3]);
+            if constexpr (PREC == PREC_FP32) {   // d = Y + radius x sine or cosine, rounded once
+                F2 sn, cs, r;
+                boxmuller32_f_polar(v0, v1, sn, cs, r);
+                const F2 Y2 = f2(Y, Y);
+                sn = f2_fma(sn, r, Y2);
+                cs = f2_fma(cs, r, Y2);
+                z[0] = f2_lo(sn); z[1] = f2_lo(cs); z[2] = f2_hi(sn); z[3] = f2_hi(cs);
+            } else {
+                bm_block<PREC, RT>(v0, v1, z);
+            }
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                RT d = (PREC == PREC_FP32) ? (RT)(Y + z[q]) : xadd(Y, z[q]);
+                RT d = (PREC == PREC_FP32) ? z[q] : xadd(Y, z[q]);
                 if (PREC == PREC_FP32 && S2) d = (RT)((float)d + shift);
                 z[q] = d;
                 if (S2) { if (PREC == PREC_FP32) a2.add_sq(d); else a2.add(xmul(d, d)); }
@@ -781,13 +800,12 @@ __device__ __forceinline__ void eval_chunk_c(const DevLevel<RT>& D, uint32_t ite
         for (uint32_t b = 0; b < C / 2; b++) {   // one block = two inner samples
             uint64_t v0, v1;
             threefry2x64((s0 >> 1) + b, tag, key, v0, v1);
-            RT X[2], Y2[2];
-            bm_pair<PREC, RT>((uint32_t)v0, (uint32_t)(v0 >> 32), X[0], Y2[0]);
-            bm_pair<PREC, RT>((uint32_t)v1, (uint32_t)(v1 >> 32), X[1], Y2[1]);
+            RT z[4], X[2];
+            bm_block<PREC, RT>(v0, v1, z);
 #pragma unroll
             for (int q = 0; q < 2; q++) {
-                RT a = xadd(xmul(st, Y), xmul(s1t, X[q]));
-                RT c = xadd(xmul(st, Y2[q]), xmul(s1t, X[q]));
+                RT a = xadd(xmul(st, Y), xmul(s1t, z[2 * q]));
+                RT c = xadd(xmul(st, z[2 * q + 1]), xmul(s1t, z[2 * q]));
                 RT d = xsub(xmul(a, a), xmul(c, c));
                 if (PREC == PREC_FP32 && S2) d = (RT)((float)d + shift);
                 X[q] = d;
@@ -1349,8 +1367,7 @@ __global__ void __launch_bounds__(kTile) k_outer(DevLevel<RT> D, uint32_t nb) {
                 uint64_t v0, v1;
                 threefry2x64(b, PH_OUTER, key, v0, v1);
                 RT z[4];
-                bm_pair<PREC, RT>((uint32_t)v0, (uint32_t)(v0 >> 32), z[0], z[1]);
-                bm_pair<PREC, RT>((uint32_t)v1, (uint32_t)(v1 >> 32), z[2], z[3]);
+                bm_block<PREC, RT>(v0, v1, z);
                 for (uint32_t q = 0; q < 4; q++) {
                     const uint32_t k = 4 * b + q;
                     if (k >= nnorm) break;

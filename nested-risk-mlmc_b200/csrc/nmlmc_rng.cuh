@@ -104,6 +104,48 @@ __device__ __forceinline__ void boxmuller32_d(uint32_t u0, uint32_t u1, double& 
     y = __dmul_rn(c, r);
 }
 
+// ---- pairs of floats in one 64-bit register (PTX f32x2, sm_100) ------------------------------
+// One instruction for two independent FP32 operations, each rounded as the scalar one: half the
+// issue slots of the arithmetic around the generator, whose kernels are issue- and ALU-bound.
+struct F2 { unsigned long long v; };
+__device__ __forceinline__ F2 f2(float a, float b) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float f2_lo(F2 a) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+    return x;
+}
+__device__ __forceinline__ float f2_hi(F2 a) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.v));
+    return y;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 f2_add(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+
+// SFU functions without the handling of subnormal operands, which none of the arguments below can
+// be: the same values for normal ones, three or four instructions fewer each.
+__device__ __forceinline__ float sin_sfu(float x) { float r; asm("sin.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+__device__ __forceinline__ float cos_sfu(float x) { float r; asm("cos.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+__device__ __forceinline__ float lg2_sfu(float x) { float r; asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+__device__ __forceinline__ float rsqrt_sfu(float x) { float r; asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+
 // FP32 fast Box-Muller on the SFU: MUFU sin/cos of the angle pi*a (absolute error <= 2^-21.4 on
 // [-pi, pi]; pi*a formed in one FMA from the word), MUFU lg2 for the log and MUFU rsqrt for the
 // root.  Near u = 1 the MUFU log's absolute error (2^-22) would dominate the small radius, so
@@ -116,14 +158,43 @@ __device__ __forceinline__ void boxmuller32_f(uint32_t u0, uint32_t u1, float& x
     const float th = fmaf((float)(int32_t)u0, PI * 0x1p-31f, PI * 0x1p-32f);
     const float u = fmaf((float)u1, 0x1p-32f, 0x1p-33f);
     const float q = fmaf((float)(~u1), 0x1p-32f, 0x1p-33f);
-    float s, c;
-    __sincosf(th, &s, &c);
-    const float t_log = (-2.0f * 0.69314718055994531f) * __log2f(u);
+    const float t_log = (-2.0f * 0.69314718055994531f) * lg2_sfu(u);
     const float t_ser = q * fmaf(q, fmaf(q, 0.66666667f, 1.0f), 2.0f);
     const float t = (q < 0.015625f) ? t_ser : t_log;   // -2 ln u > 0: t_ser >= 2q >= 2^-32, t_log > 0.03
-    const float r = t * rsqrtf(t);
-    x = s * r;
-    y = c * r;
+    const float r = t * rsqrt_sfu(t);
+    x = sin_sfu(th) * r;
+    y = cos_sfu(th) * r;
+}
+
+// Box-Muller of the two word pairs of a block (v0: normals 0 and 1, v1: normals 2 and 3) before the
+// last product: sines s, cosines c and radii r of both pairs, the arithmetic two pairs at a time
+// (13 instructions instead of 22).  Normals (s.lo r.lo, c.lo r.lo, s.hi r.hi, c.hi r.hi), each equal
+// to boxmuller32_f's.
+__device__ __forceinline__ void boxmuller32_f_polar(uint64_t v0, uint64_t v1, F2& s, F2& c, F2& r) {
+    const float PI = 3.14159265358979f;
+    const uint32_t a0 = (uint32_t)v0, a1 = (uint32_t)(v0 >> 32), b0 = (uint32_t)v1, b1 = (uint32_t)(v1 >> 32);
+    const F2 k32 = f2(0x1p-32f, 0x1p-32f), k33 = f2(0x1p-33f, 0x1p-33f);
+    const F2 th = f2_fma(f2((float)(int32_t)a0, (float)(int32_t)b0), f2(PI * 0x1p-31f, PI * 0x1p-31f),
+                         f2(PI * 0x1p-32f, PI * 0x1p-32f));
+    const F2 u = f2_fma(f2((float)a1, (float)b1), k32, k33);
+    const F2 q = f2_fma(f2((float)(~a1), (float)(~b1)), k32, k33);
+    const float kl = -2.0f * 0.69314718055994531f;
+    const F2 t_log = f2_mul(f2(kl, kl), f2(lg2_sfu(f2_lo(u)), lg2_sfu(f2_hi(u))));
+    const F2 t_ser = f2_mul(q, f2_fma(q, f2_fma(q, f2(0.66666667f, 0.66666667f), f2(1.0f, 1.0f)), f2(2.0f, 2.0f)));
+    const float ta = f2_lo(q) < 0.015625f ? f2_lo(t_ser) : f2_lo(t_log);
+    const float tb = f2_hi(q) < 0.015625f ? f2_hi(t_ser) : f2_hi(t_log);
+    r = f2_mul(f2(ta, tb), f2(rsqrt_sfu(ta), rsqrt_sfu(tb)));
+    s = f2(sin_sfu(f2_lo(th)), sin_sfu(f2_hi(th)));
+    c = f2(cos_sfu(f2_lo(th)), cos_sfu(f2_hi(th)));
+}
+
+// The block's four normals.
+__device__ __forceinline__ void boxmuller32_f4(uint64_t v0, uint64_t v1, float* z) {
+    F2 s, c, r;
+    boxmuller32_f_polar(v0, v1, s, c, r);
+    s = f2_mul(s, r);
+    c = f2_mul(c, r);
+    z[0] = f2_lo(s); z[1] = f2_lo(c); z[2] = f2_hi(s); z[3] = f2_hi(c);
 }
 
 // ---- OUTER layout addressing --------------------------------------------------------------
