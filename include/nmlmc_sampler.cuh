@@ -188,8 +188,8 @@ public:
         const bool adapt = adaptive();
         L.adaptive_f = adapt && L.cf.max_count > 2 * L.cf.base_count;
         L.adaptive_c = !L.fine_only && adapt && L.cc.max_count > 2 * L.cc.base_count;
-        cudaError_t e = outer_level_begin(B_, stream_);
-        if (e == cudaSuccess && M) e = sample_level_t<RT, KIND_USER, kPrec, SAMPLER>(L, B_, nullptr, stream_);
+        cudaError_t e = M ? cudaSuccess : outer_level_begin(B_, stream_);
+        if (M) e = sample_level_t<RT, KIND_USER, kPrec, SAMPLER>(L, B_, nullptr, stream_);
         double acc[16];
         if (e == cudaSuccess) e = cudaMemcpyAsync(acc, B_.level_acc, sizeof acc, cudaMemcpyDeviceToHost, stream_);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream_);

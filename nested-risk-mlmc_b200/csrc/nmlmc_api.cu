@@ -175,7 +175,6 @@ struct nmlmc_ctx {
     double* h_pin = nullptr;          // 32 doubles
     // one-submission level rounds (nmlmc_sample_levels on the OUTER layout)
     double* h_lev = nullptr;          // pinned [kMaxSubmit][16] sums, then [kMaxSubmit][2] stamps
-    uint64_t* d_stamps = nullptr;     // device [kMaxSubmit][2] level begin / end (ns)
     std::vector<GraphSlot> graphs;    // executable graphs of recent submissions, by topology
     uint64_t graph_clock = 0;
     uint64_t graph_instantiations = 0, graph_updates = 0, graph_launches = 0;
@@ -767,11 +766,11 @@ cudaError_t time_phase_config(nmlmc_ctx* c, uint32_t ell, uint64_t Mp, const Pha
     L.variant = pc.variant;
     OuterBuffers B = c->ob;
     B.prof_mark = nullptr;
+    B.stamps = nullptr;
     cudaError_t e = cudaSuccess;
     float ms = 0;
     for (int rep = 0; rep < 2 && e == cudaSuccess; rep++) {       // the first run warms up
         e = cudaEventRecord(c->ev0, c->stream);
-        if (e == cudaSuccess) e = outer_level_begin(B, c->stream);
         if (e == cudaSuccess) e = outer_sample_level<RT>(L, c->kind, c->cfg.precision, B, nullptr, c->stream);
         if (e == cudaSuccess) e = cudaEventRecord(c->ev1, c->stream);
         if (e == cudaSuccess) e = cudaEventSynchronize(c->ev1);
@@ -865,24 +864,17 @@ int sample_outer(nmlmc_ctx* c, uint32_t ell, uint64_t Mtotal, nmlmc_level_result
     if (rc) return rc;
     OuterLevel<RT> L = outer_level_params<RT>(c, ell, M, c->next_outer[ell] + lo);
     TraceRec* tr = c->trace_host ? c->d_trace : nullptr;
-    c->ob.prof_mark = c->prof ? prof_mark : nullptr;
-    c->ob.prof_user = c;
+    OuterBuffers B = c->ob;
+    B.prof_mark = c->prof ? prof_mark : nullptr;
+    B.prof_user = c;
+    B.level_acc = c->h_pin;                      // pinned: the level's last kernel stores the sums there
+    memset(c->h_pin, 0, 16 * sizeof(double));
     NM_CUDA(cudaEventRecord(c->ev0, c->stream), "event");
-    NM_CUDA(outer_level_begin(c->ob, c->stream), "level begin");
-    if (M) NM_CUDA(outer_sample_level<RT>(L, c->kind, c->cfg.precision, c->ob, tr, c->stream), "outer level kernels");
+    if (M) NM_CUDA(outer_sample_level<RT>(L, c->kind, c->cfg.precision, B, tr, c->stream), "outer level kernels");
     NM_CUDA(cudaEventRecord(c->ev1, c->stream), "event");
-    NM_CUDA(cudaMemcpyAsync(c->h_pin, c->ob.level_acc, 16 * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "d2h");
     if (tr && M) NM_CUDA(cudaMemcpyAsync(c->trace_host, tr, M * sizeof(TraceRec), cudaMemcpyDeviceToHost, c->stream), "d2h");
-    uint32_t path_limit = 0;
-    const bool paths = c->kind == KIND_PORTFOLIO && c->pf.mixed();
-    if (paths)
-        NM_CUDA(cudaMemcpyAsync(&path_limit, c->ob.counters + kCounterPathLimit, sizeof path_limit,
-                                cudaMemcpyDeviceToHost, c->stream), "d2h");
     NM_CUDA(cudaStreamSynchronize(c->stream), "sync");
-    if (path_limit) {                            // a sample exceeded kMaxPathSteps
-        NM_CUDA(cudaMemset(c->ob.counters + kCounterPathLimit, 0, sizeof path_limit), "memset");
-        return set_err(NMLMC_ERR_LIMIT);
-    }
+    if (c->h_pin[12] != 0) return set_err(NMLMC_ERR_LIMIT);   // a sample exceeded kMaxPathSteps
     if (c->prof) prof_collect(c);
     float ms = 0;
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
@@ -917,6 +909,8 @@ int sample_outer_levels(nmlmc_ctx* c, uint32_t n, const uint32_t* ells, const ui
         int rc = ensure_tuned<RT>(c, ells[i], M);
         if (rc) return rc;
     }
+    uint64_t* h_st = reinterpret_cast<uint64_t*>(c->h_lev + kMaxSubmit * 16);
+    memset(c->h_lev, 0, kMaxSubmit * 18 * sizeof(double));
     NM_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
     cudaError_t err = cudaSuccess;
     for (uint32_t i = 0; i < n && err == cudaSuccess; i++) {
@@ -927,18 +921,11 @@ int sample_outer_levels(nmlmc_ctx* c, uint32_t n, const uint32_t* ells, const ui
         OuterLevel<RT> L = outer_level_params<RT>(c, ell, M, next[ell] + lo);
         next[ell] += Mtot[i];
         OuterBuffers B = c->ob;
-        B.level_acc = c->ob.level_acc + 16 * (size_t)i;
+        B.level_acc = c->h_lev + 16 * (size_t)i;       // pinned: sums and stamps go straight to the host
+        B.stamps = h_st + 2 * i;
         B.prof_mark = nullptr;
-        err = launch_stamp(c->d_stamps + 2 * i, c->stream);
-        if (err == cudaSuccess) err = outer_level_begin(B, c->stream);
-        if (err == cudaSuccess && M) err = outer_sample_level<RT>(L, c->kind, c->cfg.precision, B, nullptr, c->stream);
-        if (err == cudaSuccess) err = launch_stamp(c->d_stamps + 2 * i + 1, c->stream);
+        if (M) err = outer_sample_level<RT>(L, c->kind, c->cfg.precision, B, nullptr, c->stream);
     }
-    uint64_t* h_st = reinterpret_cast<uint64_t*>(c->h_lev + kMaxSubmit * 16);
-    if (err == cudaSuccess)
-        err = cudaMemcpyAsync(c->h_lev, c->ob.level_acc, (size_t)n * 16 * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
-    if (err == cudaSuccess)
-        err = cudaMemcpyAsync(h_st, c->d_stamps, (size_t)n * 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, c->stream);
     cudaGraph_t graph = nullptr;
     cudaError_t e2 = cudaStreamEndCapture(c->stream, &graph);
     if (err == cudaSuccess) err = e2;
@@ -952,6 +939,9 @@ int sample_outer_levels(nmlmc_ctx* c, uint32_t n, const uint32_t* ells, const ui
         key.push_back(ells[i]);
         key.push_back((Ms[i] + c->ob.cap - 1) / c->ob.cap);
     }
+    size_t nodes = 0;                              // small levels are one launch instead of a sequence
+    cudaGraphGetNodes(graph, nullptr, &nodes);
+    key.push_back(nodes);
     GraphSlot* slot = nullptr;
     for (GraphSlot& g : c->graphs)
         if (g.key == key) slot = &g;
@@ -1055,7 +1045,6 @@ int nmlmc_destroy(nmlmc_ctx* c) {
     dfree(c->adj_mem);
     free_outer(c);
     for (cudaEvent_t e : c->pev) cudaEventDestroy(e);
-    dfree(c->d_stamps);
     drop_graphs(c);
     if (c->h_lev) cudaFreeHost(c->h_lev);
     if (c->h_pin) cudaFreeHost(c->h_pin);
@@ -1436,8 +1425,6 @@ int nmlmc_sample_levels(nmlmc_ctx* c, uint32_t n, const uint32_t* ells, const ui
         int rc = ensure_portfolio(c);
         if (rc || (rc = alloc_outer(c, want))) return rc;
         if (!c->h_lev && cudaMallocHost(&c->h_lev, kMaxSubmit * 18 * sizeof(double)) != cudaSuccess)
-            return set_err(NMLMC_ERR_NOMEM);
-        if (!c->d_stamps && dev_malloc(&c->d_stamps, kMaxSubmit * 2 * sizeof(uint64_t)) != cudaSuccess)
             return set_err(NMLMC_ERR_NOMEM);
         for (uint32_t i = 0; i < n; i++) memset(&outs[i], 0, sizeof(outs[i]));
         return k.precision == NMLMC_PREC_FP64 ? sample_outer_levels<double>(c, n, ells, Ms, outs)

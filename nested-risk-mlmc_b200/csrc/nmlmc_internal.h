@@ -66,8 +66,11 @@ struct OuterBuffers {
     uint32_t* class_items;   // cap: items sorted by final class
     uint32_t* counters;      // device counters (see nmlmc_outer.cu)
     double* block_sums;      // per-CTA partial moments [grid][16]
-    double* level_acc;       // accumulated level result [16]
-    int grid;
+    double* level_acc;       // the level's result [16] (device or pinned host memory), written by its last
+                             // kernel: the sums of block_sums, entry 12 the path-limit flag
+    int grid;                // CTA slots of block_sums
+    int slots;               // slots the current level uses (set per level)
+    uint64_t* stamps;        // optional: %globaltimer at the level's begin and end [2] (as level_acc)
     // KIND_USER only (caller-written SAMPLER classes): the SAMPLER object of every outer sample
     // (its outer state, state_bytes each) and its workspace (ws_bytes each)
     void* user_state;
@@ -93,8 +96,8 @@ uint64_t launches_total();
 template <class RT>
 cudaError_t outer_sample_level(const OuterLevel<RT>& L, int kind, int prec, OuterBuffers& B,
                                TraceRec* trace, cudaStream_t stream);
+// Zeroes the level's result: for levels without outer samples, which launch nothing.
 cudaError_t outer_level_begin(OuterBuffers& B, cudaStream_t stream);
-cudaError_t launch_stamp(uint64_t* slot, cudaStream_t stream);   // %globaltimer -> *slot
 
 // Portfolio loss sweep L(Y) over all options (K-quantile precompute).
 template <class RT>

@@ -156,7 +156,7 @@ extern "C" int nmlmc_sample_level_noalloc(int32_t kind, double tau, double max_l
 
     // clear what the kernels accumulate into (the array keeps the previous call's contents)
     cudaError_t e = cudaMemsetAsync(B.counters, 0, 256 * sizeof(uint32_t), st);
-    if (e == cudaSuccess) e = outer_level_begin(B, st);
+    if (e == cudaSuccess && !M) e = outer_level_begin(B, st);
     if (e == cudaSuccess && M) {
         if (precision == NMLMC_PREC_FP32) {
             OuterLevel<float> L{};

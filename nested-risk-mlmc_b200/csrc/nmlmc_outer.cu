@@ -8,29 +8,13 @@
 
 namespace nmlmc {
 
-// Device timestamp (%globaltimer, nanoseconds): marks level boundaries inside a CUDA graph,
-// where event-record nodes carry no elapsed time.
-__global__ void k_stamp(uint64_t* slot) {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    *slot = t;
-}
-
-cudaError_t launch_stamp(uint64_t* slot, cudaStream_t stream) {
-    k_stamp<<<1, 1, 0, stream>>>(slot);
-    count_launch();
-    return cudaGetLastError();
-}
-
 // ---- host orchestration ----------------------------------------------------------------------
 static std::atomic<uint64_t> g_launches{0};
 void count_launch(uint64_t n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 uint64_t launches_total() { return g_launches.load(std::memory_order_relaxed); }
 
 cudaError_t outer_level_begin(OuterBuffers& B, cudaStream_t stream) {
-    cudaError_t e = cudaMemsetAsync(B.level_acc, 0, 16 * sizeof(double), stream);
-    if (e != cudaSuccess) return e;
-    return cudaMemsetAsync(B.block_sums, 0, (size_t)B.grid * 16 * sizeof(double), stream);
+    return cudaMemsetAsync(B.level_acc, 0, 16 * sizeof(double), stream);
 }
 
 // Level sequences instantiated per kind in nmlmc_outer_kind.cu.
@@ -161,13 +145,13 @@ cudaError_t outer_full_loss(const OuterLevel<RT>& L, int prec, OuterBuffers& B, 
         if (og < 1) og = 1;
         if (prec == PREC_FP64) {
             if constexpr (sizeof(RT) == 8) {
-                k_outer<RT, KIND_PORTFOLIO, PREC_FP64><<<og, kTile, 0, stream>>>(D, (uint32_t)nb);
+                k_outer<RT, KIND_PORTFOLIO, PREC_FP64><<<og, kTile, 0, stream>>>(D, (uint32_t)nb, 0);
                 k_full_loss<RT, PREC_FP64><<<B.grid, kTile, 0, stream>>>(D, (uint32_t)nb, d_loss + done);
             }
         } else {
             if constexpr (sizeof(RT) == 4) {
                 if (prec == PREC_FP32 && L.ot.fast) {
-                    k_outer<RT, KIND_PORTFOLIO, PREC_FP32><<<og, kTile, 0, stream>>>(D, (uint32_t)nb);
+                    k_outer<RT, KIND_PORTFOLIO, PREC_FP32><<<og, kTile, 0, stream>>>(D, (uint32_t)nb, 0);
                     const size_t smem = (size_t)2 * kLossTile * L.ot.Q * sizeof(float);
                     if (smem > 200 * 1024) return cudaErrorInvalidValue;   // Q above 800 stocks
                     if (smem > 48 * 1024) {
@@ -178,10 +162,10 @@ cudaError_t outer_full_loss(const OuterLevel<RT>& L, int prec, OuterBuffers& B, 
                     k_full_loss_fast<<<lg, kTile, smem, stream>>>(D, (uint32_t)nb, d_loss + done);
                     count_launch(2);
                 } else if (prec == PREC_FP32) {
-                    k_outer<RT, KIND_PORTFOLIO, PREC_FP32><<<og, kTile, 0, stream>>>(D, (uint32_t)nb);
+                    k_outer<RT, KIND_PORTFOLIO, PREC_FP32><<<og, kTile, 0, stream>>>(D, (uint32_t)nb, 0);
                     k_full_loss<RT, PREC_FP32><<<B.grid, kTile, 0, stream>>>(D, (uint32_t)nb, d_loss + done);
                 } else {
-                    k_outer<RT, KIND_PORTFOLIO, PREC_REF32><<<og, kTile, 0, stream>>>(D, (uint32_t)nb);
+                    k_outer<RT, KIND_PORTFOLIO, PREC_REF32><<<og, kTile, 0, stream>>>(D, (uint32_t)nb, 0);
                     k_full_loss<RT, PREC_REF32><<<B.grid, kTile, 0, stream>>>(D, (uint32_t)nb, d_loss + done);
                 }
             }

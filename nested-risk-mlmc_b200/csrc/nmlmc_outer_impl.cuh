@@ -20,8 +20,8 @@
 //                round's list)
 //   k_classify   bucket outer samples by their final count (a power of two)
 //   k_phase      final: antithetic groups and the big-count mean, phi, 4 moments into per-CTA
-//                partial sums (fixed order, no atomics on the sums)
-//   k_reduce     per-CTA partials -> the level's sums
+//                partial sums (fixed order, no atomics on the sums); the CTA that finishes last adds
+//                the partials to the level's sums
 //
 // Every thread does the same unit of work (one chunk), so the device stays full whatever the
 // spread of inner counts.  An item with more chunks than a CTA has threads is walked tile by
@@ -38,18 +38,22 @@ namespace nmlmc {
 
 constexpr int kTile = 256;           // threads per CTA = chunks per tile
 constexpr int kWarps = kTile / 32;
-constexpr int kMaxSegs = 40;
+constexpr int kMaxRounds = 32;       // pilot rounds of a level (inner counts are below 2^32)
+constexpr int kMaxSegs = 36;         // final classes: counts of 1 .. 2^31 chunks
 
-// device counter slots (uint32 each)
+// Device counter slots (uint32 each).  k_outer, the first kernel of a batch, zeroes [0, CNT_ZEROED):
+// every round has its own list sizes and work queue, so nothing is reset between the launches of
+// a level (a memset node between two kernels costs about as much as a small kernel).
 enum : int {
-    CNT_LIST = 0,        // [4]: fine list size (ping-pong slots 0/1), coarse list size (2/3)
-    CNT_CLASS = 8,       // [64]: outer samples per final class
-    CNT_FILL = 72,       // [64]: scatter fill per class
-    CNT_TOTAL = 144,
-    CNT_QUEUE = 192,     // [kMaxSegs]: tile tickets of the phase kernel's work queue, per segment
-    CNT_ERR = kCounterPathLimit   // set when a path-simulated inner sample exceeds kMaxPathSteps
+    CNT_LIST = 0,                            // [2 kMaxRounds]: list sizes entering round r (2r fine, 2r + 1 coarse)
+    CNT_CLASS = CNT_LIST + 2 * kMaxRounds,   // [kMaxSegs]: outer samples per final class
+    CNT_FILL = CNT_CLASS + kMaxSegs,         // [kMaxSegs]: scatter fill per class
+    CNT_QUEUE = CNT_FILL + kMaxSegs,         // tile tickets: two segments per pilot round, then the final segments
+    CNT_ZEROED = CNT_QUEUE + 2 * kMaxRounds + kMaxSegs,
+    CNT_ERR = kCounterPathLimit,  // set when a path-simulated inner sample exceeds kMaxPathSteps
+    CNT_DONE = CNT_ERR + 1        // CTAs of the level's last kernel that have finished (it resets the slot)
 };
-static_assert(CNT_QUEUE + kMaxSegs <= CNT_ERR && CNT_ERR < 256, "counter slots");
+static_assert(CNT_ZEROED <= CNT_ERR && CNT_DONE < 256, "counter slots");
 
 // ---- accumulators -------------------------------------------------------------------------
 // FP32: compensated pair (hi + lo) — Kahan accumulation inside a thread (of pairs of consecutive
@@ -169,6 +173,35 @@ template <int PREC, class RT>
 __device__ __forceinline__ RT u01_word(uint32_t w) {
     if (PREC == PREC_FP64) return (RT)__dadd_rn(__dmul_rn((double)w, 0x1p-32), 0x1p-33);
     return (RT)__fadd_rn(__fmul_rn(__uint2float_rn(w), 0x1p-32f), 0x1p-33f);
+}
+
+// Inner values of one block: X = Y + Z of the shift model (four; FP32 rounds Y + radius x sine or
+// cosine once), and the reference model's difference (model_sampler.cpp:62-76; two).
+template <int PREC, class RT>
+__device__ __forceinline__ void shift_values(uint64_t v0, uint64_t v1, RT Y, RT* d) {
+    if constexpr (PREC == PREC_FP32) {
+        F2 sn, cs, r;
+        boxmuller32_f_polar(v0, v1, sn, cs, r);
+        const F2 Y2 = f2(Y, Y);
+        sn = f2_fma(sn, r, Y2);
+        cs = f2_fma(cs, r, Y2);
+        d[0] = f2_lo(sn); d[1] = f2_lo(cs); d[2] = f2_hi(sn); d[3] = f2_hi(cs);
+    } else {
+        bm_block<PREC, RT>(v0, v1, d);
+#pragma unroll
+        for (int q = 0; q < 4; q++) d[q] = xadd(Y, d[q]);
+    }
+}
+template <int PREC, class RT>
+__device__ __forceinline__ void ref_values(uint64_t v0, uint64_t v1, RT Y, RT st, RT s1t, RT* d) {
+    RT z[4];
+    bm_block<PREC, RT>(v0, v1, z);
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const RT a = xadd(xmul(st, Y), xmul(s1t, z[2 * q]));
+        const RT c = xadd(xmul(st, z[2 * q + 1]), xmul(s1t, z[2 * q]));
+        d[q] = xsub(xmul(a, a), xmul(c, c));
+    }
 }
 
 // normal k of an OUTER phase (used for the outer draws)
@@ -772,19 +805,10 @@ __device__ __forceinline__ void eval_chunk_c(const DevLevel<RT>& D, uint32_t ite
             uint64_t v0, v1;
             threefry2x64((s0 >> 2) + b, tag, key, v0, v1);
             RT z[4];
-            if constexpr (PREC == PREC_FP32) {   // d = Y + radius x sine or cosine, rounded once
-                F2 sn, cs, r;
-                boxmuller32_f_polar(v0, v1, sn, cs, r);
-                const F2 Y2 = f2(Y, Y);
-                sn = f2_fma(sn, r, Y2);
-                cs = f2_fma(cs, r, Y2);
-                z[0] = f2_lo(sn); z[1] = f2_lo(cs); z[2] = f2_hi(sn); z[3] = f2_hi(cs);
-            } else {
-                bm_block<PREC, RT>(v0, v1, z);
-            }
+            shift_values<PREC, RT>(v0, v1, Y, z);
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-                RT d = (PREC == PREC_FP32) ? z[q] : xadd(Y, z[q]);
+                RT d = z[q];
                 if (PREC == PREC_FP32 && S2) d = (RT)((float)d + shift);
                 z[q] = d;
                 if (S2) { if (PREC == PREC_FP32) a2.add_sq(d); else a2.add(xmul(d, d)); }
@@ -800,13 +824,11 @@ __device__ __forceinline__ void eval_chunk_c(const DevLevel<RT>& D, uint32_t ite
         for (uint32_t b = 0; b < C / 2; b++) {   // one block = two inner samples
             uint64_t v0, v1;
             threefry2x64((s0 >> 1) + b, tag, key, v0, v1);
-            RT z[4], X[2];
-            bm_block<PREC, RT>(v0, v1, z);
+            RT X[2];
+            ref_values<PREC, RT>(v0, v1, Y, st, s1t, X);
 #pragma unroll
             for (int q = 0; q < 2; q++) {
-                RT a = xadd(xmul(st, Y), xmul(s1t, z[2 * q]));
-                RT c = xadd(xmul(st, z[2 * q + 1]), xmul(s1t, z[2 * q]));
-                RT d = xsub(xmul(a, a), xmul(c, c));
+                RT d = X[q];
                 if (PREC == PREC_FP32 && S2) d = (RT)((float)d + shift);
                 X[q] = d;
                 if (S2) { if (PREC == PREC_FP32) a2.add_sq(d); else a2.add(xmul(d, d)); }
@@ -945,18 +967,16 @@ struct Seg {
 
 struct SegSet {
     int n;
+    int queue;               // counter slot of the first segment's tile tickets
+    int reduce;              // the level's last launch: its last CTA forms the level's sums
     Seg s[kMaxSegs];
 };
 
 // Adaptive decision after a pilot of `cur` samples (get_samples_count, 240-273, with
-// sample_inner_delta2, 120-129).  Writes the final count of a decided item; returns true when
-// the item goes on to the next pilot round.
+// sample_inner_delta2, 120-129): the side's final count, or 0 when it goes on to the next round.
 template <class RT, int PREC>
-__device__ __forceinline__ bool pilot_decide(const DevLevel<RT>& D, const Seg& g, uint32_t item, RT start,
-                                             const Acc<PREC>& a1, const Acc<PREC>& a2) {
-    const OuterLevel<RT>& L = D.L;
-    const CountParams& cp = (g.mode == 0) ? L.cf : L.cc;
-    const uint64_t cur = g.count;
+__device__ __forceinline__ uint32_t pilot_count(const OuterLevel<RT>& L, const CountParams& cp, uint64_t cur, RT start,
+                                                const Acc<PREC>& a1, const Acc<PREC>& a2) {
     bool done;
     if (PREC == PREC_FP32) {
         // the sums are of d + start (eval_chunk): their mean is the distance start + mean(d);
@@ -986,11 +1006,18 @@ __device__ __forceinline__ bool pilot_decide(const DevLevel<RT>& D, const Seg& g
         else newc = xmul(xpow(delta2, xdiv(-L.adaptive_r, (RT)2)), (RT)cp.tmp);
         done = newc <= (RT)cur;
     }
-    uint32_t* cnt = (g.mode == 0) ? D.B.cnt_f : D.B.cnt_c;
-    if (done) { cnt[item] = (uint32_t)cur; return false; }
-    const uint64_t nxt = cur * 2;
-    if (cp.max_count <= 2 * nxt) { cnt[item] = (uint32_t)cp.max_count; return false; }
-    return true;
+    if (done) return (uint32_t)cur;
+    return cp.max_count <= 4 * cur ? (uint32_t)cp.max_count : 0u;
+}
+
+// The decision of one item of a pilot segment: stores the count of a decided item, returns true
+// for one that goes on.
+template <class RT, int PREC>
+__device__ __forceinline__ bool pilot_decide(const DevLevel<RT>& D, const Seg& g, uint32_t item, RT start,
+                                             const Acc<PREC>& a1, const Acc<PREC>& a2) {
+    const uint32_t n = pilot_count<RT, PREC>(D.L, g.mode == 0 ? D.L.cf : D.L.cc, g.count, start, a1, a2);
+    if (n) (g.mode == 0 ? D.B.cnt_f : D.B.cnt_c)[item] = n;
+    return n == 0;
 }
 
 // Appends the warp's surviving items to the next round's list: one atomic per warp (all 32
@@ -1023,7 +1050,7 @@ __device__ __forceinline__ uint32_t pilots_taken(uint32_t cnt, const CountParams
 // moment slots mom[q * kTile] (q = 0..3 phi_f^k, 4..7 (phi_f - phi_c)^k; a zero phi adds
 // nothing and touches no slot), the counts of items that hit the maximum / stayed at the base
 // count, and the trace record.
-template <class RT, int KIND, class S>
+template <class RT, int KIND, class S, int STRIDE = kTile>
 __device__ __forceinline__ void final_item(const DevLevel<RT>& D, uint32_t item, RT mean_big, RT phi_small,
                                            bool fine_big, double* mom, uint32_t& n_max, uint32_t& n_base,
                                            TraceRec* trace) {
@@ -1035,14 +1062,14 @@ __device__ __forceinline__ void final_item(const DevLevel<RT>& D, uint32_t item,
     if (f_phi != (RT)0) {
         RT p = 1;
 #pragma unroll
-        for (int q = 0; q < 4; q++) { p = xmul(p, f_phi); mom[q * kTile] += (double)p; }
+        for (int q = 0; q < 4; q++) { p = xmul(p, f_phi); mom[q * STRIDE] += (double)p; }
     }
     if (!D.L.fine_only) {
         const RT dphi = xsub(f_phi, c_phi);
         if (dphi != (RT)0) {
             RT p = 1;
 #pragma unroll
-            for (int q = 0; q < 4; q++) { p = xmul(p, dphi); mom[(4 + q) * kTile] += (double)p; }
+            for (int q = 0; q < 4; q++) { p = xmul(p, dphi); mom[(4 + q) * STRIDE] += (double)p; }
         }
     }
     const uint32_t cf = D.B.cnt_f[item];
@@ -1060,6 +1087,46 @@ __device__ __forceinline__ void final_item(const DevLevel<RT>& D, uint32_t item,
         tr.pilots = pilots_taken(cf, D.L.cf, D.L.adaptive_f) +
                     (D.L.fine_only ? 0u : pilots_taken((uint32_t)tr.count_c, D.L.cc, D.L.adaptive_c));
         trace[item] = tr;
+    }
+}
+
+// Device timestamp (%globaltimer, nanoseconds) of a level's begin (slot 0) or end (slot 1).
+__device__ __forceinline__ void level_stamp(uint64_t* stamps, int slot) {
+    if (!stamps) return;
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    stamps[slot] = t;
+}
+
+// End of a level's last kernel, called by all T threads of every CTA after its partial sums are
+// written: the CTA that arrives last adds the partials of all `slots` CTAs to the level's 16 sums
+// (thread t sum t % 16 of slots t / 16, t / 16 + T / 16, ..., then the groups in order: a fixed
+// order) and stores them, with the path-limit flag in entry 12, where the caller reads them — in
+// the host's pinned memory, so a call needs neither a reduction kernel (7 us) nor a copy back.
+template <int T>
+__device__ __forceinline__ void level_finish(const OuterBuffers& B, int slots) {
+    __shared__ double red[T / 16][17];
+    __shared__ uint32_t arrived;
+    const int t = threadIdx.x, q = t & 15, g = t >> 4;
+    __threadfence();
+    __syncthreads();
+    if (t == 0) arrived = atomicAdd(B.counters + CNT_DONE, 1u);
+    __syncthreads();
+    if (arrived != gridDim.x - 1) return;
+    __threadfence();
+    double v = 0;
+    for (int b = g; b < slots; b += T / 16) v += __ldcg(B.block_sums + (size_t)b * 16 + q);
+    red[g][q] = v;
+    __syncthreads();
+    if (t < 16) {
+        double s = 0;
+        for (int k = 0; k < T / 16; k++) s += red[k][t];
+        if (t == 12) s = (double)__ldcg(B.counters + CNT_ERR);
+        B.level_acc[t] = s;
+    }
+    if (t == 0) {
+        B.counters[CNT_DONE] = 0;
+        level_stamp(B.stamps, 1);
     }
 }
 
@@ -1115,7 +1182,7 @@ __global__ void __launch_bounds__(kTile, MINB) k_phase(DevLevel<RT> D, SegSet SS
         // device work queue: one ticket per tile, so no CTA waits for a second wave and uneven
         // tiles balance themselves.  The next ticket is claimed while the current tile is
         // evaluated.  Which CTA evaluates a tile does not change any result.
-        uint32_t* queue = counters + CNT_QUEUE + si;
+        uint32_t* queue = counters + SS.queue + si;
         if (t == 0) sm_ticket = atomicAdd(queue, 1u);
         __syncthreads();
         uint64_t ticket = sm_ticket;
@@ -1329,16 +1396,44 @@ __global__ void __launch_bounds__(kTile, MINB) k_phase(DevLevel<RT> D, SegSet SS
         for (int w = 0; w < kWarps; w++) v += sm_acc[w][t];
         D.B.block_sums[(size_t)blockIdx.x * 16 + t] += v;
     }
+    if (SS.reduce) level_finish<kTile>(D.B, D.B.slots);
 }
 
 // ---- outer draws ---------------------------------------------------------------------------
 // sample_outer of the model (Y = randn_sync, model_sampler.cpp:57-59) or of the portfolio (the
 // stocks at tau and the delta-CV constant, portfolio_sampler.cpp:293-311, 606-614) per outer
-// sample, from the OUTER layout's phase-0 draws.
+// sample, from the OUTER layout's phase-0 draws.  Also clears what the batch's later kernels count
+// in, and (first batch of a level) their partial sums.
+// GBM of stock s at tau and its row entry (R, ln R) on the FP32 path, R alone otherwise.
+template <class RT, int PREC>
+__device__ __forceinline__ RT stock_at_tau(const OptionTable<RT>& ot, uint32_t s, RT W, RT* Rrow) {
+    constexpr uint32_t RS = RStride<PREC>::v;
+    RT R;
+    if (PREC == PREC_FP32) {                     // in float (expf), with its logarithm
+        const float sg = (float)ot.sigma[s], S0 = (float)ot.S0[s];
+        const float e = sg * (float)W + ((float)ot.mu[s] - 0.5f * sg * sg) * (float)ot.tau;
+        R = (RT)(S0 * expf(e));
+        Rrow[s * RS + 1] = (RT)(logf(S0) + e);
+    } else {
+        R = simulate_stock_ref<RT>(ot.S0[s], ot.mu[s], ot.sigma[s], ot.tau, W);
+    }
+    Rrow[s * RS] = R;
+    return R;
+}
+
 template <class RT, int KIND, int PREC, class S = NoSampler>
-__global__ void __launch_bounds__(kTile) k_outer(DevLevel<RT> D, uint32_t nb) {
+__global__ void __launch_bounds__(kTile) k_outer(DevLevel<RT> D, uint32_t nb, int first) {
     const OuterLevel<RT>& L = D.L;
     RT* Yv = reinterpret_cast<RT*>(D.B.Yv);
+    const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x, gsz = gridDim.x * blockDim.x;
+    for (uint32_t k = gid; k < (uint32_t)CNT_ZEROED; k += gsz) D.B.counters[k] = 0;
+    if (first) {
+        for (uint32_t k = gid; k < (uint32_t)D.B.slots * 16; k += gsz) D.B.block_sums[k] = 0;
+        if (gid == 0) {
+            D.B.counters[CNT_ERR] = 0;
+            level_stamp(D.B.stamps, 0);
+        }
+    }
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nb; i += gridDim.x * blockDim.x) {
         const TfKey key = tf_key(L.seed, outer_stream_id(L.ell, L.first_index + i));
         D.B.cnt_f[i] = L.adaptive_f ? 0u : (uint32_t)L.cf.max_count;
@@ -1374,16 +1469,7 @@ __global__ void __launch_bounds__(kTile) k_outer(DevLevel<RT> D, uint32_t nb) {
                     if (k == 0) { dW_sys = xmul(ot.stau, z[0]); if (ot.Q > 1) continue; }
                     const uint32_t s = ot.Q == 1 ? 0 : k - 1;
                     RT W = ot.Q == 1 ? dW_sys : xadd(xmul(ot.rho, dW_sys), xmul(ot.s1_rho2, xmul(ot.stau, z[q])));
-                    RT R;
-                    if (PREC == PREC_FP32) {     // GBM at tau in float (expf) and its logarithm
-                        const float sg = (float)ot.sigma[s], S0 = (float)ot.S0[s];
-                        const float e = sg * (float)W + ((float)ot.mu[s] - 0.5f * sg * sg) * (float)ot.tau;
-                        R = (RT)(S0 * expf(e));
-                        Rrow[s * RS + 1] = (RT)(logf(S0) + e);
-                    } else {
-                        R = simulate_stock_ref<RT>(ot.S0[s], ot.mu[s], ot.sigma[s], ot.tau, W);
-                    }
-                    Rrow[s * RS] = R;
+                    const RT R = stock_at_tau<RT, PREC>(ot, s, W, Rrow);
                     if (ot.use_delta_cv) cv = xadd(cv, xmul(xsub(R, ot.S0[s]), ot.delta_coalesce[s]));
                 }
             }
@@ -1400,13 +1486,13 @@ template <class RT>
 __global__ void k_classify(DevLevel<RT> D, uint32_t nb, int pass) {
     uint32_t* counters = D.B.counters;
     const uint32_t C = D.L.chunk;
-    __shared__ uint32_t offs[64], hist[64], base[64];
+    __shared__ uint32_t offs[kMaxSegs], hist[kMaxSegs], base[kMaxSegs];
     if (pass == 1 && threadIdx.x == 0) {
         uint32_t a = 0;
-        for (int k = 0; k < 64; k++) { offs[k] = a; a += counters[CNT_CLASS + k]; }
+        for (int k = 0; k < kMaxSegs; k++) { offs[k] = a; a += counters[CNT_CLASS + k]; }
     }
     for (uint32_t t0 = blockIdx.x * blockDim.x; t0 < nb; t0 += gridDim.x * blockDim.x) {
-        if (threadIdx.x < 64) hist[threadIdx.x] = 0;
+        if (threadIdx.x < kMaxSegs) hist[threadIdx.x] = 0;
         __syncthreads();
         const uint32_t i = t0 + threadIdx.x;
         const bool valid = i < nb;
@@ -1418,30 +1504,13 @@ __global__ void k_classify(DevLevel<RT> D, uint32_t nb, int pass) {
             rank = atomicAdd(&hist[k], 1u);
         }
         __syncthreads();
-        if (threadIdx.x < 64 && hist[threadIdx.x]) {
+        if (threadIdx.x < kMaxSegs && hist[threadIdx.x]) {
             if (pass == 0) atomicAdd(&counters[CNT_CLASS + threadIdx.x], hist[threadIdx.x]);
             else base[threadIdx.x] = atomicAdd(&counters[CNT_FILL + threadIdx.x], hist[threadIdx.x]);
         }
         __syncthreads();
         if (pass == 1 && valid) D.B.class_items[offs[k] + base[k] + rank] = i;
         __syncthreads();
-    }
-}
-
-// Per-CTA partials -> the level's 16 sums, one CTA of 256 threads: thread t adds sum q = t % 16 of
-// CTA slots t / 16, t / 16 + 16, ... (consecutive threads read consecutive doubles), then thread q
-// adds its 16 group sums in a fixed order.  Launch with 256 threads.
-static __global__ void __launch_bounds__(256) k_reduce_blocks(const double* block_sums, int grid, double* level_acc) {
-    __shared__ double sm[16][17];
-    const int t = threadIdx.x, q = t & 15, g = t >> 4;
-    double v = 0;
-    for (int b = g; b < grid; b += 16) v += block_sums[(size_t)b * 16 + q];
-    sm[g][q] = v;
-    __syncthreads();
-    if (t < 16) {
-        double s = 0;
-        for (int k = 0; k < 16; k++) s += sm[k][t];
-        level_acc[t] += s;
     }
 }
 
@@ -1474,9 +1543,8 @@ static int phase_grid(int cap) {
 
 template <class RT, int KIND, int PREC, int MINB, class S = NoSampler>
 static void launch_phase_v(const DevLevel<RT>& D, const SegSet& SS, TraceRec* trace, cudaStream_t stream) {
-    cudaMemsetAsync(D.B.counters + CNT_QUEUE, 0, kMaxSegs * sizeof(uint32_t), stream);
     if (D.B.prof_mark) D.B.prof_mark(D.B.prof_user, 0, stream);
-    const int grid = phase_grid<RT, KIND, PREC, MINB, S>(D.B.grid);
+    const int grid = phase_grid<RT, KIND, PREC, MINB, S>(D.B.slots);
     k_phase<RT, KIND, PREC, MINB, S><<<grid, kTile, phase_dyn_smem<KIND, PREC>(), stream>>>(D, SS, trace);
     if (D.B.prof_mark) D.B.prof_mark(D.B.prof_user, 1, stream);
     count_launch();
@@ -1506,7 +1574,7 @@ static inline uint32_t ilog2_u64(uint64_t v) {
 }
 
 template <class RT, int KIND, int PREC, class S = NoSampler>
-static cudaError_t run_batch(DevLevel<RT>& D, uint32_t nb, TraceRec* trace, cudaStream_t stream) {
+static cudaError_t run_batch(DevLevel<RT>& D, uint32_t nb, TraceRec* trace, cudaStream_t stream, bool first, bool last) {
     const OuterLevel<RT>& L = D.L;
     OuterBuffers& B = D.B;
     const uint32_t C = L.chunk;
@@ -1515,7 +1583,14 @@ static cudaError_t run_batch(DevLevel<RT>& D, uint32_t nb, TraceRec* trace, cuda
     int og = (int)((nb + kTile - 1) / kTile);
     if (og > grid) og = grid;
     if (og < 1) og = 1;
-    k_outer<RT, KIND, PREC, S><<<og, kTile, 0, stream>>>(D, nb);
+    const uint64_t maxc = (L.fine_only || L.cf.max_count >= L.cc.max_count) ? L.cf.max_count : L.cc.max_count;
+    if (first) {
+        // CTAs of the phase launches: at most two tiles (fine and coarse) per 256 chunks of the
+        // largest count, so a small call neither starts nor sums hundreds of idle CTAs
+        const uint64_t nch = maxc / C, tiles = nch <= (uint64_t)kTile ? 2 * (((uint64_t)nb * nch + kTile - 1) / kTile) : 2ull * nb;
+        B.slots = tiles + 16 < (uint64_t)grid ? (int)tiles + 16 : grid;     // 16: partly filled tiles of the final classes
+    }
+    k_outer<RT, KIND, PREC, S><<<og, kTile, 0, stream>>>(D, nb, first ? 1 : 0);
     count_launch();
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
 
@@ -1524,45 +1599,44 @@ static cudaError_t run_batch(DevLevel<RT>& D, uint32_t nb, TraceRec* trace, cuda
         if (L.adaptive_f) for (uint64_t c = L.cf.base_count; L.cf.max_count > 2 * c; c *= 2) rounds_f++;
         if (L.adaptive_c) for (uint64_t c = L.cc.base_count; L.cc.max_count > 2 * c; c *= 2) rounds_c++;
         const uint32_t rounds = rounds_f > rounds_c ? rounds_f : rounds_c;
+        if (rounds >= (uint32_t)kMaxRounds) return cudaErrorInvalidValue;
         uint32_t* listF[2] = {B.lists, B.lists + B.cap};
         uint32_t* listC[2] = {B.lists + 2 * B.cap, B.lists + 3 * B.cap};
         for (uint32_t r = 0; r < rounds; r++) {
             const int cur = r & 1, nxt = cur ^ 1;
-            e = cudaMemsetAsync(B.counters + CNT_LIST + nxt, 0, sizeof(uint32_t), stream);
-            if (e == cudaSuccess) e = cudaMemsetAsync(B.counters + CNT_LIST + 2 + nxt, 0, sizeof(uint32_t), stream);
-            if (e != cudaSuccess) return e;
             SegSet SS;
             SS.n = 0;
+            SS.queue = CNT_QUEUE + 2 * (int)r;
+            SS.reduce = 0;
             for (int which = 0; which < 2; which++) {
                 const bool fine = which == 0;
                 if (fine ? (r >= rounds_f) : (r >= rounds_c)) continue;
                 const CountParams& cp = fine ? L.cf : L.cc;
                 Seg& g = SS.s[SS.n++];
                 g.list = (r == 0) ? nullptr : (fine ? listF[cur] : listC[cur]);
-                g.n_slot = CNT_LIST + (fine ? 0 : 2) + cur;
+                g.n_slot = CNT_LIST + 2 * r + (fine ? 0 : 1);
                 g.n_host = nb;
                 g.count = cp.base_count << r;
                 g.nch_log2 = ilog2_u64(g.count / C);
                 g.tag = (fine ? PH_FINE : PH_COARSE) + r;
                 g.mode = fine ? 0 : 1;
                 g.class_k = 0;
-                g.next_slot = CNT_LIST + (fine ? 0 : 2) + nxt;
+                g.next_slot = CNT_LIST + 2 * (r + 1) + (fine ? 0 : 1);
                 g.next_list = fine ? listF[nxt] : listC[nxt];
             }
             if (SS.n == 0) continue;
             launch_phase<RT, KIND, PREC, S>(D, SS, nullptr, stream);
             if ((e = cudaGetLastError()) != cudaSuccess) return e;
         }
-        e = cudaMemsetAsync(B.counters + CNT_CLASS, 0, 128 * sizeof(uint32_t), stream);
-        if (e != cudaSuccess) return e;
         k_classify<RT><<<og, kTile, 0, stream>>>(D, nb, 0);
         k_classify<RT><<<og, kTile, 0, stream>>>(D, nb, 1);
         count_launch(2);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        const uint64_t maxc = L.cf.max_count > L.cc.max_count ? L.cf.max_count : L.cc.max_count;
-        const uint32_t kmax = ilog2_u64(maxc / C);
+        const uint32_t kmax = ilog2_u64((L.cf.max_count > L.cc.max_count ? L.cf.max_count : L.cc.max_count) / C);
         SegSet SS;
         SS.n = 0;
+        SS.queue = CNT_QUEUE + 2 * kMaxRounds;
+        SS.reduce = last;
         for (uint32_t k = 0; k <= kmax && SS.n < kMaxSegs; k++) {
             Seg& g = SS.s[SS.n++];
             g.list = B.class_items;
@@ -1579,15 +1653,16 @@ static cudaError_t run_batch(DevLevel<RT>& D, uint32_t nb, TraceRec* trace, cuda
         launch_phase<RT, KIND, PREC, S>(D, SS, trace, stream);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     } else {
-        const uint64_t cbig = (L.fine_only || L.cf.max_count >= L.cc.max_count) ? L.cf.max_count : L.cc.max_count;
         SegSet SS;
         SS.n = 1;
+        SS.queue = CNT_QUEUE + 2 * kMaxRounds;
+        SS.reduce = last;
         Seg& g = SS.s[0];
         g.list = nullptr;
         g.n_slot = 0;
         g.n_host = nb;
-        g.count = cbig;
-        g.nch_log2 = ilog2_u64(cbig / C);
+        g.count = maxc;
+        g.nch_log2 = ilog2_u64(maxc / C);
         g.tag = PH_FINAL;
         g.mode = 2;
         g.class_k = 0;
@@ -1608,13 +1683,12 @@ cudaError_t sample_level_t(const OuterLevel<RT>& L, OuterBuffers& B, TraceRec* t
     for (uint64_t done = 0; done < L.M;) {
         const uint64_t nb = (L.M - done) < B.cap ? (L.M - done) : B.cap;
         D.L.first_index = L.first_index + done;
-        cudaError_t e = run_batch<RT, KIND, PREC, S>(D, (uint32_t)nb, trace ? trace + done : nullptr, stream);
+        cudaError_t e = run_batch<RT, KIND, PREC, S>(D, (uint32_t)nb, trace ? trace + done : nullptr, stream, done == 0,
+                                                     done + nb == L.M);
         if (e != cudaSuccess) return e;
         done += nb;
     }
-    k_reduce_blocks<<<1, 256, 0, stream>>>(B.block_sums, B.grid, B.level_acc);
-    count_launch();
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 }  // namespace nmlmc
