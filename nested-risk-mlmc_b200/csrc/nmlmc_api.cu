@@ -134,10 +134,12 @@ struct DevPortfolio {
 // counts (the launch sequence of a level follows from its level and batch count).
 struct GraphSlot {
     std::vector<uint64_t> key;
+    uint64_t small = 0;           // levels (by position) that run as one kernel, the others as sequences
     cudaGraphExec_t exec = nullptr;
     uint64_t last_use = 0;
 };
-constexpr size_t kGraphCache = 16;
+// A continuation run meets about 30 topologies; instantiating one takes 100 us and more.
+constexpr size_t kGraphCache = 48;
 
 // Phase-kernel configuration of one level: register/occupancy variant and chunk length.
 struct PhaseChoice {
@@ -911,15 +913,38 @@ int sample_outer_levels(nmlmc_ctx* c, uint32_t n, const uint32_t* ells, const ui
     }
     uint64_t* h_st = reinterpret_cast<uint64_t*>(c->h_lev + kMaxSubmit * 16);
     memset(c->h_lev, 0, kMaxSubmit * 18 * sizeof(double));
+    // the round's levels, and which of them are small enough to run as one kernel
+    std::vector<OuterLevel<RT>> levels(n);
+    std::vector<uint64_t> key;
+    uint64_t small = 0;
+    const OuterBuffers& ob = c->ob;
+    for (uint32_t i = 0; i < n; i++) {
+        const uint32_t ell = ells[i];
+        uint64_t lo;
+        shard_range(c, Mtot[i], lo, Ms[i]);
+        levels[i] = outer_level_params<RT>(c, ell, Ms[i], next[ell] + lo);
+        next[ell] += Mtot[i];
+        key.push_back(ell);
+        key.push_back((Ms[i] + ob.cap - 1) / ob.cap);
+        if (Ms[i] && level_is_small(levels[i], c->kind, c->cfg.precision, ob)) small |= 1ull << i;
+    }
+    // the executable graph of a recent round with the same levels is reused if it runs no level as
+    // one kernel that is too large for it now, and at most one small level as a sequence (60 us more,
+    // an instantiation costs 100 us)
+    GraphSlot* slot = nullptr;
+    for (GraphSlot& g : c->graphs) {
+        const int more = __builtin_popcountll(small & ~g.small);
+        if (g.key == key && (g.small & ~small) == 0 && more <= 1 &&
+            (!slot || __builtin_popcountll(g.small) > __builtin_popcountll(slot->small)))
+            slot = &g;
+    }
+    if (slot) small = slot->small;
     NM_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
     cudaError_t err = cudaSuccess;
     for (uint32_t i = 0; i < n && err == cudaSuccess; i++) {
-        const uint32_t ell = ells[i];
-        uint64_t lo, M;
-        shard_range(c, Mtot[i], lo, M);
-        Ms[i] = M;
-        OuterLevel<RT> L = outer_level_params<RT>(c, ell, M, next[ell] + lo);
-        next[ell] += Mtot[i];
+        const uint64_t M = Ms[i];
+        OuterLevel<RT>& L = levels[i];
+        L.no_small = !(small >> i & 1);
         OuterBuffers B = c->ob;
         B.level_acc = c->h_lev + 16 * (size_t)i;       // pinned: sums and stamps go straight to the host
         B.stamps = h_st + 2 * i;
@@ -933,18 +958,7 @@ int sample_outer_levels(nmlmc_ctx* c, uint32_t n, const uint32_t* ells, const ui
         if (graph) cudaGraphDestroy(graph);
         return cuda_status(err, "capture level round");
     }
-    // the executable graph of this topology, if a recent round had it: update it in place
-    std::vector<uint64_t> key;
-    for (uint32_t i = 0; i < n; i++) {
-        key.push_back(ells[i]);
-        key.push_back((Ms[i] + c->ob.cap - 1) / c->ob.cap);
-    }
-    size_t nodes = 0;                              // small levels are one launch instead of a sequence
-    cudaGraphGetNodes(graph, nullptr, &nodes);
-    key.push_back(nodes);
-    GraphSlot* slot = nullptr;
-    for (GraphSlot& g : c->graphs)
-        if (g.key == key) slot = &g;
+    // update it in place
     if (slot && slot->exec) {
         cudaGraphExecUpdateResultInfo info;
         if (cudaGraphExecUpdate(slot->exec, graph, &info) == cudaSuccess) {
@@ -971,7 +985,7 @@ int sample_outer_levels(nmlmc_ctx* c, uint32_t n, const uint32_t* ells, const ui
                 if (c->graphs[lru].exec) cudaGraphExecDestroy(c->graphs[lru].exec);
                 c->graphs.erase(c->graphs.begin() + lru);
             }
-            c->graphs.push_back(GraphSlot{key, nullptr, 0});
+            c->graphs.push_back(GraphSlot{key, small, nullptr, 0});
             slot = &c->graphs.back();
         }
         slot->exec = exec;

@@ -1514,6 +1514,275 @@ __global__ void k_classify(DevLevel<RT> D, uint32_t nb, int pass) {
     }
 }
 
+// ---- small calls: one warp per outer sample, one launch --------------------------------------
+// A call of few outer samples is all latency in the breadth-first sequence: 2 + rounds + 3 launches
+// of one or two CTAs each, whose threads draw a whole chunk (32 inner samples, 8 to 16 generator
+// blocks in a row, 4 to 7 us) alone.  Here a warp takes an outer sample through its draw, pilots and
+// final estimate depth-first; the lanes draw the blocks of up to 32 chunks side by side into shared
+// memory, then lane c adds chunk c's values in their order.  Chunks, chunk sums and merges are those
+// of k_phase (same grouping, same order), so every mean, count and phi is the same bit for bit and a
+// call split into small ones gives the same samples.
+constexpr int kSmallThreads = 128, kSmallWarps = kSmallThreads / 32;
+
+template <class RT, int KIND, int PREC>
+struct SmallWarp {
+    const DevLevel<RT>& D;
+    TfKey key;
+    RT Y;                    // models: the outer draw
+    RT start;                // start value of the inner estimates
+    RT* row;                 // portfolio: R_tau row in shared memory
+    RT* st;                  // staged inner values [32][kSmallMaxChunk + 1]
+    double work, inner;
+    int lane;
+
+    static constexpr uint32_t kStride = kSmallMaxChunk + 1;
+    static constexpr uint32_t kPerBlock = KIND == KIND_SHIFT_MODEL ? 4 : 2;    // inner samples per block
+
+    // outer draws (k_outer)
+    __device__ __forceinline__ void outer(uint32_t item) {
+        const OuterLevel<RT>& L = D.L;
+        key = tf_key(L.seed, outer_stream_id(L.ell, L.first_index + item));
+        if constexpr (!is_portfolio_kind(KIND)) {
+            Y = outer_normal_at<PREC, RT>(key, PH_OUTER, 0);
+            start = -L.mp.max_loss;
+        } else {
+            const OptionTable<RT>& ot = L.ot;
+            const uint32_t nnorm = ot.Q == 1 ? 1 : ot.Q + 1;
+            RT dW_sys = 0, cv = (RT)0;
+            for (uint32_t b0 = 0; 4 * b0 < nnorm; b0 += 32) {
+                uint64_t v0, v1;
+                threefry2x64(b0 + lane, PH_OUTER, key, v0, v1);
+                RT z[4], c[4];
+                bm_block<PREC, RT>(v0, v1, z);
+                if (b0 == 0) dW_sys = xmul(ot.stau, __shfl_sync(0xffffffffu, z[0], 0));
+#pragma unroll
+                for (uint32_t q = 0; q < 4; q++) {
+                    const uint32_t k = 4 * (b0 + lane) + q;
+                    c[q] = (RT)0;
+                    if (k >= nnorm || (k == 0 && ot.Q > 1)) continue;
+                    const uint32_t s = ot.Q == 1 ? 0 : k - 1;
+                    const RT W = ot.Q == 1 ? dW_sys : xadd(xmul(ot.rho, dW_sys), xmul(ot.s1_rho2, xmul(ot.stau, z[q])));
+                    const RT R = stock_at_tau<RT, PREC>(ot, s, W, row);
+                    c[q] = xmul(xsub(R, ot.S0[s]), ot.delta_coalesce[s]);
+                }
+                if (ot.use_delta_cv) {           // the control variate's sum in stock order
+                    for (uint32_t l = 0; l < 32 && 4 * (b0 + l) < nnorm; l++)
+#pragma unroll
+                        for (uint32_t q = 0; q < 4; q++) {
+                            const uint32_t k = 4 * (b0 + l) + q;
+                            const RT t = __shfl_sync(0xffffffffu, c[q], l);
+                            if (k < nnorm && !(k == 0 && ot.Q > 1)) cv = xadd(cv, t);
+                        }
+                }
+            }
+            start = xsub(-ot.max_loss, cv);
+            __syncwarp();
+        }
+    }
+
+    // the inner values of one block of a phase (eval_chunk_c)
+    __device__ __forceinline__ void values(uint32_t tag, uint64_t blk, RT* d) {
+        uint64_t v0, v1;
+        threefry2x64(blk, tag, key, v0, v1);
+        if constexpr (KIND == KIND_SHIFT_MODEL) {
+            shift_values<PREC, RT>(v0, v1, Y, d);
+        } else if constexpr (KIND == KIND_REF_MODEL) {
+            ref_values<PREC, RT>(v0, v1, Y, D.L.mp.stau, D.L.mp.s1tau, d);
+        } else {
+            const OptionTable<RT>& ot = D.L.ot;
+            const uint64_t v[2] = {v0, v1};
+            if (PREC == PREC_FP32 && ot.fast_s) {
+                if constexpr (sizeof(RT) == 4) {
+                    const float2* r = reinterpret_cast<const float2*>(row);
+                    if (ot.fast_col) {
+                        for (int q = 0; q < 2; q++) d[q] = pf_sample_loss<PF_COLUMN>(v[q], ot, r);
+                    } else if (ot.subsample == SUB_UNIFORM) {
+                        for (int q = 0; q < 2; q++) d[q] = pf_sample_loss<PF_UNIFORM_L1>(v[q], ot, r);
+                    } else {
+                        for (int q = 0; q < 2; q++) d[q] = pf_sample_loss<PF_ALIAS>(v[q], ot, r);
+                    }
+                }
+            } else {
+                for (int q = 0; q < 2; q++) {
+                    RT prob;
+                    const uint32_t j = pf_pick<RT>(ot, v[q], prob);
+                    d[q] = xdiv(pf_value<RT, RStride<PREC>::v>(ot, row, j), prob);
+                    work += (double)ot.W_est[j];
+                }
+            }
+        }
+    }
+
+    // One phase: `count` inner samples in chunks of C.  Pilots sum the (FP32: shifted) values and
+    // their squares; the final phase also the phi of every small group of gs chunks (csmall samples,
+    // weight coeff).  Results in every lane.
+    __device__ __forceinline__ void phase(uint32_t tag, uint64_t count, bool pilot, uint32_t gs, uint64_t csmall,
+                                          float coeff, Acc<PREC>& tot1, Acc<PREC>& tot2, float& tind) {
+        const uint32_t C = D.L.chunk, nch = (uint32_t)(count / C);
+        const uint32_t bpc = C / kPerBlock, bsh = 31 - __clz(bpc);     // blocks per chunk (a power of two)
+        const bool unit_work = !is_portfolio_kind(KIND) || (PREC == PREC_FP32 && D.L.ot.fast_s);
+        // eval_chunk_c adds pairs of consecutive values on the FP32 path, singles in the generic one
+        const bool pairs = PREC != PREC_FP32 || unit_work;
+        const float shift = pilot && PREC == PREC_FP32 ? (float)start : 0.f;
+        tot1.zero();
+        tot2.zero();
+        tind = 0.f;
+        Acc<PREC> t1, gacc, gsum;
+        t1.zero();
+        gacc.zero();
+        gsum.zero();
+        for (uint32_t c0 = 0; c0 < nch; c0 += 32) {
+            const uint32_t n = nch - c0 < 32 ? nch - c0 : 32, nb = n << bsh;
+            for (uint32_t b = lane; b < nb; b += 32) {
+                RT d[kPerBlock];
+                values(tag, ((uint64_t)c0 << bsh) + b, d);
+                RT* to = st + (b >> bsh) * kStride + (b & (bpc - 1)) * kPerBlock;
+#pragma unroll
+                for (uint32_t q = 0; q < kPerBlock; q++)
+                    to[q] = (PREC == PREC_FP32 && pilot) ? (RT)((float)d[q] + shift) : d[q];
+            }
+            __syncwarp();
+            Acc<PREC> a1, a2;
+            a1.zero();
+            a2.zero();
+            float ind = 0.f;
+            if ((uint32_t)lane < n) {
+                const RT* v = st + lane * kStride;
+#pragma unroll 4
+                for (uint32_t k = 0; k < C; k += 2) {
+                    const RT x0 = v[k], x1 = v[k + 1];
+                    if (pilot) {
+                        if constexpr (PREC == PREC_FP32) { a2.add_sq(x0); a2.add_sq(x1); }
+                        else { a2.add(xmul(x0, x0)); a2.add(xmul(x1, x1)); }
+                    }
+                    if (pairs) a1.add2(x0, x1);
+                    else { a1.add(x0); a1.add(x1); }
+                }
+                if (unit_work) work += (double)C;
+                if (!pilot && gs == 1) ind = phi_of<KIND, NoSampler, RT>(inner_mean<RT, PREC>(start, a1, csmall), coeff);
+            }
+            __syncwarp();
+            for (uint32_t m = 1; m < n; m <<= 1) {
+                a1.merge(a1.shfl_xor(m));
+                if (pilot) a2.sq_merge_xor(m);
+                else {
+                    ind += __shfl_xor_sync(0xffffffffu, ind, m);
+                    if (2 * m == gs) ind = phi_of<KIND, NoSampler, RT>(inner_mean<RT, PREC>(start, a1, csmall), coeff);
+                }
+            }
+            if (nch <= 32) {
+                tot1 = a1;
+                tot2 = a2;
+                tind = ind;
+                break;
+            }
+            // warp sums in k_phase's order: groups of gs / 32 warps (32 < gs < kTile), else whole
+            // tiles of kWarps warps, with small groups of whole tiles summed across them
+            const uint32_t w = c0 / 32 + 1;
+            if (!pilot && gs > 32 && gs < (uint32_t)kTile) {
+                gsum.merge(a1);
+                if (w % (gs / 32) == 0) {
+                    tind += phi_of<KIND, NoSampler, RT>(inner_mean<RT, PREC>(start, gsum, csmall), coeff);
+                    tot1.merge(gsum);
+                    gsum.zero();
+                }
+            } else {
+                t1.merge(a1);
+                if (pilot) tot2.merge(a2);
+                else if (gs <= 32) tind += ind;
+                if (w % kWarps == 0 || c0 + 32 >= nch) {
+                    tot1.merge(t1);
+                    if (!pilot && gs >= (uint32_t)kTile) {
+                        gacc.merge(t1);
+                        if ((c0 + 32) % gs == 0) {
+                            tind += phi_of<KIND, NoSampler, RT>(inner_mean<RT, PREC>(start, gacc, csmall), coeff);
+                            gacc.zero();
+                        }
+                    }
+                    t1.zero();
+                }
+            }
+        }
+        inner += (double)count;
+        // lane 0's results (lanes past the chunks of a short phase hold nothing)
+        tot1 = bcast(tot1);
+        tot2 = bcast(tot2);
+        tind = __shfl_sync(0xffffffffu, tind, 0);
+    }
+    __device__ __forceinline__ static Acc<PREC> bcast(const Acc<PREC>& a) {
+        Acc<PREC> r;
+        if constexpr (PREC == PREC_FP32) {
+            r.hi = __shfl_sync(0xffffffffu, a.hi, 0);
+            r.lo = __shfl_sync(0xffffffffu, a.lo, 0);
+        } else {
+            r.v = __shfl_sync(0xffffffffu, a.v, 0);
+        }
+        return r;
+    }
+
+    // get_samples_count (nested_sampler.hpp:240-273) of one side
+    __device__ __forceinline__ uint32_t count(const CountParams& cp, uint32_t tag) {
+        for (uint64_t cur = cp.base_count;; cur *= 2, tag++) {
+            Acc<PREC> a1, a2;
+            float ind;
+            phase(tag, cur, true, 1, 1, 0.f, a1, a2, ind);
+            const uint32_t n = pilot_count<RT, PREC>(D.L, cp, cur, start, a1, a2);
+            if (n) return n;
+        }
+    }
+};
+
+template <class RT, int KIND, int PREC>
+__global__ void __launch_bounds__(kSmallThreads) k_small(DevLevel<RT> D, uint32_t nb, TraceRec* trace) {
+    using W = SmallWarp<RT, KIND, PREC>;
+    __shared__ RT sm_st[kSmallWarps][32 * W::kStride];
+    __shared__ double sm_mom[kSmallWarps * 8];
+    __shared__ double sm_acc[kSmallWarps][16];
+    extern __shared__ float2 k_small_rows[];             // [kSmallWarps][Q] rows of 8 bytes per stock
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const OuterLevel<RT>& L = D.L;
+    if (blockIdx.x == 0 && threadIdx.x == 0) level_stamp(D.B.stamps, 0);
+    W w{D, {}, (RT)0, (RT)0, reinterpret_cast<RT*>(k_small_rows + (size_t)warp * L.ot.Q), sm_st[warp], 0.0, 0.0, lane};
+    if (lane < 8) sm_mom[lane * kSmallWarps + warp] = 0;
+    __syncwarp();
+    uint32_t n_max = 0, n_base = 0;
+    for (uint32_t item = blockIdx.x * kSmallWarps + warp; item < nb; item += gridDim.x * kSmallWarps) {
+        w.outer(item);
+        const uint32_t cf = L.adaptive_f ? w.count(L.cf, PH_FINE) : (uint32_t)L.cf.max_count;
+        const uint32_t cc = L.adaptive_c ? w.count(L.cc, PH_COARSE) : (uint32_t)L.cc.max_count;
+        const bool fine_big = L.fine_only || cf > cc;
+        const uint32_t big = fine_big ? cf : cc, small = L.fine_only ? big : (fine_big ? cc : cf);
+        const uint32_t nch = big / L.chunk, gs = small / L.chunk;
+        Acc<PREC> a1, a2;
+        float ind;
+        w.phase(PH_FINAL, big, false, gs, small, (float)gs / (float)nch, a1, a2, ind);
+        if (lane == 0) {
+            D.B.cnt_f[item] = cf;
+            D.B.cnt_c[item] = cc;
+            final_item<RT, KIND, NoSampler, kSmallWarps>(D, item, inner_mean<RT, PREC>(w.start, a1, big), (RT)ind, fine_big,
+                                                         sm_mom + warp, n_max, n_base, trace);
+        }
+        __syncwarp();
+    }
+    double ws = w.work;
+    for (int m = 16; m > 0; m >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, m);
+    if (lane < 16) sm_acc[warp][lane] = lane < 8 ? sm_mom[lane * kSmallWarps + warp] : 0.0;
+    __syncwarp();
+    if (lane == 0) {
+        sm_acc[warp][8] = ws;
+        sm_acc[warp][9] = w.inner;
+        sm_acc[warp][10] = (double)n_max;
+        sm_acc[warp][11] = (double)n_base;
+    }
+    __syncthreads();
+    if (threadIdx.x < 16) {
+        double v = 0;
+        for (int k = 0; k < kSmallWarps; k++) v += sm_acc[k][threadIdx.x];
+        D.B.block_sums[(size_t)blockIdx.x * 16 + threadIdx.x] = v;
+    }
+    level_finish<kSmallThreads>(D.B, gridDim.x);
+}
+
 // Persistent grid of the phase kernel: the CTAs that are resident at once (occupancy x SMs),
 // at most the grid the partial-sum buffer was sized for.
 // Dynamic shared memory of a phase-kernel instantiation: the staged R_tau rows of the FP32
@@ -1680,6 +1949,16 @@ cudaError_t sample_level_t(const OuterLevel<RT>& L, OuterBuffers& B, TraceRec* t
     DevLevel<RT> D;
     D.L = L;
     D.B = B;
+    if constexpr (KIND != KIND_USER && KIND != KIND_PF_PATHS) {
+        if (!L.no_small && level_is_small(L, KIND, PREC, B)) {
+            const uint64_t ctas = (L.M + kSmallWarps - 1) / kSmallWarps;
+            const int grid = (int)(ctas < (uint64_t)B.grid ? ctas : (uint64_t)B.grid);
+            const size_t rows = is_portfolio_kind(KIND) ? kSmallWarps * (size_t)L.ot.Q * sizeof(float2) : 0;
+            k_small<RT, KIND, PREC><<<grid, kSmallThreads, rows, stream>>>(D, (uint32_t)L.M, trace);
+            count_launch();
+            return cudaGetLastError();
+        }
+    }
     for (uint64_t done = 0; done < L.M;) {
         const uint64_t nb = (L.M - done) < B.cap ? (L.M - done) : B.cap;
         D.L.first_index = L.first_index + done;
