@@ -1621,21 +1621,17 @@ int nmlmc_portfolio_full_loss(nmlmc_ctx* c, uint32_t ell, uint64_t first, uint64
     cudaSetDevice(c->device);
     int rc = ensure_portfolio(c);
     if (rc || (rc = alloc_outer(c, n))) return rc;
-    double* d_loss = nullptr;
-    if (dev_malloc(&d_loss, n * sizeof(double)) != cudaSuccess) return set_err(NMLMC_ERR_NOMEM);
     cudaError_t e;
     if (c->cfg.precision == NMLMC_PREC_FP64) {
         OuterLevel<double> L{};
         L.ell = ell; L.M = n; L.first_index = first; L.seed = c->cfg.seed; L.ot = c->dpf64.table;
-        e = outer_full_loss<double>(L, c->cfg.precision, c->ob, d_loss, c->stream);
+        e = outer_full_loss<double>(L, c->cfg.precision, c->ob, host_loss, c->stream);
     } else {
         OuterLevel<float> L{};
         L.ell = ell; L.M = n; L.first_index = first; L.seed = c->cfg.seed; L.ot = c->dpf32.table;
-        e = outer_full_loss<float>(L, c->cfg.precision, c->ob, d_loss, c->stream);
+        e = outer_full_loss<float>(L, c->cfg.precision, c->ob, host_loss, c->stream);
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(host_loss, d_loss, n * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
-    cudaFree(d_loss);
     return cuda_status(e, "full loss");
 }
 

@@ -26,6 +26,8 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "nmlmc_rng.cuh"
+
 namespace nmlmc {
 
 // Packed option record of the FP32 path: 32 bytes, read with one 256-bit load.
@@ -86,6 +88,29 @@ __device__ __forceinline__ float norm_cdf_fast(float x) {
     return x >= 0.f ? 1.0f - h : h;
 }
 
+// Phi of two arguments, the polynomial arithmetic two at a time (f32x2): both components equal to
+// norm_cdf_fast's.
+__device__ __forceinline__ F2 norm_cdf_fast2(F2 x) {
+    const float xa = f2_lo(x), xb = f2_hi(x);
+    const F2 one = f2(1.0f, 1.0f);
+    const F2 d = f2_fma(f2(fabsf(xa), fabsf(xb)), f2(0.35355339f, 0.35355339f), one);
+    const F2 t = f2(rcp_sfu(f2_lo(d)), rcp_sfu(f2_hi(d)));
+    F2 p = f2_fma(t, f2(0.24651730f, 0.24651730f), f2(-1.18611491f, -1.18611491f));
+    p = f2_fma(t, p, f2(2.14747453f, 2.14747453f));
+    p = f2_fma(t, p, f2(-1.63775313f, -1.63775313f));
+    p = f2_fma(t, p, f2(0.40232158f, 0.40232158f));
+    p = f2_fma(t, p, f2(-0.26875687f, -0.26875687f));
+    p = f2_fma(t, p, f2(0.13963005f, 0.13963005f));
+    p = f2_fma(t, p, f2(0.53970063f, 0.53970063f));
+    p = f2_fma(t, p, f2(1.44272923f, 1.44272923f));
+    p = f2_fma(t, p, f2(-2.82574821f, -2.82574821f));
+    const F2 q = f2_fma(x, f2_mul(x, f2(-0.72134751f, -0.72134751f)), p);     // -|x| (|x| c) = x (x (-c))
+    const F2 e = f2(ex2_sfu(f2_lo(q)), ex2_sfu(f2_hi(q)));
+    const F2 h = f2_mul(t, e);
+    const F2 u = f2_fma(h, f2(-1.0f, -1.0f), one);
+    return f2(xa >= 0.f ? f2_lo(u) : f2_lo(h), xb >= 0.f ? f2_hi(u) : f2_hi(h));
+}
+
 // loss_i(R) of one option (see the header comment); lnR = ln R of its stock at this outer sample.
 __device__ __forceinline__ float option_loss_fast(const FastOption& o, float R, float lnR) {
     const float d1 = (lnR + o.c1) * o.inv_s;           // m d1
@@ -93,6 +118,15 @@ __device__ __forceinline__ float option_loss_fast(const FastOption& o, float R, 
     const float n1 = norm_cdf_fast(d1), n2 = norm_cdf_fast(d2);
     const float v = fmaf(o.wR * R, n1, fmaf(o.wK, n2, o.wV0));
     return fmaf(o.cv, R, v);
+}
+
+// The record's loss without a control variate (cv = 0) at two outer samples, both equal to
+// option_loss_fast's.
+__device__ __forceinline__ F2 option_loss_fast2(const FastOption& o, F2 R, F2 lnR) {
+    const F2 d1 = f2_mul(f2_add(lnR, f2(o.c1, o.c1)), f2(o.inv_s, o.inv_s));
+    const F2 d2 = f2_add(d1, f2(-o.s, -o.s));
+    const F2 n1 = norm_cdf_fast2(d1), n2 = norm_cdf_fast2(d2);
+    return f2_fma(f2_mul(f2(o.wR, o.wR), R), n1, f2_fma(f2(o.wK, o.wK), n2, f2(o.wV0, o.wV0)));
 }
 
 // The same loss from an alias column: m d1 as above, m s = 1 / (m inv_s) from the SFU estimate

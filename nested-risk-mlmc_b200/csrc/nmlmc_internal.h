@@ -121,10 +121,10 @@ cudaError_t outer_sample_level(const OuterLevel<RT>& L, int kind, int prec, Oute
 // Zeroes the level's result: for levels without outer samples, which launch nothing.
 cudaError_t outer_level_begin(OuterBuffers& B, cudaStream_t stream);
 
-// Portfolio loss sweep L(Y) over all options (K-quantile precompute).
+// Portfolio loss sweep L(Y) over all options (K-quantile precompute) into a host array; the copies
+// are queued on the stream.
 template <class RT>
-cudaError_t outer_full_loss(const OuterLevel<RT>& L, int prec, OuterBuffers& B, double* d_loss,
-                            cudaStream_t stream);
+cudaError_t outer_full_loss(const OuterLevel<RT>& L, int prec, OuterBuffers& B, double* host_loss, cudaStream_t stream);
 
 // ---- path-simulated loss and its adjoint (nmlmc_adjoint.cu) --------------------------------
 constexpr uint32_t kAdjMaxTile = 64;     // outer samples per CTA of the path kernels

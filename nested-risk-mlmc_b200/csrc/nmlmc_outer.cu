@@ -80,44 +80,49 @@ __global__ void k_full_loss(DevLevel<RT> D, uint32_t nb, double* loss) {
     }
 }
 
-// FP32 sweep of the packed option table: a CTA takes a tile of kLossTile outer samples (their
-// R and ln R rows in shared memory) and streams the table once per tile, so every 32-byte
-// record fetched from L2/HBM feeds kLossTile Black-Scholes evaluations.  Per-thread partial sums
-// are float (each thread adds P/256 options), combined in double across the CTA.
-constexpr int kLossTile = 32;
-
+// FP32 sweep of the packed option table: a CTA takes a tile of TILE outer samples and streams the
+// table once per tile, so every 32-byte record fetched from L2/HBM feeds TILE Black-Scholes
+// evaluations.  Two outer samples share each instruction (f32x2); their R and ln R sit in shared
+// memory as one 16-byte entry per stock (R_o, R_o+1, ln R_o, ln R_o+1), rows one entry longer than
+// the tile so that the lanes' random stocks spread over the banks.  Per-thread partial sums are
+// float (each thread adds P/256 options in table order), combined in double across the CTA, so the
+// tile's length changes no result.  Bound by the four SFU operations of an evaluation (8 cycles per
+// warp and SM).
+template <int TILE>
 __global__ void __launch_bounds__(kTile) k_full_loss_fast(DevLevel<float> D, uint32_t nb, double* loss) {
-    extern __shared__ float sm_rows[];   // R[kLossTile][Q], lnR[kLossTile][Q]
-    __shared__ double red[kWarps][kLossTile];
+    constexpr int H = TILE / 2;
+    extern __shared__ float4 sm_rows[];  // [Q][H + 1]
+    __shared__ double red[kWarps][TILE];
     const OptionTable<float>& ot = D.L.ot;
     const uint32_t Q = ot.Q, P = ot.P;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    float* sR = sm_rows;
-    float* slnR = sm_rows + (size_t)kLossTile * Q;
     const float2* Rt = reinterpret_cast<const float2*>(D.B.Rt);     // (R, ln R) per stock
-    const uint32_t ntiles = (nb + kLossTile - 1) / kLossTile;
+    const uint32_t ntiles = (nb + TILE - 1) / TILE;
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const uint32_t o0 = tile * kLossTile;
-        const uint32_t n_here = (nb - o0) < (uint32_t)kLossTile ? (nb - o0) : (uint32_t)kLossTile;
-        for (uint32_t k = t; k < (uint32_t)kLossTile * Q; k += blockDim.x) {
-            const uint32_t o = k / Q;
-            const float2 R = o < n_here ? Rt[(size_t)(o0 + o) * Q + (k - o * Q)] : make_float2(1.0f, 0.0f);
-            sR[k] = R.x;
-            slnR[k] = R.y;
+        const uint32_t o0 = tile * TILE;
+        const uint32_t n_here = (nb - o0) < (uint32_t)TILE ? (nb - o0) : (uint32_t)TILE;
+        for (uint32_t k = t; k < (uint32_t)H * Q; k += blockDim.x) {
+            const uint32_t o = k / Q, q = k - o * Q;
+            const float2 a = 2 * o < n_here ? Rt[(size_t)(o0 + 2 * o) * Q + q] : make_float2(1.0f, 0.0f);
+            const float2 b = 2 * o + 1 < n_here ? Rt[(size_t)(o0 + 2 * o + 1) * Q + q] : make_float2(1.0f, 0.0f);
+            sm_rows[(size_t)q * (H + 1) + o] = make_float4(a.x, b.x, a.y, b.y);
         }
         __syncthreads();
-        float acc[kLossTile];
+        F2 acc[H];
 #pragma unroll
-        for (int o = 0; o < kLossTile; o++) acc[o] = 0.f;
+        for (int o = 0; o < H; o++) acc[o] = f2(0.f, 0.f);
         for (uint32_t j = t; j < P; j += blockDim.x) {
-            const FastOption op = ot.fast[j];     // full-loss records: no control variate
-            const uint32_t st = op.stock;
+            const FastOption op = load_record_l1(ot.fast + j);     // full-loss records: no control variate
+            const float4* row = sm_rows + (size_t)op.stock * (H + 1);
 #pragma unroll
-            for (int o = 0; o < kLossTile; o++) acc[o] += option_loss_fast(op, sR[o * Q + st], slnR[o * Q + st]);
+            for (int o = 0; o < H; o++) {
+                const float4 r = row[o];
+                acc[o] = f2_add(acc[o], option_loss_fast2(op, f2(r.x, r.y), f2(r.z, r.w)));
+            }
         }
 #pragma unroll
-        for (int o = 0; o < kLossTile; o++) {
-            double v = (double)acc[o];
+        for (int o = 0; o < TILE; o++) {
+            double v = (double)((o & 1) ? f2_hi(acc[o / 2]) : f2_lo(acc[o / 2]));
             for (int m = 16; m > 0; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
             if (lane == 0) red[warp][o] = v;
         }
@@ -131,46 +136,65 @@ __global__ void __launch_bounds__(kTile) k_full_loss_fast(DevLevel<float> D, uin
     }
 }
 
+template <int TILE>
+static cudaError_t launch_full_loss_fast(const DevLevel<float>& D, uint32_t nb, double* loss, cudaStream_t stream) {
+    const size_t smem = (size_t)D.L.ot.Q * (TILE / 2 + 1) * sizeof(float4);
+    if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(k_full_loss_fast<TILE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    const uint32_t tiles = (nb + TILE - 1) / TILE;
+    k_full_loss_fast<TILE><<<tiles < (uint32_t)D.B.grid * 2 ? tiles : D.B.grid * 2, kTile, smem, stream>>>(D, nb, loss);
+    count_launch();
+    return cudaGetLastError();
+}
+
+// Losses of outer samples L.first_index .. + L.M - 1 into the host's array.  A batch's losses sit in
+// the item lists, which the sweep does not use (two doubles per outer sample), so a call allocates
+// nothing (a device allocation and its release took up to 0.8 ms of a call).
 template <class RT>
-cudaError_t outer_full_loss(const OuterLevel<RT>& L, int prec, OuterBuffers& B, double* d_loss,
-                            cudaStream_t stream) {
+cudaError_t outer_full_loss(const OuterLevel<RT>& L, int prec, OuterBuffers& B, double* host_loss, cudaStream_t stream) {
     DevLevel<RT> D;
     D.L = L;
     D.B = B;
+    double* loss = reinterpret_cast<double*>(B.lists);
     for (uint64_t done = 0; done < L.M;) {
         const uint64_t nb = (L.M - done) < B.cap ? (L.M - done) : B.cap;
         D.L.first_index = L.first_index + done;
         int og = (int)((nb + kTile - 1) / kTile);
         if (og > B.grid) og = B.grid;
         if (og < 1) og = 1;
+        const uint32_t n = (uint32_t)nb;
+        cudaError_t e = cudaSuccess;
         if (prec == PREC_FP64) {
             if constexpr (sizeof(RT) == 8) {
-                k_outer<RT, KIND_PORTFOLIO, PREC_FP64><<<og, kTile, 0, stream>>>(D, (uint32_t)nb, 0);
-                k_full_loss<RT, PREC_FP64><<<B.grid, kTile, 0, stream>>>(D, (uint32_t)nb, d_loss + done);
+                k_outer<RT, KIND_PORTFOLIO, PREC_FP64><<<og, kTile, 0, stream>>>(D, n, 0);
+                k_full_loss<RT, PREC_FP64><<<B.grid, kTile, 0, stream>>>(D, n, loss);
+                count_launch(2);
             }
         } else {
             if constexpr (sizeof(RT) == 4) {
+                if (prec == PREC_FP32) k_outer<RT, KIND_PORTFOLIO, PREC_FP32><<<og, kTile, 0, stream>>>(D, n, 0);
+                else k_outer<RT, KIND_PORTFOLIO, PREC_REF32><<<og, kTile, 0, stream>>>(D, n, 0);
+                count_launch();
                 if (prec == PREC_FP32 && L.ot.fast) {
-                    k_outer<RT, KIND_PORTFOLIO, PREC_FP32><<<og, kTile, 0, stream>>>(D, (uint32_t)nb, 0);
-                    const size_t smem = (size_t)2 * kLossTile * L.ot.Q * sizeof(float);
-                    if (smem > 200 * 1024) return cudaErrorInvalidValue;   // Q above 800 stocks
-                    if (smem > 48 * 1024) {
-                        cudaError_t ea = cudaFuncSetAttribute(k_full_loss_fast, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                        if (ea != cudaSuccess) return ea;
-                    }
-                    const int lg = (int)((nb + kLossTile - 1) / kLossTile) < B.grid ? (int)((nb + kLossTile - 1) / kLossTile) : B.grid;
-                    k_full_loss_fast<<<lg, kTile, smem, stream>>>(D, (uint32_t)nb, d_loss + done);
-                    count_launch(2);
-                } else if (prec == PREC_FP32) {
-                    k_outer<RT, KIND_PORTFOLIO, PREC_FP32><<<og, kTile, 0, stream>>>(D, (uint32_t)nb, 0);
-                    k_full_loss<RT, PREC_FP32><<<B.grid, kTile, 0, stream>>>(D, (uint32_t)nb, d_loss + done);
+                    if (L.ot.Q > 800) return cudaErrorInvalidValue;      // rows beyond the shared memory
+                    // Tiles: long ones read the table less often, short ones fill the chip at few outer
+                    // samples.  10^5 / 3 10^4 / 1.2 10^4 / 5000 / 1000 outer samples (10^4 to 10^5
+                    // options), us: tile 16 1535 / 492 / 991 / 1085 / 520, tile 8 1578 / 518 / 931 / 948 / 378,
+                    // tile 4 1647 / 530 / 969 / 865 / 306
+                    if (n >= 20000) e = launch_full_loss_fast<16>(D, n, loss, stream);
+                    else if (n >= 8000) e = launch_full_loss_fast<8>(D, n, loss, stream);
+                    else e = launch_full_loss_fast<4>(D, n, loss, stream);
                 } else {
-                    k_outer<RT, KIND_PORTFOLIO, PREC_REF32><<<og, kTile, 0, stream>>>(D, (uint32_t)nb, 0);
-                    k_full_loss<RT, PREC_REF32><<<B.grid, kTile, 0, stream>>>(D, (uint32_t)nb, d_loss + done);
+                    if (prec == PREC_FP32) k_full_loss<RT, PREC_FP32><<<B.grid, kTile, 0, stream>>>(D, n, loss);
+                    else k_full_loss<RT, PREC_REF32><<<B.grid, kTile, 0, stream>>>(D, n, loss);
+                    count_launch();
                 }
             }
         }
-        cudaError_t e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaMemcpyAsync(host_loss + done, loss, nb * sizeof(double), cudaMemcpyDeviceToHost, stream);
         if (e != cudaSuccess) return e;
         done += nb;
     }

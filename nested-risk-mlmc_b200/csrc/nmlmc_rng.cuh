@@ -120,6 +120,8 @@ __device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
     return r;
 }
+// The assembler fuses an f2_mul with an f2_add of its result: where the product has to be rounded on
+// its own, the sum is two scalar __fadd_rn.
 __device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
     F2 r;
     asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
