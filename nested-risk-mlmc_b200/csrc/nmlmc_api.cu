@@ -120,6 +120,8 @@ struct DevPortfolio {
        *delta_coalesce = nullptr;
     uint32_t* stock_ind = nullptr;
     int8_t* type = nullptr;
+    RefOption<RT>* ref = nullptr;     // per-option constants in reference arithmetic
+    uint32_t* guide = nullptr;        // guide tables of the CORE layout's inverse-CDF draw
     FastOption* fast = nullptr;       // packed records of the FP32 path
     FastOption* fast_s = nullptr;     // the same, scaled by 1 / sampling probability
     FastColumn* fast_col = nullptr;   // sampler records fused with the alias table
@@ -269,7 +271,7 @@ template <class RT>
 void free_dev_portfolio(DevPortfolio<RT>& d) {
     dfree(d.strike); dfree(d.maturity); dfree(d.start); dfree(d.w); dfree(d.prob); dfree(d.W_est);
     dfree(d.cdf); dfree(d.S0); dfree(d.mu); dfree(d.sigma); dfree(d.delta_coalesce);
-    dfree(d.stock_ind); dfree(d.type); dfree(d.fast); dfree(d.fast_s); dfree(d.fast_col); dfree(d.alias); dfree(d.phat);
+    dfree(d.stock_ind); dfree(d.type); dfree(d.ref); dfree(d.guide); dfree(d.fast); dfree(d.fast_s); dfree(d.fast_col); dfree(d.alias); dfree(d.phat);
     d.table = OptionTable<RT>{};
 }
 
@@ -390,6 +392,28 @@ int build_dev_portfolio(nmlmc_ctx* c, DevPortfolio<RT>& d) {
     t.dt_h0inv = h.dt_h0inv; t.dt_beta = h.dt_beta; t.dt_prob_expo = (RT)h.dt_prob_expo;
     t.use_coarse_delta_cv = h.use_coarse_delta_cv; t.use_antithetic_risk = h.use_antithetic_risk;
     t.use_milstein = h.use_milstein;
+    t.guide = nullptr;
+    if (h.subsample == SUB_RANDOM) {
+        // guide_n = m_n buckets per method; entry k is the last option whose CDF value lies in a
+        // bucket before k (0 if none does), entry n closes the last bucket
+        std::vector<uint32_t> guide;
+        for (int m = 0; m < 3; m++) {
+            const uint32_t n = h.m_n[m];
+            t.guide_off[m] = (uint32_t)guide.size();
+            t.guide_n[m] = n;
+            t.guide_scale[m] = n ? (RT)n / cprob[m] : (RT)0;
+            uint32_t i = 0;                               // options whose bucket is before k
+            for (uint32_t k = 0; n && k <= n; k++) {
+                while (i < n && (k == n || guide_bucket<RT>(cdf[m_off[m] + i], t.guide_scale[m], n) < k)) i++;
+                guide.push_back(i ? i - 1 : 0);
+            }
+        }
+        if ((rc = upload(d.guide, guide))) return rc;
+        t.guide = d.guide;
+    }
+    if (dev_malloc(&d.ref, P * sizeof(RefOption<RT>)) != cudaSuccess) return set_err(NMLMC_ERR_NOMEM);
+    NM_CUDA(launch_ref_records(t, d.ref, c->stream), "option constants");
+    t.ref = d.ref;
     t.fast = nullptr;
     t.fast_s = nullptr;
     t.fast_col = nullptr;

@@ -43,6 +43,22 @@ enum Method : int { METHOD_BS = 0, METHOD_EXACT = 1, METHOD_UNBIASED = 2 };
 // draw above it stops the call with NMLMC_ERR_LIMIT instead of running unbounded.
 constexpr uint64_t kMaxPathSteps = 1ull << 24;
 
+// Black-Scholes constants of one option in the reference's real_t evaluation order (REF32 / FP64
+// tables; k_ref_records): what calc_bs, the discount and the delta control variate of an inner
+// sample recompute from the option alone, evaluated once with the same device functions, so an
+// inner sample's value is unchanged.  It is left with one log, two erfc and the divisions by
+// R-dependent values: three erfc, two logs, two exponentials and four square roots were evaluated
+// before, from ten scattered table reads (now one record).
+template <class RT>
+struct __align__(16) RefOption {
+    RT strike, v2, v3;    // v2 = (r + sigma^2 / 2) (T - tau), v3 = sigma sqrt(T - tau)
+    RT kdisc;             // type K e^{-r (T - tau)}
+    RT w, start, derv;    // derv = w Delta_BS(S0, T)
+    RT S0, prob, disc;    // prob: the CORE layout's sampling probability; disc = e^{-r tau} or 1
+    uint32_t stock;
+    int32_t type;
+};
+
 // Option table in HBM, structure of arrays.  Options are grouped by compute method
 // (portfolio::data::options[3], portfolio_sampler.cpp:62-92): method m occupies
 // [m_off[m], m_off[m] + m_n[m]) and its CDF restarts at 0.
@@ -62,6 +78,12 @@ struct OptionTable {
     const RT* mu;
     const RT* sigma;
     const RT* delta_coalesce;
+    const RefOption<RT>* ref;        // per-option constants in reference arithmetic
+    // guide table of the CORE layout's inverse-CDF draw, per method m (Subsampling::Random): entry
+    // guide_off[m] + k brackets the option of a draw in bucket k (rand_int_cdf, nmlmc_core.cu)
+    const uint32_t* guide;
+    uint32_t guide_off[3], guide_n[3];
+    RT guide_scale[3];
     const struct FastOption* fast;   // FP32 path: packed records (nmlmc_bs.cuh), else nullptr
     const struct FastOption* fast_s; // the same records scaled by 1 / (sampling probability)
     const uint2* alias;              // OUTER Subsampling::Random: alias table {threshold, alias}
@@ -156,10 +178,30 @@ __device__ __forceinline__ RT calc_bs_ref(int type, RT S0, RT strike, RT r, RT t
     return xsub(a, b);
 }
 
+// The bucket of a CDF value in its method's guide table: non-decreasing in x.
+template <class RT>
+__host__ __device__ __forceinline__ uint32_t guide_bucket(RT x, RT scale, uint32_t n) {
+    const RT b = x * scale;
+    return b < (RT)n ? (uint32_t)b : n - 1;
+}
+
 template <class RT>
 __device__ __forceinline__ RT calc_delta_ref(int type, RT S0, RT strike, RT r, RT t, RT sigma) {  // :152-160
     RT d1 = bs_d1_ref(S0, strike, r, t, sigma);
     return xsub(norm_cdf_ref(d1), (RT)(type == -1 ? 1 : 0));
+}
+
+// option_diff_from_blackscholes with the delta control variate (portfolio_sampler.cpp:186-210,
+// 453-468) at the stock value R, from the option's constants.
+template <class RT>
+__device__ __forceinline__ RT ref_option_value(const RefOption<RT>& o, RT R, bool use_delta_cv) {
+    const RT d1 = xdiv(xadd(xlog(xdiv(R, o.strike)), o.v2), o.v3);
+    const RT d2 = xsub(d1, o.v3);
+    const RT mod = (RT)o.type;
+    const RT a = xmul(xmul(mod, R), norm_cdf_ref(xmul(mod, d1)));
+    const RT b = xmul(o.kdisc, norm_cdf_ref(xmul(mod, d2)));
+    const RT val = xmul(o.w, xsub(o.start, xmul(o.disc, xsub(a, b))));
+    return use_delta_cv ? xadd(val, xmul(xsub(R, o.S0), o.derv)) : val;
 }
 #endif  // __CUDACC__
 

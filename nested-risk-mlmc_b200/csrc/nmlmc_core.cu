@@ -118,18 +118,25 @@ __device__ __forceinline__ RT portfolio_bs_value(const OptionTable<RT>& ot, cons
                                                  double& work) {
     // sample_inner_bs (portfolio_sampler.cpp:453-468) -> option_diff_from_blackscholes (186-200)
     work += (double)ot.W_est[j];
-    uint32_t s = ot.stock_ind[j];
-    int type = ot.type[j];
-    RT sigma = ot.sigma[s];
-    RT bs = calc_bs_ref<RT>(type, Rt[s], ot.strike[j], ot.r, xsub(ot.maturity[j], ot.tau), sigma);
-    RT finish = ot.discount ? xmul(xexp(xmul(-ot.r, ot.tau)), bs) : bs;
-    RT val = xmul(ot.w[j], xsub(ot.start[j], finish));
-    RT cv = (RT)0;
-    if (ot.use_delta_cv) {
-        RT derv = xmul(ot.w[j], calc_delta_ref<RT>(type, ot.S0[s], ot.strike[j], ot.r, ot.maturity[j], sigma));
-        cv = xmul(xsub(Rt[s], ot.S0[s]), derv);
+    const RefOption<RT> o = ot.ref[j];
+    return ref_option_value<RT>(o, Rt[o.stock], ot.use_delta_cv != 0);
+}
+
+// rand_int_cdf (common.hpp:160-176) over method m's CDF: the last option whose CDF value is at
+// most uu (the first one if none is).  The reference halves [0, n) with log2 n dependent reads (14
+// for 10^4 options); the guide table's two entries of the draw's bucket bracket the same option to
+// about two, so one or two reads remain.
+template <class RT>
+__device__ __forceinline__ uint32_t cdf_index(const OptionTable<RT>& ot, uint32_t m, RT uu) {
+    const uint32_t* g = ot.guide + ot.guide_off[m];
+    const uint32_t k = guide_bucket<RT>(uu, ot.guide_scale[m], ot.guide_n[m]);
+    const RT* cdf = ot.cdf + ot.m_off[m];
+    uint32_t lo = g[k], hi = g[k + 1];                   // the option is in [lo, hi]
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) / 2;
+        if (uu < cdf[mid]) hi = mid - 1; else lo = mid;
     }
-    return xadd(val, cv);
+    return lo;
 }
 
 template <class RT>
@@ -187,17 +194,9 @@ __device__ __forceinline__ uint32_t pick_option(const OptionTable<RT>& ot, uint3
         prob = ot.inv_count_prob;
         return off + (uint32_t)(xceil(xmul(u, (RT)nm)) - (RT)1);
     }
-    const RT uu = xmul(u, ot.compute_prob[m]);
-    uint32_t pos0 = 0, pos1 = nm;
-    if (nm > 1) {
-        const uint32_t steps = 32 - __clz(nm - 1);
-        for (uint32_t t = 0; t < steps; t++) {
-            const uint32_t mid = (pos0 + pos1) / 2;
-            if (mid > 0 && uu < ot.cdf[off + mid]) pos1 = mid; else pos0 = mid;
-        }
-    }
-    prob = xdiv(ot.prob[off + pos0], ot.prob_norm);
-    return off + pos0;
+    const uint32_t j = off + cdf_index<RT>(ot, m, xmul(u, ot.compute_prob[m]));
+    prob = ot.ref[j].prob;
+    return j;
 }
 
 __device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, uint32_t n) {   // 32 when absent
@@ -426,18 +425,8 @@ __device__ void core_phase(CoreCtx<RT, KIND>& c, uint64_t count, bool want_s2, d
                 idx = (uint32_t)(xceil(xmul(u, (RT)c.ot.P)) - (RT)1);
                 prob = c.ot.inv_count_prob;
             } else {
-                RT uu = xmul(u, c.ot.compute_prob0);
-                // rand_int_cdf (common.hpp:160-176)
-                uint32_t pos0 = 0, pos1 = c.ot.P;
-                if (c.ot.P > 1) {
-                    uint32_t steps = 32 - __clz(c.ot.P - 1);
-                    for (uint32_t s = 0; s < steps; s++) {
-                        uint32_t mid = (pos0 + pos1) / 2;
-                        if (mid > 0 && uu < c.ot.cdf[mid]) pos1 = mid; else pos0 = mid;
-                    }
-                }
-                idx = pos0;
-                prob = xdiv(c.ot.prob[idx], c.ot.prob_norm);
+                idx = cdf_index<RT>(c.ot, METHOD_BS, xmul(u, c.ot.compute_prob0));
+                prob = c.ot.ref[idx].prob;
             }
             RT v = portfolio_bs_value<RT>(c.ot, c.Rt, idx, w);
             RT d = xdiv(v, prob);
@@ -675,6 +664,43 @@ __global__ void core_reduce_kernel(uint32_t cores, const double* in_sums, const 
         for (int j = 0; j < 10; j++) out_sums[j] = sd[0][j];
         for (int j = 0; j < 6; j++) out_stats[j] = su[0][j];
     }
+}
+
+template <class RT>
+__global__ void __launch_bounds__(128) k_ref_records(OptionTable<RT> t, RefOption<RT>* out) {
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < t.P; j += gridDim.x * blockDim.x) {
+        const uint32_t s = t.stock_ind[j];
+        const int type = t.type[j];
+        const RT K = t.strike[j], sg = t.sigma[s], Tr = xsub(t.maturity[j], t.tau);
+        RefOption<RT> o;
+        o.strike = K;
+        o.v2 = to_rt<RT>(__dmul_rn(__dadd_rn((double)t.r, __ddiv_rn((double)xmul(sg, sg), 2.0)), (double)Tr));   // bs_d1_ref
+        o.v3 = xmul(sg, xsqrt(Tr));
+        o.kdisc = xmul(xmul((RT)type, K), xexp(xmul(-t.r, Tr)));
+        o.w = t.w[j];
+        o.start = t.start[j];
+        o.derv = xmul(t.w[j], calc_delta_ref<RT>(type, t.S0[s], K, t.r, t.maturity[j], sg));
+        o.S0 = t.S0[s];
+        o.prob = xdiv(t.prob[j], t.prob_norm);
+        o.disc = t.discount ? xexp(xmul(-t.r, t.tau)) : (RT)1;
+        o.stock = s;
+        o.type = type;
+        out[j] = o;
+    }
+}
+
+template <class RT>
+static cudaError_t launch_ref_records_t(const OptionTable<RT>& t, RefOption<RT>* out, cudaStream_t stream) {
+    const uint32_t blocks = (t.P + 127) / 128;
+    k_ref_records<RT><<<blocks < 2048 ? blocks : 2048, 128, 0, stream>>>(t, out);
+    count_launch();
+    return cudaGetLastError();
+}
+cudaError_t launch_ref_records(const OptionTable<float>& t, RefOption<float>* out, cudaStream_t stream) {
+    return launch_ref_records_t<float>(t, out, stream);
+}
+cudaError_t launch_ref_records(const OptionTable<double>& t, RefOption<double>* out, cudaStream_t stream) {
+    return launch_ref_records_t<double>(t, out, stream);
 }
 
 template <class RT>

@@ -33,6 +33,9 @@ cudaError_t launch_core(const CoreLaunch<float>& L, int kind, CoreStream* states
 cudaError_t launch_core(const CoreLaunch<double>& L, int kind, CoreStream* states, double* part_sums,
                         uint64_t* part_stats, double* out_sums, uint64_t* out_stats, TraceRec* trace,
                         cudaStream_t stream);
+// Per-option constants of the reference-arithmetic tables (RefOption), P records.
+cudaError_t launch_ref_records(const OptionTable<float>& t, RefOption<float>* out, cudaStream_t stream);
+cudaError_t launch_ref_records(const OptionTable<double>& t, RefOption<double>* out, cudaStream_t stream);
 
 // ---- OUTER layout (batched) ----------------------------------------------------------------
 enum Prec : int { PREC_REF32 = 0, PREC_FP64 = 1, PREC_FP32 = 2 };

@@ -70,10 +70,8 @@ __global__ void k_full_loss(DevLevel<RT> D, uint32_t nb, double* loss) {
         const RT* Rrow = reinterpret_cast<const RT*>(D.B.Rt) + (size_t)i * ot.Q * RS;
         double s = 0;
         for (uint32_t j = lane; j < ot.P; j += 32) {
-            uint32_t st = ot.stock_ind[j];
-            RT bs = calc_bs_ref<RT>(ot.type[j], Rrow[st * RS], ot.strike[j], ot.r, xsub(ot.maturity[j], ot.tau), ot.sigma[st]);
-            RT finish = ot.discount ? xmul(xexp(xmul(-ot.r, ot.tau)), bs) : bs;
-            s += (double)xmul(ot.w[j], xsub(ot.start[j], finish));
+            const RefOption<RT> o = ot.ref[j];
+            s += (double)ref_option_value<RT>(o, Rrow[o.stock * RS], false);
         }
         s = warp_sum(s);
         if (lane == 0) loss[i] = s;

@@ -271,18 +271,8 @@ template <int PREC> struct RStride { static constexpr uint32_t v = PREC == PREC_
 
 template <class RT, uint32_t RS>
 __device__ __forceinline__ RT pf_value(const OptionTable<RT>& ot, const RT* Rrow, uint32_t j) {
-    uint32_t s = ot.stock_ind[j];
-    int type = ot.type[j];
-    RT sigma = ot.sigma[s];
-    const RT R = Rrow[s * RS];
-    RT bs = calc_bs_ref<RT>(type, R, ot.strike[j], ot.r, xsub(ot.maturity[j], ot.tau), sigma);
-    RT finish = ot.discount ? xmul(xexp(xmul(-ot.r, ot.tau)), bs) : bs;
-    RT val = xmul(ot.w[j], xsub(ot.start[j], finish));
-    if (ot.use_delta_cv) {
-        RT derv = xmul(ot.w[j], calc_delta_ref<RT>(type, ot.S0[s], ot.strike[j], ot.r, ot.maturity[j], sigma));
-        val = xadd(val, xmul(xsub(R, ot.S0[s]), derv));
-    }
-    return val;
+    const RefOption<RT> o = ot.ref[j];
+    return ref_option_value<RT>(o, Rrow[o.stock * RS], ot.use_delta_cv != 0);
 }
 
 // Option index of one inner sample from one 64-bit value of the OUTER layout (the draw of
