@@ -166,10 +166,9 @@ struct nmlmc_ctx {
     DevPortfolio<double> dpf64;
     // CORE layout
     CoreStream* d_states = nullptr;
-    double* d_part_sums = nullptr;
-    uint64_t* d_part_stats = nullptr;
-    double* d_out_sums = nullptr;     // [10]
-    uint64_t* d_out_stats = nullptr;  // [6]
+    CoreStream* d_states_next = nullptr;
+    uint64_t* d_core_part = nullptr;  // per-CTA partial results
+    uint32_t* d_core_counts = nullptr;
     uint32_t states_cores = 0;
     // OUTER layout
     OuterBuffers ob{};
@@ -527,14 +526,17 @@ CountParams count_params(const nmlmc_config& cfg, uint32_t ell) {
 int alloc_core(nmlmc_ctx* c) {
     const uint32_t cores = c->cfg.cores;
     if (c->states_cores == cores && c->d_states) return NMLMC_OK;
-    dfree(c->d_states); dfree(c->d_part_sums); dfree(c->d_part_stats);
+    dfree(c->d_states); dfree(c->d_states_next); dfree(c->d_core_part); dfree(c->d_core_counts);
     c->states_cores = 0;
+    const size_t nc = core_counts(cores) * sizeof(uint32_t);
     if (dev_malloc(&c->d_states, (size_t)cores * 2 * sizeof(CoreStream)) != cudaSuccess ||
-        dev_malloc(&c->d_part_sums, (size_t)cores * 10 * sizeof(double)) != cudaSuccess ||
-        dev_malloc(&c->d_part_stats, (size_t)cores * 6 * sizeof(uint64_t)) != cudaSuccess) {
-        dfree(c->d_states); dfree(c->d_part_sums); dfree(c->d_part_stats);
+        dev_malloc(&c->d_states_next, (size_t)cores * 2 * sizeof(CoreStream)) != cudaSuccess ||
+        dev_malloc(&c->d_core_part, core_part_words(cores) * sizeof(uint64_t)) != cudaSuccess ||
+        dev_malloc(&c->d_core_counts, nc) != cudaSuccess) {
+        dfree(c->d_states); dfree(c->d_states_next); dfree(c->d_core_part); dfree(c->d_core_counts);
         return set_err(NMLMC_ERR_NOMEM);
     }
+    NM_CUDA(cudaMemset(c->d_core_counts, 0, nc), "memset");
     c->states_cores = cores;
     return NMLMC_OK;
 }
@@ -650,11 +652,10 @@ int sample_core(nmlmc_ctx* c, uint32_t ell, uint64_t M, nmlmc_level_result* out)
     }
     TraceRec* tr = c->trace_host ? c->d_trace : nullptr;
     NM_CUDA(cudaEventRecord(c->ev0, c->stream), "event");
-    NM_CUDA(launch_core(L, c->kind, c->d_states, c->d_part_sums, c->d_part_stats, c->d_out_sums,
-                        c->d_out_stats, tr, c->stream), "core level kernel");
+    NM_CUDA(launch_core(L, c->kind, c->d_states, c->d_states_next, c->d_core_part, c->d_core_counts,
+                        reinterpret_cast<uint64_t*>(c->h_pin), tr, c->stream), "core level kernel");
+    std::swap(c->d_states, c->d_states_next);
     NM_CUDA(cudaEventRecord(c->ev1, c->stream), "event");
-    NM_CUDA(cudaMemcpyAsync(c->h_pin, c->d_out_sums, 10 * sizeof(double), cudaMemcpyDeviceToHost, c->stream), "d2h");
-    NM_CUDA(cudaMemcpyAsync(c->h_pin + 16, c->d_out_stats, 6 * sizeof(uint64_t), cudaMemcpyDeviceToHost, c->stream), "d2h");
     if (tr) NM_CUDA(cudaMemcpyAsync(c->trace_host, tr, M * sizeof(TraceRec), cudaMemcpyDeviceToHost, c->stream), "d2h");
     NM_CUDA(cudaStreamSynchronize(c->stream), "sync");
     float ms = 0;
@@ -662,7 +663,7 @@ int sample_core(nmlmc_ctx* c, uint32_t ell, uint64_t M, nmlmc_level_result* out)
     for (int j = 0; j < 4; j++) { out->fsums[j] = c->h_pin[j]; out->diffsums[j] = c->h_pin[4 + j]; }
     out->total_work = c->h_pin[8];
     out->M = M;
-    memcpy(out->inner_stats, c->h_pin + 16, 6 * sizeof(uint64_t));
+    memcpy(out->inner_stats, c->h_pin + 10, 6 * sizeof(uint64_t));
     out->seconds = ms * 1e-3;
     c->trace_host = nullptr;
     if (c->h_pin[9] != 0) return set_err(NMLMC_ERR_LIMIT);   // a sample exceeded kMaxPathSteps
@@ -1062,9 +1063,7 @@ int nmlmc_create(nmlmc_ctx** out, int device) {
     c->device = device;
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
-        cudaMallocHost(&c->h_pin, 64 * sizeof(double)) != cudaSuccess ||
-        dev_malloc(&c->d_out_sums, 16 * sizeof(double)) != cudaSuccess ||
-        dev_malloc(&c->d_out_stats, 8 * sizeof(uint64_t)) != cudaSuccess) {
+        cudaMallocHost(&c->h_pin, 64 * sizeof(double)) != cudaSuccess) {
         nmlmc_destroy(c);
         return set_err(NMLMC_ERR_CUDA);
     }
@@ -1078,8 +1077,8 @@ int nmlmc_destroy(nmlmc_ctx* c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     free_dev_portfolio(c->dpf32);
     free_dev_portfolio(c->dpf64);
-    dfree(c->d_states); dfree(c->d_part_sums); dfree(c->d_part_stats);
-    dfree(c->d_out_sums); dfree(c->d_out_stats); dfree(c->d_trace);
+    dfree(c->d_states); dfree(c->d_states_next); dfree(c->d_core_part); dfree(c->d_core_counts);
+    dfree(c->d_trace);
     dfree(c->adj_mem);
     free_outer(c);
     for (cudaEvent_t e : c->pev) cudaEventDestroy(e);

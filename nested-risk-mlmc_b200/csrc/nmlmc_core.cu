@@ -101,6 +101,29 @@ __device__ __forceinline__ void advance_normals(CoreStream& s, const TfKey& k, u
     s.wpos += 2 * pairs;
 }
 
+// The models' outer draws: normal i of a CORE sync stream that draws nothing else, 32 pairs (64
+// outer samples) at a time, one pair per lane — the pair's latency was paid for every outer sample
+// by the whole warp, twice when its second normal was kept.  Warp-uniform i, non-decreasing.
+template <class RT>
+struct OuterNormals {
+    uint64_t base;                                       // first cached pair (~0: none)
+    RT x, y;
+    __device__ __forceinline__ RT get(const TfKey& key, const CoreStream& s, uint64_t i, int lane) {
+        if (s.saved) {
+            if (i == 0) return (RT)s.sval;
+            i -= 1;
+        }
+        const uint64_t p = i >> 1;
+        if (base == ~0ull || p - base >= 32) {
+            base = p;
+            core_pair<RT>(key, s.wpos + 2 * (p + (uint64_t)lane), x, y);
+        }
+        const int src = (int)(p - base);
+        const RT a = __shfl_sync(0xffffffffu, x, src), b = __shfl_sync(0xffffffffu, y, src);
+        return (i & 1) ? b : a;
+    }
+};
+
 // ---- samplers -----------------------------------------------------------------------------
 template <class RT, int KIND>
 struct CoreCtx {
@@ -380,25 +403,56 @@ __device__ void core_phase(CoreCtx<RT, KIND>& c, uint64_t count, bool want_s2, d
     const uint64_t lo = (uint64_t)lane * count / 32, hi = (uint64_t)(lane + 1) * count / 32;
     double a1 = 0, a2 = 0, w = 0;
     if (KIND == KIND_REF_MODEL || KIND == KIND_SHIFT_MODEL) {
-        PhaseNormals<RT> pn;
-        pn.init(c.key, c.inner);
-        for (uint64_t i = lo; i < hi; i++) {
-            RT d;
-            if (KIND == KIND_REF_MODEL) {       // model_sampler.cpp:62-76
-                RT X = pn.get(2 * i), Y2 = pn.get(2 * i + 1);
-                RT a = xadd(xmul(c.mp.stau, c.Y), xmul(c.mp.s1tau, X));
-                RT b = xadd(xmul(c.mp.stau, Y2), xmul(c.mp.s1tau, X));
-                d = xsub(xmul(a, a), xmul(b, b));
-            } else {                            // X = Y + Z
-                d = xadd(c.Y, pn.get(i));
-            }
-            w += 1.0;
-            a1 += (double)d;
-            if (want_s2) a2 += (double)xmul(d, d);
-        }
         const uint64_t per = (KIND == KIND_REF_MODEL) ? 2 : 1;
-        __syncwarp();
-        advance_normals<RT>(c.inner, c.key, per * count);
+        if (!c.inner.saved && !(c.inner.wpos & 1) && (KIND == KIND_REF_MODEL || count % 64 == 0)) {
+            // whole pairs, each one block of the stream: the reference model's sample i is pair i, the
+            // shift model's samples 2p and 2p + 1 share pair p
+            const uint64_t blk = c.inner.wpos >> 1;
+            const uint32_t p0 = (uint32_t)(KIND == KIND_REF_MODEL ? lo : lo / 2), p1 = (uint32_t)(KIND == KIND_REF_MODEL ? hi : hi / 2);
+#pragma unroll 1
+            for (uint32_t p = p0; p < p1; p++) {
+                uint64_t v0, v1;
+                threefry2x64(blk + p, 0, c.key, v0, v1);
+                double dx, dy;
+                boxmuller64(v0, v1, dx, dy);
+                const RT x = to_rt<RT>(dx), y = to_rt<RT>(dy);
+                if (KIND == KIND_REF_MODEL) {
+                    const RT a = xadd(xmul(c.mp.stau, c.Y), xmul(c.mp.s1tau, x));
+                    const RT b = xadd(xmul(c.mp.stau, y), xmul(c.mp.s1tau, x));
+                    const RT d = xsub(xmul(a, a), xmul(b, b));
+                    a1 += (double)d;
+                    if (want_s2) a2 += (double)xmul(d, d);
+                } else {
+                    const RT d0 = xadd(c.Y, x), d1 = xadd(c.Y, y);
+                    a1 += (double)d0;
+                    a1 += (double)d1;
+                    if (want_s2) {
+                        a2 += (double)xmul(d0, d0);
+                        a2 += (double)xmul(d1, d1);
+                    }
+                }
+            }
+            c.inner.wpos += per * count;
+        } else {
+            PhaseNormals<RT> pn;
+            pn.init(c.key, c.inner);
+            for (uint64_t i = lo; i < hi; i++) {
+                RT d;
+                if (KIND == KIND_REF_MODEL) {       // model_sampler.cpp:62-76
+                    RT X = pn.get(2 * i), Y2 = pn.get(2 * i + 1);
+                    RT a = xadd(xmul(c.mp.stau, c.Y), xmul(c.mp.s1tau, X));
+                    RT b = xadd(xmul(c.mp.stau, Y2), xmul(c.mp.s1tau, X));
+                    d = xsub(xmul(a, a), xmul(b, b));
+                } else {                            // X = Y + Z
+                    d = xadd(c.Y, pn.get(i));
+                }
+                a1 += (double)d;
+                if (want_s2) a2 += (double)xmul(d, d);
+            }
+            __syncwarp();
+            advance_normals<RT>(c.inner, c.key, per * count);
+        }
+        w = (double)(hi - lo);
         nrandn += per * count;
     } else if (c.ot.mixed) {
         if constexpr (KIND == KIND_PORTFOLIO) {
@@ -445,18 +499,10 @@ __device__ void core_phase(CoreCtx<RT, KIND>& c, uint64_t count, bool want_s2, d
     work += warp_sum(w);
 }
 
+// Outer draw of the portfolio (the models draw theirs in batches, OuterNormals).
 template <class RT, int KIND>
 __device__ void core_sample_outer(CoreCtx<RT, KIND>& c, uint64_t& nrandn, int lane) {
     __syncwarp();
-    if (KIND != KIND_PORTFOLIO) {                     // model_sampler.cpp:53-55
-        PhaseNormals<RT> pn;
-        pn.init(c.key, c.sync);
-        c.Y = pn.get(0);
-        __syncwarp();
-        advance_normals<RT>(c.sync, c.key, 1);
-        nrandn += 1;
-        return;
-    }
     // portfolio_sampler.cpp:293-311: dW_sys then one normal per stock
     const OptionTable<RT>& ot = c.ot;
     PhaseNormals<RT> pn;
@@ -518,23 +564,18 @@ __device__ uint64_t core_count(CoreCtx<RT, KIND>& c, const CountParams& cp, RT r
     return cur;
 }
 
+// The outer samples of unit (core, sub): results in sums[16] (10 sums, 6 counts), streams stored
+// by the core's last unit.
 template <class RT, int KIND>
-__global__ void __launch_bounds__(256) core_level_kernel(CoreLaunch<RT> L, CoreStream* states,
-                                                         double* out_sums, uint64_t* out_stats,
-                                                         TraceRec* trace) {
-    extern __shared__ unsigned char smem_raw[];
-    const int lane = threadIdx.x & 31;
-    const uint32_t warp_in_block = threadIdx.x >> 5;
-    const uint32_t core = blockIdx.x * (blockDim.x >> 5) + warp_in_block;
-    if (core >= L.cores) return;
-
+__device__ __forceinline__ void core_run(const CoreLaunch<RT>& L, uint32_t core, uint32_t sub, const CoreStream* states,
+                                         CoreStream* states_out, uint64_t* sums, unsigned char* smem_raw, TraceRec* trace, int lane) {
     CoreCtx<RT, KIND> c;
     c.mp = L.mp;
     c.ot = L.ot;
     c.key = tf_key(L.seed, core);
     c.sync = states[2 * core];
     c.inner = states[2 * core + 1];
-    c.Rt = reinterpret_cast<RT*>(smem_raw) + (size_t)warp_in_block * (L.ot.Q ? L.ot.Q : 1);
+    c.Rt = reinterpret_cast<RT*>(smem_raw) + (size_t)(threadIdx.x >> 5) * (L.ot.Q ? L.ot.Q : 1);
     c.Y = 0;
     c.constant = 0;
     c.err = 0;
@@ -542,6 +583,11 @@ __global__ void __launch_bounds__(256) core_level_kernel(CoreLaunch<RT> L, CoreS
     const uint64_t q = L.M / L.cores, rem = L.M % L.cores;
     const uint64_t mcount = q + (core < rem ? 1 : 0);
     const uint64_t mfirst = q * core + (core < rem ? core : rem);
+    const uint64_t mm0 = mcount * sub / L.subs, mm1 = mcount * (sub + 1) / L.subs;
+    const CoreStream sync0 = c.sync;                     // models: the outer draws count from here
+    OuterNormals<RT> on;
+    on.base = ~0ull;
+    if (KIND != KIND_PORTFOLIO && mm0 > 0) advance_normals<RT>(c.inner, c.key, mm0 * L.outer_normals);
     const bool fine_only = L.fine_only;
     const RT r = (RT)L.adaptive_r;
 
@@ -549,13 +595,18 @@ __global__ void __launch_bounds__(256) core_level_kernel(CoreLaunch<RT> L, CoreS
     uint64_t st[6] = {0, 0, 0, 0, 0, 0};
     uint64_t nu = 0, nn = 0;
 
-    for (uint64_t mm = 0; mm < mcount; mm++) {
+    for (uint64_t mm = mm0; mm < mm1; mm++) {
         TraceRec tr;
         tr.core = core;
         tr.pilots = 0;
         tr.min_abs_small = INFINITY;
         tr.mean_big = 0;
-        core_sample_outer<RT, KIND>(c, nn, lane);
+        if constexpr (KIND == KIND_PORTFOLIO) {
+            core_sample_outer<RT, KIND>(c, nn, lane);
+        } else {
+            c.Y = on.get(c.key, sync0, mm, lane);        // model_sampler.cpp:53-55
+            nn += 1;
+        }
         uint64_t cf = core_count<RT, KIND>(c, L.cf, r, true, st, work, nu, nn, tr.pilots, lane);
         uint64_t cc = 0;
         RT f_phi = (RT)0, c_phi = (RT)0;
@@ -624,46 +675,109 @@ __global__ void __launch_bounds__(256) core_level_kernel(CoreLaunch<RT> L, CoreS
             trace[mfirst + mm] = tr;
         }
     }
+    if (sub == L.subs - 1) {
+        if (KIND != KIND_PORTFOLIO) advance_normals<RT>(c.sync, c.key, mcount);
+        if (lane == 0) {
+            states_out[2 * core] = c.sync;
+            states_out[2 * core + 1] = c.inner;
+        }
+    }
     if (lane == 0) {
-        states[2 * core] = c.sync;
-        states[2 * core + 1] = c.inner;
-        double* o = out_sums + (size_t)core * 10;
-        for (int j = 0; j < 4; j++) { o[j] = f_sums[j]; o[4 + j] = d_sums[j]; }
-        o[8] = work;
-        o[9] = c.err ? 1.0 : 0.0;
-        uint64_t* s = out_stats + (size_t)core * 6;
-        for (int j = 0; j < 4; j++) s[j] = st[j];
-        s[4] = nu;
-        s[5] = nn;
+        for (int j = 0; j < 4; j++) {
+            sums[j] = (uint64_t)__double_as_longlong(f_sums[j]);
+            sums[4 + j] = (uint64_t)__double_as_longlong(d_sums[j]);
+            sums[10 + j] = st[j];
+        }
+        sums[8] = (uint64_t)__double_as_longlong(work);
+        sums[9] = (uint64_t)__double_as_longlong(c.err ? 1.0 : 0.0);
+        sums[14] = nu;
+        sums[15] = nn;
     }
 }
 
-// Sums the per-core partials in core order (one block).
-__global__ void core_reduce_kernel(uint32_t cores, const double* in_sums, const uint64_t* in_stats,
-                                   double* out_sums, uint64_t* out_stats) {
-    __shared__ double sd[256][10];
-    __shared__ uint64_t su[256][6];
-    const uint32_t t = threadIdx.x;
-    double a[10] = {0};
-    uint64_t b[6] = {0};
-    for (uint32_t c = t; c < cores; c += blockDim.x) {
-        for (int j = 0; j < 10; j++) a[j] += in_sums[(size_t)c * 10 + j];
-        for (int j = 0; j < 6; j++) b[j] += in_stats[(size_t)c * 6 + j];
+// Threads per CTA: two virtual cores, so that 2048 cores spread evenly over the SMs (CTAs of eight
+// left 108 SMs with 16 warps and 40 with 8).
+constexpr int kCoreThreads = 64, kCoreWarps = kCoreThreads / 32;
+// CTAs whose partial sums are added together before the groups are.
+constexpr uint32_t kCoreGroup = 32;
+
+// Adds `n` partial results of 16 words (10 sums, 6 counts) in a fixed order, by all kCoreThreads
+// threads: word t % 16 of partials t / 16, t / 16 + 4, ..., then the four threads of a word in order.
+__device__ __forceinline__ uint64_t core_add(const uint64_t* part, uint32_t n) {
+    __shared__ uint64_t red[kCoreThreads / 16][16];
+    const int t = threadIdx.x, q = t & 15, g = t >> 4;
+    double a = 0;
+    uint64_t u = 0;
+    for (uint32_t b = g; b < n; b += kCoreThreads / 16) {
+        const uint64_t v = __ldcg(part + (size_t)b * 16 + q);
+        if (q < 10) a += __longlong_as_double((long long)v); else u += v;
     }
-    for (int j = 0; j < 10; j++) sd[t][j] = a[j];
-    for (int j = 0; j < 6; j++) su[t][j] = b[j];
     __syncthreads();
-    for (uint32_t s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (t < s) {
-            for (int j = 0; j < 10; j++) sd[t][j] += sd[t + s][j];
-            for (int j = 0; j < 6; j++) su[t][j] += su[t + s][j];
+    red[g][q] = q < 10 ? (uint64_t)__double_as_longlong(a) : u;
+    __syncthreads();
+    if (q < 10) {
+        a = 0;
+        for (int k = 0; k < kCoreThreads / 16; k++) a += __longlong_as_double((long long)red[k][q]);
+        return (uint64_t)__double_as_longlong(a);
+    }
+    u = 0;
+    for (int k = 0; k < kCoreThreads / 16; k++) u += red[k][q];
+    return u;
+}
+
+// Whether this CTA is the last of `n` to arrive at *count (then reset for the next launch).
+__device__ __forceinline__ bool core_last(uint32_t* count, uint32_t n) {
+    __shared__ uint32_t arrived;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) arrived = atomicAdd(count, 1u);
+    __syncthreads();
+    if (arrived != n - 1) return false;
+    if (threadIdx.x == 0) *count = 0;
+    __threadfence();
+    return true;
+}
+
+// The level's results from the cores' partials, inside the level kernel: the last CTA of a group of
+// kCoreGroup adds the group's, the last group's adds the groups' and stores the 16 words in the
+// host's pinned memory (a one-CTA kernel over all cores took 18 us, two copies back followed).
+__device__ __forceinline__ void core_finish(uint64_t* part, uint32_t* counts, uint64_t* out) {
+    const uint32_t groups = (gridDim.x + kCoreGroup - 1) / kCoreGroup, g = blockIdx.x / kCoreGroup;
+    const uint32_t first = g * kCoreGroup, n = gridDim.x - first < kCoreGroup ? gridDim.x - first : kCoreGroup;
+    if (!core_last(counts + 1 + g, n)) return;
+    const uint64_t v = core_add(part + (size_t)first * 16, n);
+    uint64_t* gpart = part + (size_t)gridDim.x * 16;
+    if (threadIdx.x < 16) gpart[(size_t)g * 16 + threadIdx.x] = v;
+    if (!core_last(counts, groups)) return;
+    const uint64_t r = core_add(gpart, groups);
+    if (threadIdx.x < 16) out[threadIdx.x] = r;
+}
+
+// A level whose inner counts are fixed (no pilots on either side) draws a known number of normals
+// per outer sample, so the models' outer samples of one core can be split over several warps
+// (CoreLaunch::subs), each starting at its own stream position.  At most 128 registers: 16 warps per
+// SM hold the 13.8 of 2048 cores in one wave.
+template <class RT, int KIND>
+__global__ void __launch_bounds__(kCoreThreads, 8) core_level_kernel(CoreLaunch<RT> L, const CoreStream* states, CoreStream* states_out,
+                                                                  uint64_t* part, uint32_t* counts, uint64_t* out, TraceRec* trace) {
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ uint64_t sm_part[kCoreWarps][16];
+    const int lane = threadIdx.x & 31;
+    const uint32_t warp_in_block = threadIdx.x >> 5;
+    const uint32_t unit = blockIdx.x * kCoreWarps + warp_in_block, core = unit / L.subs, sub = unit % L.subs;
+    if (core < L.cores) core_run<RT, KIND>(L, core, sub, states, states_out, sm_part[warp_in_block], smem_raw, trace, lane);
+    else if (lane < 16) sm_part[warp_in_block][lane] = 0;
+    __syncthreads();
+    if (threadIdx.x < 16) {
+        const int q = threadIdx.x;
+        uint64_t u = 0;
+        double a = 0;
+        for (int k = 0; k < kCoreWarps; k++) {
+            if (q < 10) a += __longlong_as_double((long long)sm_part[k][q]); else u += sm_part[k][q];
         }
-        __syncthreads();
+        part[(size_t)blockIdx.x * 16 + q] = q < 10 ? (uint64_t)__double_as_longlong(a) : u;
     }
-    if (t == 0) {
-        for (int j = 0; j < 10; j++) out_sums[j] = sd[0][j];
-        for (int j = 0; j < 6; j++) out_stats[j] = su[0][j];
-    }
+    core_finish(part, counts, out);
 }
 
 template <class RT>
@@ -703,41 +817,60 @@ cudaError_t launch_ref_records(const OptionTable<double>& t, RefOption<double>* 
     return launch_ref_records_t<double>(t, out, stream);
 }
 
+// Warps per core of a level with fixed counts: enough for 16 warps on each of 148 SMs, at most one
+// per outer sample.
+static uint32_t core_subs(uint32_t cores, uint64_t M) {
+    const uint64_t per_core = (M + cores - 1) / cores, want = (148ull * 16 + cores - 1) / cores;
+    return (uint32_t)(want < per_core ? want : per_core ? per_core : 1);
+}
+
+uint32_t core_ctas(uint32_t cores) {
+    const uint64_t units = cores > 148u * 16u ? cores : (uint64_t)cores * ((148ull * 16 + cores - 1) / cores);
+    return (uint32_t)((units + kCoreWarps - 1) / kCoreWarps);
+}
+size_t core_part_words(uint32_t cores) {
+    const size_t ctas = core_ctas(cores);
+    return (ctas + (ctas + kCoreGroup - 1) / kCoreGroup) * 16;
+}
+size_t core_counts(uint32_t cores) { return 1 + (core_ctas(cores) + kCoreGroup - 1) / kCoreGroup; }
+
 template <class RT>
-static cudaError_t launch_core_t(const CoreLaunch<RT>& L, int kind, CoreStream* states, double* part_sums,
-                                 uint64_t* part_stats, double* out_sums, uint64_t* out_stats,
-                                 TraceRec* trace, cudaStream_t stream) {
-    const int threads = 256, warps = threads / 32;
-    const uint32_t blocks = (L.cores + warps - 1) / warps;
-    size_t smem = (kind == KIND_PORTFOLIO) ? (size_t)warps * (L.ot.Q ? L.ot.Q : 1) * sizeof(RT) : 0;
+static cudaError_t launch_core_t(CoreLaunch<RT> L, int kind, const CoreStream* states, CoreStream* states_out, uint64_t* part, uint32_t* counts,
+                                 uint64_t* out, TraceRec* trace, cudaStream_t stream) {
+    L.subs = 1;
+    L.outer_normals = 0;
+    const bool fixed = L.cf.max_count <= 2 * L.cf.base_count && (L.fine_only || L.cc.max_count <= 2 * L.cc.base_count);
+    if (fixed && (kind == KIND_REF_MODEL || kind == KIND_SHIFT_MODEL)) {
+        const uint64_t big = L.cf.max_count > L.cc.max_count ? L.cf.max_count : L.cc.max_count;
+        const uint64_t n = L.fine_only ? L.cf.max_count : (L.antithetic ? big : L.cf.max_count + L.cc.max_count);
+        L.outer_normals = n * (kind == KIND_REF_MODEL ? 2 : 1);
+        L.subs = core_subs(L.cores, L.M);
+    }
+    const uint32_t blocks = (uint32_t)(((uint64_t)L.cores * L.subs + kCoreWarps - 1) / kCoreWarps);
+    size_t smem = (kind == KIND_PORTFOLIO) ? (size_t)kCoreWarps * (L.ot.Q ? L.ot.Q : 1) * sizeof(RT) : 0;
     if (kind == KIND_REF_MODEL)
-        core_level_kernel<RT, KIND_REF_MODEL><<<blocks, threads, smem, stream>>>(L, states, part_sums, part_stats, trace);
+        core_level_kernel<RT, KIND_REF_MODEL><<<blocks, kCoreThreads, smem, stream>>>(L, states, states_out, part, counts, out, trace);
     else if (kind == KIND_SHIFT_MODEL)
-        core_level_kernel<RT, KIND_SHIFT_MODEL><<<blocks, threads, smem, stream>>>(L, states, part_sums, part_stats, trace);
+        core_level_kernel<RT, KIND_SHIFT_MODEL><<<blocks, kCoreThreads, smem, stream>>>(L, states, states_out, part, counts, out, trace);
     else {
         if (smem > 48 * 1024) {
             cudaError_t e = cudaFuncSetAttribute(core_level_kernel<RT, KIND_PORTFOLIO>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e != cudaSuccess) return e;
         }
-        core_level_kernel<RT, KIND_PORTFOLIO><<<blocks, threads, smem, stream>>>(L, states, part_sums, part_stats, trace);
+        core_level_kernel<RT, KIND_PORTFOLIO><<<blocks, kCoreThreads, smem, stream>>>(L, states, states_out, part, counts, out, trace);
     }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    core_reduce_kernel<<<1, 256, 0, stream>>>(L.cores, part_sums, part_stats, out_sums, out_stats);
-    count_launch(2);
+    count_launch();
     return cudaGetLastError();
 }
 
-cudaError_t launch_core(const CoreLaunch<float>& L, int kind, CoreStream* states, double* part_sums,
-                        uint64_t* part_stats, double* out_sums, uint64_t* out_stats, TraceRec* trace,
-                        cudaStream_t stream) {
-    return launch_core_t<float>(L, kind, states, part_sums, part_stats, out_sums, out_stats, trace, stream);
+cudaError_t launch_core(const CoreLaunch<float>& L, int kind, const CoreStream* states, CoreStream* states_out, uint64_t* part, uint32_t* counts,
+                        uint64_t* out, TraceRec* trace, cudaStream_t stream) {
+    return launch_core_t<float>(L, kind, states, states_out, part, counts, out, trace, stream);
 }
-cudaError_t launch_core(const CoreLaunch<double>& L, int kind, CoreStream* states, double* part_sums,
-                        uint64_t* part_stats, double* out_sums, uint64_t* out_stats, TraceRec* trace,
-                        cudaStream_t stream) {
-    return launch_core_t<double>(L, kind, states, part_sums, part_stats, out_sums, out_stats, trace, stream);
+cudaError_t launch_core(const CoreLaunch<double>& L, int kind, const CoreStream* states, CoreStream* states_out, uint64_t* part, uint32_t* counts,
+                        uint64_t* out, TraceRec* trace, cudaStream_t stream) {
+    return launch_core_t<double>(L, kind, states, states_out, part, counts, out, trace, stream);
 }
 
 }  // namespace nmlmc

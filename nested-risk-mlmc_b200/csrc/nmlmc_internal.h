@@ -18,6 +18,8 @@ static_assert(sizeof(CoreStream) == 24, "CoreStream layout");
 template <class RT>
 struct CoreLaunch {
     uint32_t cores, ell;
+    uint32_t subs;            // warps per core (set by launch_core)
+    uint64_t outer_normals;   // inner normals per outer sample of a level with fixed counts (likewise)
     uint64_t M;
     uint64_t seed;
     bool fine_only, antithetic;
@@ -27,12 +29,16 @@ struct CoreLaunch {
     OptionTable<RT> ot;
 };
 
-cudaError_t launch_core(const CoreLaunch<float>& L, int kind, CoreStream* states, double* part_sums,
-                        uint64_t* part_stats, double* out_sums, uint64_t* out_stats, TraceRec* trace,
-                        cudaStream_t stream);
-cudaError_t launch_core(const CoreLaunch<double>& L, int kind, CoreStream* states, double* part_sums,
-                        uint64_t* part_stats, double* out_sums, uint64_t* out_stats, TraceRec* trace,
-                        cudaStream_t stream);
+// `states`: the cores' stream states, `states_out`: those after the call (another buffer: a core's
+// warps may start after its last one has ended).  `part`: core_part_words(cores) words, `counts`: core_counts(cores) zeroed counters (left zero),
+// `out`: the level's 16 words (10 sums: phi_f moments, difference moments, work, path-limit flag; 6
+// counts), in device or pinned host memory.
+size_t core_part_words(uint32_t cores);
+size_t core_counts(uint32_t cores);
+cudaError_t launch_core(const CoreLaunch<float>& L, int kind, const CoreStream* states, CoreStream* states_out, uint64_t* part, uint32_t* counts,
+                        uint64_t* out, TraceRec* trace, cudaStream_t stream);
+cudaError_t launch_core(const CoreLaunch<double>& L, int kind, const CoreStream* states, CoreStream* states_out, uint64_t* part, uint32_t* counts,
+                        uint64_t* out, TraceRec* trace, cudaStream_t stream);
 // Per-option constants of the reference-arithmetic tables (RefOption), P records.
 cudaError_t launch_ref_records(const OptionTable<float>& t, RefOption<float>* out, cudaStream_t stream);
 cudaError_t launch_ref_records(const OptionTable<double>& t, RefOption<double>* out, cudaStream_t stream);
