@@ -103,6 +103,8 @@ struct HostPortfolio {
     int subsample = SUB_UNIFORM, use_delta_cv = 0, discount = 1;
     bool s1_rho2_given = false;
     bool own_params = false;   // start / delta_est computed here (native API), per precision
+    int params_size = 0;       // size of the real_t they are computed in
+    bool unit_work = true;     // every W_est is 1
     // compute methods: options are stored grouped by method (BS, Exact, Unbiased) in the order
     // given; m_n counts them, order[k] is the caller's index of stored option k
     uint32_t m_n[3] = {0, 0, 0};
@@ -121,6 +123,9 @@ struct DevPortfolio {
     uint32_t* stock_ind = nullptr;
     int8_t* type = nullptr;
     RefOption<RT>* ref = nullptr;     // per-option constants in reference arithmetic
+    PathOption* path = nullptr;       // packed options of the FP32 path-simulated kernel
+    RT* lvl_w = nullptr;              // Unbiased level weights
+    float* lvl_wf = nullptr;
     uint32_t* guide = nullptr;        // guide tables of the CORE layout's inverse-CDF draw
     FastOption* fast = nullptr;       // packed records of the FP32 path
     FastOption* fast_s = nullptr;     // the same, scaled by 1 / sampling probability
@@ -270,7 +275,7 @@ template <class RT>
 void free_dev_portfolio(DevPortfolio<RT>& d) {
     dfree(d.strike); dfree(d.maturity); dfree(d.start); dfree(d.w); dfree(d.prob); dfree(d.W_est);
     dfree(d.cdf); dfree(d.S0); dfree(d.mu); dfree(d.sigma); dfree(d.delta_coalesce);
-    dfree(d.stock_ind); dfree(d.type); dfree(d.ref); dfree(d.guide); dfree(d.fast); dfree(d.fast_s); dfree(d.fast_col); dfree(d.alias); dfree(d.phat);
+    dfree(d.stock_ind); dfree(d.type); dfree(d.ref); dfree(d.path); dfree(d.lvl_w); dfree(d.lvl_wf); dfree(d.guide); dfree(d.fast); dfree(d.fast_s); dfree(d.fast_col); dfree(d.alias); dfree(d.phat);
     d.table = OptionTable<RT>{};
 }
 
@@ -298,6 +303,7 @@ void comp_params(HostPortfolio& h) {
         h.start[j] = (double)h_calc_bs<RT>(h.type[j], (RT)h.S0[s], (RT)h.strike[j], (RT)h.r, (RT)h.maturity[j], (RT)h.sigma[s]);
         h.delta_est[j] = (double)h_calc_delta<RT>(h.type[j], (RT)h.S0[s], (RT)h.strike[j], (RT)h.r, (RT)h.maturity[j], (RT)h.sigma[s]);
     }
+    h.params_size = (int)sizeof(RT);
 }
 
 // Alias table of the OUTER layout's importance sub-sampling (Walker's method in Vose's
@@ -342,13 +348,20 @@ void build_alias(uint32_t P, const std::vector<double>& p, std::vector<uint2>& t
     for (uint32_t j : small) tab[j].x = (uint32_t)std::min<uint64_t>(W[j], 0xffffffffull);   // == unit: exact sums
 }
 
+// Whether the context's sampling reads the reference-arithmetic records and the CDF's guide table:
+// all but the packed FP32 path of a portfolio without path-simulated options.
+bool needs_reference_tables(const nmlmc_ctx* c) {
+    return c->cfg.streams == NMLMC_STREAMS_CORE || c->cfg.precision != NMLMC_PREC_FP32 || c->pf.mixed() || !c->pf.unit_work;
+}
+
 // portfolio_comp_params + portfolio_update_data (portfolio_sampler.cpp:631-700) in real_t.
 template <class RT>
 int build_dev_portfolio(nmlmc_ctx* c, DevPortfolio<RT>& d) {
     HostPortfolio& h = c->pf;
     free_dev_portfolio(d);
-    if (h.own_params) comp_params<RT>(h);
+    if (h.own_params && h.params_size != (int)sizeof(RT)) comp_params<RT>(h);
     const uint32_t P = h.P, Q = h.Q;
+    const bool reference = needs_reference_tables(c);
     std::vector<RT> S0 = narrow<RT>(h.S0), mu = narrow<RT>(h.mu), sg = narrow<RT>(h.sigma);
     std::vector<RT> K = narrow<RT>(h.strike), T = narrow<RT>(h.maturity), w = narrow<RT>(h.w);
     std::vector<RT> prob = narrow<RT>(h.prob), West = narrow<RT>(h.W_est);
@@ -392,7 +405,7 @@ int build_dev_portfolio(nmlmc_ctx* c, DevPortfolio<RT>& d) {
     t.use_coarse_delta_cv = h.use_coarse_delta_cv; t.use_antithetic_risk = h.use_antithetic_risk;
     t.use_milstein = h.use_milstein;
     t.guide = nullptr;
-    if (h.subsample == SUB_RANDOM) {
+    if (h.subsample == SUB_RANDOM && reference) {
         // guide_n = m_n buckets per method; entry k is the last option whose CDF value lies in a
         // bucket before k (0 if none does), entry n closes the last bucket
         std::vector<uint32_t> guide;
@@ -410,9 +423,6 @@ int build_dev_portfolio(nmlmc_ctx* c, DevPortfolio<RT>& d) {
         if ((rc = upload(d.guide, guide))) return rc;
         t.guide = d.guide;
     }
-    if (dev_malloc(&d.ref, P * sizeof(RefOption<RT>)) != cudaSuccess) return set_err(NMLMC_ERR_NOMEM);
-    NM_CUDA(launch_ref_records(t, d.ref, c->stream), "option constants");
-    t.ref = d.ref;
     t.fast = nullptr;
     t.fast_s = nullptr;
     t.fast_col = nullptr;
@@ -430,12 +440,45 @@ int build_dev_portfolio(nmlmc_ctx* c, DevPortfolio<RT>& d) {
         t.alias = d.alias;
         t.phat = d.phat;
     }
+    t.path = nullptr;
+    if (h.mixed()) {
+        // thresholds of the Unbiased level (level_of_word): the words below thr[L] have levels >= L
+        const double den = log((double)t.dt_beta) * (double)t.dt_prob_expo;
+        t.lvl_thr[0] = 1ull << 32;
+        for (uint32_t L = 1; L < kPathLevels; L++) {
+            uint64_t lo = 0, hi = 1ull << 32;             // smallest word whose level is below L
+            while (lo < hi) {
+                const uint64_t mid = (lo + hi) / 2;
+                const double u = (double)mid * 0x1p-32 + 0x1p-33;
+                if (floor(log(u) / den) >= (double)L) lo = mid + 1; else hi = mid;
+            }
+            t.lvl_thr[L] = lo;
+        }
+        if constexpr (sizeof(RT) == 4) {
+            std::vector<PathOption> po(P);
+            for (uint32_t j = 0; j < P; j++) {
+                const uint32_t s = h.stock_ind[j];
+                po[j] = PathOption{S0[s], sg[s], K[j], T[j], w[j], West[j],
+                                   h.subsample == SUB_RANDOM ? (float)phat[j] : t.inv_count_prob, s << 1 | (h.type[j] > 0 ? 1u : 0u)};
+            }
+            if ((rc = upload(d.path, po))) return rc;
+            t.path = d.path;
+        }
+    }
+    if (reference) {
+        if (dev_malloc(&d.ref, P * sizeof(RefOption<RT>)) != cudaSuccess ||
+            dev_malloc(&d.lvl_w, kPathLevels * sizeof(RT)) != cudaSuccess ||
+            dev_malloc(&d.lvl_wf, kPathLevels * sizeof(float)) != cudaSuccess)
+            return set_err(NMLMC_ERR_NOMEM);
+        NM_CUDA(launch_ref_records(t, d.ref, d.lvl_w, d.lvl_wf, c->stream), "option constants");
+    }
+    t.ref = d.ref;
+    t.lvl_w = d.lvl_w;
+    t.lvl_wf = d.lvl_wf;
     if constexpr (sizeof(RT) == 4) {
         // packed FP32 records (nmlmc_bs.cuh): per-option constants folded in double, rounded once;
         // only for unit work estimates (every option of the BS method costs one evaluation)
-        bool unit = true;
-        for (uint32_t j = 0; j < P; j++) unit = unit && h.W_est[j] == 1.0;
-        if (unit && !h.mixed()) {
+        if (h.unit_work && !h.mixed()) {
             // Record of option j with its weights scaled by sc and, with cv_on, the delta control
             // variate: cv = sc w Delta_BS(S0, T) and its constant -cv S0 folded into wV0.
             auto record = [&](uint32_t j, double sc, bool cv_on) {
@@ -488,7 +531,9 @@ int build_dev_portfolio(nmlmc_ctx* c, DevPortfolio<RT>& d) {
 int ensure_portfolio(nmlmc_ctx* c) {
     if (c->kind != KIND_PORTFOLIO) return NMLMC_OK;
     const int want = c->cfg.precision == NMLMC_PREC_FP64 ? 1 : 0;
-    if (c->pf_prec == want) return NMLMC_OK;
+    // (a context switched to the reference streams or arithmetic builds the tables they read)
+    const bool have = want ? c->dpf64.table.ref != nullptr : c->dpf32.table.ref != nullptr;
+    if (c->pf_prec == want && (have || !needs_reference_tables(c))) return NMLMC_OK;
     int rc = want ? build_dev_portfolio<double>(c, c->dpf64) : build_dev_portfolio<float>(c, c->dpf32);
     if (rc == NMLMC_OK) c->pf_prec = want;
     return rc;
@@ -1833,7 +1878,7 @@ static int portfolio_from_ref(const portfolio_data* d) {
             if (op.stock_ind >= s.size || !(op.prob > 0) || !(prev >= op.prob)) return NMLMC_ERR_ARG;
             prev = op.prob;
             h.strike.push_back(op.strike); h.maturity.push_back(op.maturity); h.w.push_back(op.w);
-            h.prob.push_back(op.prob); h.W_est.push_back(op.W_est); h.start.push_back(op.start);
+            h.prob.push_back(op.prob); h.W_est.push_back(op.W_est); h.unit_work = h.unit_work && op.W_est == 1.0f; h.start.push_back(op.start);
             h.delta_est.push_back(op.delta_est); h.stock_ind.push_back(op.stock_ind);
             h.type.push_back((int8_t)(op.type > 0 ? 1 : -1));
             h.order.push_back((uint32_t)h.order.size());

@@ -59,6 +59,20 @@ struct __align__(16) RefOption {
     int32_t type;
 };
 
+// What a path-simulated inner sample of the FP32 path needs of its option, in one 256-bit load
+// instead of nine scattered ones: wgt is its position, prob its sampling probability, link = stock
+// << 1 | call.
+struct __align__(32) PathOption {
+    float S0, sigma, strike, maturity;
+    float wgt, W_est, prob;
+    uint32_t link;
+};
+static_assert(sizeof(PathOption) == 32, "PathOption layout");
+
+// Unbiased levels L = 0 .. kPathLevels - 1 have tables; kMaxPathSteps = 2^24 steps end before the
+// last one at any beta >= 2.
+constexpr uint32_t kPathLevels = 26;
+
 // Option table in HBM, structure of arrays.  Options are grouped by compute method
 // (portfolio::data::options[3], portfolio_sampler.cpp:62-92): method m occupies
 // [m_off[m], m_off[m] + m_n[m]) and its CDF restarts at 0.
@@ -100,6 +114,12 @@ struct OptionTable {
     uint32_t dt_h0inv, dt_beta;
     RT dt_prob_expo;
     int use_coarse_delta_cv, use_antithetic_risk, use_milstein;
+    const PathOption* path;          // FP32 path, mixed portfolios
+    const RT* lvl_w;                 // [kPathLevels] weights beta^(-e L) / (1 - beta^e), reference arithmetic
+    const float* lvl_wf;             // the same on the FP32 path (SFU exponentials)
+    // OUTER layout, FP32 and FP64: the level of a 32-bit uniform word is the number of j >= 1 with
+    // word < lvl_thr[j]
+    uint64_t lvl_thr[kPathLevels];
 };
 
 template <class RT>

@@ -781,7 +781,11 @@ __global__ void __launch_bounds__(kCoreThreads, 8) core_level_kernel(CoreLaunch<
 }
 
 template <class RT>
-__global__ void __launch_bounds__(128) k_ref_records(OptionTable<RT> t, RefOption<RT>* out) {
+__global__ void __launch_bounds__(128) k_ref_records(OptionTable<RT> t, RefOption<RT>* out, RT* lvl_w, float* lvl_wf) {
+    if (blockIdx.x == 0 && threadIdx.x < kPathLevels && t.mixed) {
+        lvl_w[threadIdx.x] = level_weight<RT>(t, threadIdx.x);
+        lvl_wf[threadIdx.x] = level_weight_fast((float)t.dt_prob_expo, t.dt_beta, threadIdx.x);
+    }
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < t.P; j += gridDim.x * blockDim.x) {
         const uint32_t s = t.stock_ind[j];
         const int type = t.type[j];
@@ -804,17 +808,18 @@ __global__ void __launch_bounds__(128) k_ref_records(OptionTable<RT> t, RefOptio
 }
 
 template <class RT>
-static cudaError_t launch_ref_records_t(const OptionTable<RT>& t, RefOption<RT>* out, cudaStream_t stream) {
+static cudaError_t launch_ref_records_t(const OptionTable<RT>& t, RefOption<RT>* out, RT* lvl_w, float* lvl_wf,
+                                        cudaStream_t stream) {
     const uint32_t blocks = (t.P + 127) / 128;
-    k_ref_records<RT><<<blocks < 2048 ? blocks : 2048, 128, 0, stream>>>(t, out);
+    k_ref_records<RT><<<blocks < 2048 ? blocks : 2048, 128, 0, stream>>>(t, out, lvl_w, lvl_wf);
     count_launch();
     return cudaGetLastError();
 }
-cudaError_t launch_ref_records(const OptionTable<float>& t, RefOption<float>* out, cudaStream_t stream) {
-    return launch_ref_records_t<float>(t, out, stream);
+cudaError_t launch_ref_records(const OptionTable<float>& t, RefOption<float>* out, float* lvl_w, float* lvl_wf, cudaStream_t stream) {
+    return launch_ref_records_t<float>(t, out, lvl_w, lvl_wf, stream);
 }
-cudaError_t launch_ref_records(const OptionTable<double>& t, RefOption<double>* out, cudaStream_t stream) {
-    return launch_ref_records_t<double>(t, out, stream);
+cudaError_t launch_ref_records(const OptionTable<double>& t, RefOption<double>* out, double* lvl_w, float* lvl_wf, cudaStream_t stream) {
+    return launch_ref_records_t<double>(t, out, lvl_w, lvl_wf, stream);
 }
 
 // Warps per core of a level with fixed counts: enough for 16 warps on each of 148 SMs, at most one

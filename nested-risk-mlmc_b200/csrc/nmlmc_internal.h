@@ -39,9 +39,12 @@ cudaError_t launch_core(const CoreLaunch<float>& L, int kind, const CoreStream* 
                         uint64_t* out, TraceRec* trace, cudaStream_t stream);
 cudaError_t launch_core(const CoreLaunch<double>& L, int kind, const CoreStream* states, CoreStream* states_out, uint64_t* part, uint32_t* counts,
                         uint64_t* out, TraceRec* trace, cudaStream_t stream);
-// Per-option constants of the reference-arithmetic tables (RefOption), P records.
-cudaError_t launch_ref_records(const OptionTable<float>& t, RefOption<float>* out, cudaStream_t stream);
-cudaError_t launch_ref_records(const OptionTable<double>& t, RefOption<double>* out, cudaStream_t stream);
+// Per-option constants of the reference-arithmetic tables (RefOption), P records, and the Unbiased
+// levels' weights, kPathLevels each.
+cudaError_t launch_ref_records(const OptionTable<float>& t, RefOption<float>* out, float* lvl_w, float* lvl_wf,
+                               cudaStream_t stream);
+cudaError_t launch_ref_records(const OptionTable<double>& t, RefOption<double>* out, double* lvl_w, float* lvl_wf,
+                               cudaStream_t stream);
 
 // ---- OUTER layout (batched) ----------------------------------------------------------------
 enum Prec : int { PREC_REF32 = 0, PREC_FP64 = 1, PREC_FP32 = 2 };

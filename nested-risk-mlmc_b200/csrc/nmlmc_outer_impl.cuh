@@ -519,27 +519,23 @@ __device__ __forceinline__ void* user_ws(const OuterBuffers& B, uint32_t item) {
 // C (inner samples per chunk) is a compile-time constant so the independent Threefry blocks of a
 // chunk can be interleaved (two at a time) for instruction-level parallelism.
 // ---- path-simulated portfolio, FP32 -------------------------------------------------------
-// Steps N_l = beta^L of an Unbiased level (false when h0 N_l exceeds kMaxPathSteps).
-__device__ __forceinline__ bool level_steps(const OptionTable<float>& ot, uint32_t Lv, uint64_t& N_l) {
-    N_l = 1;
-    bool ok = true;
-    for (uint32_t i = 0; i < Lv && ok; i++) {
-        N_l *= ot.dt_beta;
-        ok = N_l * ot.dt_h0inv <= kMaxPathSteps;
-    }
-    return ok && N_l * ot.dt_h0inv <= kMaxPathSteps;
-}
-
-// The Unbiased level of the inner sample with path namespace ns, drawn in double as the FP64 path
-// draws it (sample_inner_unbiased, portfolio_sampler.cpp:521-537), and its steps.
+// The Unbiased level of the inner sample with path namespace ns (sample_inner_unbiased,
+// portfolio_sampler.cpp:521-537), the level of the double-precision formula, and its steps.
 __device__ __forceinline__ bool level_fp32(const OptionTable<float>& ot, const TfKey& key, uint64_t ns,
                                            uint32_t& Lv, uint64_t& N_l) {
     uint64_t u0, u1;
     threefry2x64(0, ns | kPathUniform, key, u0, u1);
-    const double u = __dadd_rn(__dmul_rn((double)(uint32_t)u0, 0x1p-32), 0x1p-33);
-    const double qL = log(u) / (log((double)ot.dt_beta) * (double)ot.dt_prob_expo);
-    Lv = (uint32_t)floor(qL);
-    return level_steps(ot, Lv, N_l);
+    return level_of_word(ot, (uint32_t)u0, Lv, N_l);
+}
+
+__device__ __forceinline__ PathOption load_path_option(const PathOption* p) {
+    PathOption o;
+    float link;
+    asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=f"(o.S0), "=f"(o.sigma), "=f"(o.strike), "=f"(o.maturity), "=f"(o.wgt), "=f"(o.W_est), "=f"(o.prob), "=f"(link)
+        : "l"(p));
+    o.link = __float_as_uint(link);
+    return o;
 }
 
 // Inner samples of a chunk of at most kPathSortChunk per thread are evaluated in the order of
@@ -565,29 +561,28 @@ constexpr uint32_t kCoopLevel = 5;
 
 // loss * weight of an Unbiased sample (inner_unbiased_fast) evaluated by all 32 lanes of the warp;
 // every lane returns the value, `work` is the owner's to add.
-__device__ __forceinline__ float inner_unbiased_coop(const OptionTable<float>& ot, float Rs, uint32_t j,
+__device__ __forceinline__ float inner_unbiased_coop(const OptionTable<float>& ot, float Rs, const PathOption& o,
                                                      const TfKey& key, uint64_t ns, uint32_t L, uint64_t N_l,
                                                      uint32_t lane) {
-    const uint32_t s = ot.stock_ind[j];
-    const float S0 = ot.S0[s], sg = ot.sigma[s], r = ot.r, tau = ot.tau, T = ot.maturity[j], K = ot.strike[j];
-    const float m = (float)ot.type[j], wdisc = ot.w[j] * __expf(-r * T);
+    const float S0 = o.S0, sg = o.sigma, r = ot.r, tau = ot.tau, T = o.maturity, K = o.strike;
+    const float m = (o.link & 1u) ? 1.f : -1.f, wdisc = o.wgt * __expf(-r * T);
     const float mu_t = (r - 0.5f * sg * sg) * tau;
     OuterPathNormals<float, PREC_FP32> nz{key, ns, 0, false, 0.f, 0};
     const float dW0 = ot.stau * nz.next();
     const float S0_t_1 = S0 * __expf(fmaf(sg, dW0, mu_t));
     const float S0_t_2 = S0 * __expf(fmaf(-sg, dW0, mu_t));
-    const uint64_t N = (uint64_t)ot.dt_h0inv * N_l;
+    const uint32_t N = ot.dt_h0inv * (uint32_t)N_l;          // at most kMaxPathSteps
     const uint32_t cs = ot.dt_beta;                          // fine steps per coarse step (L > 0)
-    const uint64_t Nc = N / cs;
+    const uint32_t Nc = N / cs;
     const float Tr = T - tau;
     const float dt = Tr / (float)N, sqrt_dt = sqrtf(dt), dt_c = dt * (float)cs;
     const float hs2 = ot.use_milstein ? 0.5f * sg * sg : 0.f;
     // this lane's coarse steps [c0, c1): fine steps c0 cs .. c1 cs - 1, normals 1 + n
-    const uint64_t c0 = Nc * lane / 32, c1 = Nc * (lane + 1) / 32;
+    const uint32_t c0 = Nc * lane / 32, c1 = Nc * (lane + 1) / 32;
     double Ff = 1.0, Fc = 1.0;
     if (c1 > c0) {
-        nz.seek(1 + c0 * cs);
-        for (uint64_t c = c0; c < c1; c++) {
+        nz.seek(1 + (uint64_t)c0 * cs);
+        for (uint32_t c = c0; c < c1; c++) {
             float dW_c = 0.f;
             for (uint32_t i = 0; i < cs; i++) {
                 const float dW = sqrt_dt * nz.next();
@@ -622,8 +617,7 @@ __device__ __forceinline__ float inner_unbiased_coop(const OptionTable<float>& o
         if (do_d_c) vdc += half * opt_derv_stock_fast(wdisc, m > 0.f, K, (float)S[ic + 3], S0);
     }
     const float ret = (vf - vc) + diff * (vdf - vdc);
-    const float e = ot.dt_prob_expo, lb = __log2f((float)ot.dt_beta);
-    return ret * (exp2f(-e * lb * (float)L) / (1.0f - exp2f(e * lb)));
+    return ret * ot.lvl_wf[L];
 }
 
 // `own`: this lane evaluates a chunk (lanes past the end of a segment's last tile take part in
@@ -688,17 +682,17 @@ __device__ __forceinline__ void pf_paths_sorted(const DevLevel<float>& D, const 
         else { q = __ffs(m4) - 1; m4 &= m4 - 1; }
         const uint32_t j = jbuf[q * kTile];
         const uint32_t c = cbuf[q * kTile];
-        const float prob = ot.subsample == SUB_UNIFORM ? ot.inv_count_prob : ot.phat[j];
+        const PathOption o = load_path_option(ot.path + j);
         float val;
         if (c == 0) {
             val = pf_value<float, 2>(ot, Rrow, j);
-            work += (double)ot.W_est[j];
+            work += (double)o.W_est;
         } else {
             const uint64_t ns = path_ns(tag, s0 + q);
             OuterPathNormals<float, PREC_FP32> nz{key, ns, 0, false, 0.f, 0};
-            const float Rs = Rrow[ot.stock_ind[j] * 2];
+            const float Rs = Rrow[(o.link >> 1) * 2];
             if (c == 1) {
-                val = inner_exact_fast(ot, Rs, j, nz, work);
+                val = inner_exact_fast(ot, Rs, o, nz, work);
             } else {
                 uint32_t Lv;
                 uint64_t N_l;
@@ -706,14 +700,14 @@ __device__ __forceinline__ void pf_paths_sorted(const DevLevel<float>& D, const 
                 if (c < 15) { Lv = c - 2; ok = level_steps(ot, Lv, N_l); }
                 else ok = level_fp32(ot, key, ns, Lv, N_l);
                 if (ok) {
-                    val = inner_unbiased_fast(ot, Rs, j, nz, work, Lv, N_l);
+                    val = inner_unbiased_fast(ot, Rs, o, nz, work, Lv, N_l);
                 } else {                         // beyond kMaxPathSteps: the call fails
                     atomicOr(D.B.counters + CNT_ERR, 1u);
                     val = 0.f;
                 }
             }
         }
-        float d = __fdiv_rn(val, prob);
+        float d = __fdiv_rn(val, o.prob);
         if (S2) d = __fadd_rn(d, shift);
         a1.add(d);
         if (S2) a2.add_sq(d);
@@ -739,24 +733,23 @@ __device__ __forceinline__ void pf_paths_sorted(const DevLevel<float>& D, const 
         const TfKey skey{__shfl_sync(0xffffffffu, key.k0, src), __shfl_sync(0xffffffffu, key.k1, src),
                          __shfl_sync(0xffffffffu, key.k2, src)};
         const uint64_t ns = path_ns(tag, __shfl_sync(0xffffffffu, s0, src) + q);
-        const float Rs = __shfl_sync(0xffffffffu, lane == src ? Rrow[ot.stock_ind[j] * 2] : 0.f, src);
+        const PathOption o = load_path_option(ot.path + j);
+        const float Rs = __shfl_sync(0xffffffffu, lane == src ? Rrow[(o.link >> 1) * 2] : 0.f, src);
         uint32_t Lv;
         uint64_t N_l;
         bool ok;
         if (c < 15) { Lv = c - 2; ok = level_steps(ot, Lv, N_l); }
         else ok = level_fp32(ot, skey, ns, Lv, N_l);
         float val = 0.f;
-        if (ok) val = inner_unbiased_coop(ot, Rs, j, skey, ns, Lv, N_l, lane);
+        if (ok) val = inner_unbiased_coop(ot, Rs, o, skey, ns, Lv, N_l, lane);
         if (lane == src) {
             if (ok) {
-                const float West = ot.W_est[j];
-                work += (double)((float)N_l * West);
-                work += (double)((float)(N_l / ot.dt_beta) * West);
+                work += (double)((float)N_l * o.W_est);
+                work += (double)((float)((uint32_t)N_l / ot.dt_beta) * o.W_est);
             } else {                                     // beyond kMaxPathSteps: the call fails
                 atomicOr(D.B.counters + CNT_ERR, 1u);
             }
-            const float prob = ot.subsample == SUB_UNIFORM ? ot.inv_count_prob : ot.phat[j];
-            float d = __fdiv_rn(val, prob);
+            float d = __fdiv_rn(val, o.prob);
             if (S2) d = __fadd_rn(d, shift);
             a1.add(d);
             if (S2) a2.add_sq(d);
@@ -874,7 +867,7 @@ __device__ __forceinline__ void eval_chunk_c(const DevLevel<RT>& D, uint32_t ite
                     OuterPathNormals<RT, PREC> nz{key, ns, 0, false, (RT)0, 0};
                     const RT Rs = Rrow[ot.stock_ind[j] * RS];
                     if (j < ot.m_off[2]) {
-                        if constexpr (PREC == PREC_FP32) val = inner_exact_fast(ot, Rs, j, nz, work);
+                        if constexpr (PREC == PREC_FP32) val = inner_exact_fast(ot, Rs, load_path_option(ot.path + j), nz, work);
                         else val = inner_exact<RT>(ot, Rs, j, nz, work);
                     } else {
                         uint64_t u0, u1;
@@ -882,13 +875,13 @@ __device__ __forceinline__ void eval_chunk_c(const DevLevel<RT>& D, uint32_t ite
                         uint32_t Lv;
                         uint64_t N_l;
                         bool ok;
-                        if constexpr (PREC == PREC_FP32) {
-                            ok = level_fp32(ot, key, ns, Lv, N_l);
+                        if constexpr (PREC != PREC_REF32) {
+                            ok = level_of_word(ot, (uint32_t)u0, Lv, N_l);
                         } else {
                             ok = unbiased_level<RT>(ot, u01_word<PREC, RT>((uint32_t)u0), Lv, N_l);
                         }
                         if (ok) {
-                            if constexpr (PREC == PREC_FP32) val = inner_unbiased_fast(ot, Rs, j, nz, work, Lv, N_l);
+                            if constexpr (PREC == PREC_FP32) val = inner_unbiased_fast(ot, Rs, load_path_option(ot.path + j), nz, work, Lv, N_l);
                             else val = inner_unbiased<RT>(ot, Rs, j, nz, work, Lv, N_l);
                         } else {                 // beyond kMaxPathSteps: the call fails
                             atomicOr(D.B.counters + CNT_ERR, 1u);

@@ -30,9 +30,11 @@ __device__ __forceinline__ RT opt_derv_stock(const OptionTable<RT>& ot, uint32_t
 
 // simulate_stock_dt<with_coarse> (gbm_approx.hpp:18-57) on the three paths S[0..3) of
 // sample_inner_approx, plus (with_coarse) the coupled coarse paths S[3..6) stepping every
-// coarse_step fine steps on the summed increments.  States in double, increments in real_t.
+// coarse_step fine steps on the summed increments.  States in double, increments in real_t.  Steps
+// are counted in 32 bits (at most kMaxPathSteps): a 64-bit remainder per step cost as much as the
+// rest of the step.
 template <class RT, class NZ>
-__device__ void stock_dt(NZ& nz, double* S, uint64_t N, RT mu, RT sigma, RT t, bool milstein,
+__device__ void stock_dt(NZ& nz, double* S, uint32_t N, RT mu, RT sigma, RT t, bool milstein,
                          bool with_coarse, uint32_t coarse_step) {
     const RT dt = xdiv(t, (RT)N);
     const RT sqrt_dt = xsqrt(dt);
@@ -40,7 +42,8 @@ __device__ void stock_dt(NZ& nz, double* S, uint64_t N, RT mu, RT sigma, RT t, b
     const double hs2 = __dmul_rn(0.5, (double)xmul(sigma, sigma));
     const RT mudt = xmul(mu, dt), mudt_c = xmul(mu, dt_c);
     RT dW_c = (RT)0;
-    for (uint64_t n = 0; n < N; n++) {
+    uint32_t k = 0;                                      // fine steps since the last coarse one
+    for (uint32_t n = 0; n < N; n++) {
         const RT dW = xmul(sqrt_dt, nz.next());
         const RT m = milstein ? to_rt<RT>(__dmul_rn(hs2, (double)xsub(xmul(dW, dW), dt))) : (RT)0;
         const double inc = (double)xadd(xadd(mudt, xmul(sigma, dW)), m);
@@ -48,7 +51,8 @@ __device__ void stock_dt(NZ& nz, double* S, uint64_t N, RT mu, RT sigma, RT t, b
         for (int i = 0; i < 3; i++) S[i] = __dadd_rn(S[i], __dmul_rn(S[i], inc));
         if (with_coarse) {
             dW_c = xadd(dW_c, dW);
-            if ((n + 1) % coarse_step == 0) {
+            if (++k == coarse_step) {
+                k = 0;
                 const RT mc = milstein ? to_rt<RT>(__dmul_rn(hs2, (double)xsub(xmul(dW_c, dW_c), dt_c))) : (RT)0;
                 const double incc = (double)xadd(xadd(mudt_c, xmul(sigma, dW_c)), mc);
 #pragma unroll
@@ -99,13 +103,13 @@ __device__ RT inner_approx(const OptionTable<RT>& ot, RT Rs, uint32_t j, NZ& nz,
     const RT dW = xmul(ot.stau, nz.next());
     const RT S0_t_1 = simulate_stock_ref<RT>(S0, r, sg, tau, dW);
     const RT S0_t_2 = simulate_stock_ref<RT>(S0, r, sg, tau, -dW);
-    const uint64_t N = (uint64_t)ot.dt_h0inv * N_l;
-    work += (double)xmul((RT)N_l, ot.W_est[j]);
+    const uint32_t n_l = (uint32_t)N_l, N = ot.dt_h0inv * n_l;     // at most kMaxPathSteps
+    work += (double)xmul((RT)n_l, ot.W_est[j]);
     double S[6] = {(double)S0_t_1, (double)Rs, (double)S0_t_2, (double)S0_t_1, (double)Rs, (double)S0_t_2};
     const RT Tr = xsub(ot.maturity[j], tau);
     if (L) {
         stock_dt<RT, NZ>(nz, S, N, r, sg, Tr, ot.use_milstein != 0, true, ot.dt_beta);
-        work += (double)xmul((RT)(N_l / ot.dt_beta), ot.W_est[j]);
+        work += (double)xmul((RT)(n_l / ot.dt_beta), ot.W_est[j]);
     } else {
         stock_dt<RT, NZ>(nz, S, N, r, sg, Tr, ot.use_milstein != 0, false, 2);
     }
@@ -146,10 +150,43 @@ __device__ __forceinline__ bool unbiased_level(const OptionTable<RT>& ot, RT u, 
 template <class RT, class NZ>
 __device__ __forceinline__ RT inner_unbiased(const OptionTable<RT>& ot, RT Rs, uint32_t j, NZ& nz,
                                              double& work, uint32_t L, uint64_t N_l) {
-    const RT ret = inner_approx<RT, NZ>(ot, Rs, j, nz, work, L, N_l);
+    return xmul(inner_approx<RT, NZ>(ot, Rs, j, nz, work, L, N_l), ot.lvl_w[L]);
+}
+
+// The weights of the Unbiased levels (sample_inner_unbiased, portfolio_sampler.cpp:531-536) in
+// reference arithmetic and on the FP32 path: two double pow, or two exponentials and a division, per
+// level instead of per sample (k_ref_records).
+template <class RT>
+__device__ __forceinline__ RT level_weight(const OptionTable<RT>& ot, uint32_t L) {
     const RT e = ot.dt_prob_expo, x = (RT)ot.dt_beta;
-    const RT Lp = to_rt<RT>(__ddiv_rn((double)xpow(x, xmul(-e, (RT)L)), __dsub_rn(1.0, (double)xpow(x, e))));
-    return xmul(ret, Lp);
+    return to_rt<RT>(__ddiv_rn((double)xpow(x, xmul(-e, (RT)L)), __dsub_rn(1.0, (double)xpow(x, e))));
+}
+__device__ __forceinline__ float level_weight_fast(float e, uint32_t beta, uint32_t L) {
+    const float lb = __log2f((float)beta);
+    return exp2f(-e * lb * (float)L) / (1.0f - exp2f(e * lb));
+}
+
+// Steps N_l = beta^L of an Unbiased level (false when h0 N_l exceeds kMaxPathSteps).
+template <class RT>
+__device__ __forceinline__ bool level_steps(const OptionTable<RT>& ot, uint32_t Lv, uint64_t& N_l) {
+    N_l = 1;
+    bool ok = true;
+    for (uint32_t i = 0; i < Lv && ok; i++) {
+        N_l *= ot.dt_beta;
+        ok = N_l * ot.dt_h0inv <= kMaxPathSteps;
+    }
+    return ok && N_l * ot.dt_h0inv <= kMaxPathSteps;
+}
+
+// The level of an OUTER uniform word by its thresholds: floor(log u / (log beta e)) in double takes
+// the same value for all words between two of them (neighbouring u differ by 2e-10 or more
+// relatively, the logarithm by 1e-16), so the two logarithms and the division per sample are a
+// comparison or two (65 % of the draws stop at the first).
+template <class RT>
+__device__ __forceinline__ bool level_of_word(const OptionTable<RT>& ot, uint32_t word, uint32_t& L, uint64_t& N_l) {
+    L = 0;
+    while (L + 1 < kPathLevels && word < ot.lvl_thr[L + 1]) L++;
+    return level_steps(ot, L, N_l);
 }
 
 // ---- FP32 versions for the batched fast path -------------------------------------------------
@@ -161,21 +198,23 @@ __device__ __forceinline__ RT inner_unbiased(const OptionTable<RT>& ot, RT Rs, u
 
 // simulate_stock_dt<with_coarse> (gbm_approx.hpp:18-57) in float increments.
 template <class NZ>
-__device__ void stock_dt_fast(NZ& nz, double* S, uint64_t N, float mu, float sigma, float t, bool milstein,
+__device__ void stock_dt_fast(NZ& nz, double* S, uint32_t N, float mu, float sigma, float t, bool milstein,
                               bool with_coarse, uint32_t coarse_step) {
     const float dt = t / (float)N;
     const float sqrt_dt = sqrtf(dt);
     const float dt_c = dt * (float)coarse_step;
     const float hs2 = milstein ? 0.5f * sigma * sigma : 0.f;
     float dW_c = 0.f;
-    for (uint64_t n = 0; n < N; n++) {
+    uint32_t k = 0;
+    for (uint32_t n = 0; n < N; n++) {
         const float dW = sqrt_dt * nz.next();
         const double inc = (double)fmaf(hs2, fmaf(dW, dW, -dt), fmaf(sigma, dW, mu * dt));
 #pragma unroll
         for (int i = 0; i < 3; i++) S[i] = fma(S[i], inc, S[i]);
         if (with_coarse) {
             dW_c += dW;
-            if ((n + 1) % coarse_step == 0) {
+            if (++k == coarse_step) {
+                k = 0;
                 const double incc = (double)fmaf(hs2, fmaf(dW_c, dW_c, -dt_c), fmaf(sigma, dW_c, mu * dt_c));
 #pragma unroll
                 for (int i = 3; i < 6; i++) S[i] = fma(S[i], incc, S[i]);
@@ -195,12 +234,11 @@ __device__ __forceinline__ float opt_derv_stock_fast(float wdisc, bool call, flo
 }
 
 template <class NZ>
-__device__ float inner_exact_fast(const OptionTable<float>& ot, float Rs, uint32_t j, NZ& nz, double& work) {
+__device__ float inner_exact_fast(const OptionTable<float>& ot, float Rs, const PathOption& o, NZ& nz, double& work) {
     const bool anti = ot.use_antithetic_risk != 0;
-    work += (double)ot.W_est[j];
-    const uint32_t s = ot.stock_ind[j];
-    const float S0 = ot.S0[s], sg = ot.sigma[s], r = ot.r, tau = ot.tau, T = ot.maturity[j], K = ot.strike[j];
-    const float m = (float)ot.type[j], Tr = T - tau, wdisc = ot.w[j] * __expf(-r * T);
+    work += (double)o.W_est;
+    const float S0 = o.S0, sg = o.sigma, r = ot.r, tau = ot.tau, T = o.maturity, K = o.strike;
+    const float m = (o.link & 1u) ? 1.f : -1.f, Tr = T - tau, wdisc = o.wgt * __expf(-r * T);
     const float mu_t = (r - 0.5f * sg * sg) * tau, mu_T = (r - 0.5f * sg * sg) * Tr;
     const float dW_0_tau = ot.stau * nz.next();
     const float dW_tau_T = sqrtf(Tr) * nz.next();
@@ -220,23 +258,22 @@ __device__ float inner_exact_fast(const OptionTable<float>& ot, float Rs, uint32
 }
 
 template <class NZ>
-__device__ float inner_approx_fast(const OptionTable<float>& ot, float Rs, uint32_t j, NZ& nz, double& work,
+__device__ float inner_approx_fast(const OptionTable<float>& ot, float Rs, const PathOption& o, NZ& nz, double& work,
                                    uint32_t L, uint64_t N_l) {
-    const uint32_t s = ot.stock_ind[j];
-    const float S0 = ot.S0[s], sg = ot.sigma[s], r = ot.r, tau = ot.tau, T = ot.maturity[j], K = ot.strike[j];
-    const float m = (float)ot.type[j], wdisc = ot.w[j] * __expf(-r * T);
+    const float S0 = o.S0, sg = o.sigma, r = ot.r, tau = ot.tau, T = o.maturity, K = o.strike;
+    const float m = (o.link & 1u) ? 1.f : -1.f, wdisc = o.wgt * __expf(-r * T);
     const float mu_t = (r - 0.5f * sg * sg) * tau;
     const float dW = ot.stau * nz.next();
     const float S0_t_1 = S0 * __expf(fmaf(sg, dW, mu_t));
     const float S0_t_2 = S0 * __expf(fmaf(-sg, dW, mu_t));
-    const uint64_t N = (uint64_t)ot.dt_h0inv * N_l;
-    const float West = ot.W_est[j];
-    work += (double)((float)N_l * West);
+    const uint32_t n_l = (uint32_t)N_l, N = ot.dt_h0inv * n_l;
+    const float West = o.W_est;
+    work += (double)((float)n_l * West);
     double S[6] = {(double)S0_t_1, (double)Rs, (double)S0_t_2, (double)S0_t_1, (double)Rs, (double)S0_t_2};
     const float Tr = T - tau;
     if (L) {
         stock_dt_fast<NZ>(nz, S, N, r, sg, Tr, ot.use_milstein != 0, true, ot.dt_beta);
-        work += (double)((float)(N_l / ot.dt_beta) * West);
+        work += (double)((float)(n_l / ot.dt_beta) * West);
     } else {
         stock_dt_fast<NZ>(nz, S, N, r, sg, Tr, ot.use_milstein != 0, false, 2);
     }
@@ -261,11 +298,9 @@ __device__ float inner_approx_fast(const OptionTable<float>& ot, float Rs, uint3
 
 // sample_inner_unbiased (521-537): ret * beta^{-e L} / (1 - beta^e), the weight in float
 template <class NZ>
-__device__ __forceinline__ float inner_unbiased_fast(const OptionTable<float>& ot, float Rs, uint32_t j, NZ& nz,
+__device__ __forceinline__ float inner_unbiased_fast(const OptionTable<float>& ot, float Rs, const PathOption& o, NZ& nz,
                                                      double& work, uint32_t L, uint64_t N_l) {
-    const float ret = inner_approx_fast<NZ>(ot, Rs, j, nz, work, L, N_l);
-    const float e = ot.dt_prob_expo, lb = __log2f((float)ot.dt_beta);
-    return ret * (exp2f(-e * lb * (float)L) / (1.0f - exp2f(e * lb)));
+    return inner_approx_fast<NZ>(ot, Rs, o, nz, work, L, N_l) * ot.lvl_wf[L];
 }
 
 }  // namespace nmlmc
