@@ -148,17 +148,21 @@ __global__ void __launch_bounds__(256) k_adj_setup(AdjLaunch<RT> A, AdjInputs in
 template <class RT>
 struct PairSums { RT C, dC; };
 
-template <class RT, bool TAN>
+// Products that a sum follows are rounded on their own (no contraction), whatever MIL is.
+__device__ __forceinline__ float rmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double rmul(double a, double b) { return __dmul_rn(a, b); }
+
+// MIL: Milstein steps, else Euler.
+template <class RT, bool TAN, bool MIL>
 struct AntitheticPaths {
     RT Sp, Sm, Dp, Dm;
     __device__ __forceinline__ void start(RT R, RT dR) { Sp = Sm = R; Dp = Dm = dR; }
-    // one Milstein (or Euler) step of both paths on the normal z (gbm_approx.hpp:18-57)
-    __device__ __forceinline__ void step(RT z, RT sh, RT h, RT rh1, RT sg, RT hs2, bool milstein) {
+    // one step of both paths on the normal z (gbm_approx.hpp:18-57)
+    __device__ __forceinline__ void step(RT z, RT sh, RT h, RT rh1, RT sg, RT hs2) {
         const RT dW = sh * z;
-        const RT corr = milstein ? hs2 * (dW * dW - h) : (RT)0;
+        const RT q = dW * dW - h, corr = MIL ? rmul(hs2, q) : (RT)0, dc = MIL ? rmul(sg, q) : (RT)0;
         const RT gp = rh1 + sg * dW + corr, gm = rh1 - sg * dW + corr;
         if (TAN) {
-            const RT dc = milstein ? sg * (dW * dW - h) : (RT)0;
             Dp = Dp * gp + Sp * (dW + dc);
             Dm = Dm * gm + Sm * (dc - dW);
         }
@@ -184,7 +188,7 @@ enum AdjMode { ADJ_LOSS, ADJ_STORE, ADJ_PULL };
 // k_adj_weights multiply are kept (two RT per option and outer sample, 8 bytes in FP32: 205 MB
 // written and read once for 1e5 options x 256 outer samples, 0.06 ms of HBM time) instead of
 // drawing and stepping every path a second time (4.4 ms).
-template <class RT, int MODE>
+template <class RT, int MODE, bool MIL>
 __global__ void __launch_bounds__(kAdjThreads) k_adj_paths(AdjLaunch<RT> A) {
     constexpr bool TAN = MODE != ADJ_LOSS;
     extern __shared__ double adj_sh[];                  // [tile][warps] | 2 * Qmax (ADJ_PULL)
@@ -219,7 +223,6 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_paths(AdjLaunch<RT> A) {
     const RT V0 = A.V0[i], vega = A.vega[i];
     const RT invN = (RT)1 / (RT)A.pairs;
     const uint64_t ctr1 = ((uint64_t)il << 32) | PH_ADJOINT;
-    const bool mil = A.milstein != 0;
 
     double gwE = 0, gwP = 0, gsE = 0, gsP = 0;
     for (uint64_t m = m0; m < m1; m++) {
@@ -228,7 +231,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_paths(AdjLaunch<RT> A) {
         const RT Rt = A.R[ridx];
         const RT Dt = TAN ? A.dR[ridx] : (RT)0;
         PairSums<RT> sum{(RT)0, (RT)0};
-        AntitheticPaths<RT, TAN> S;
+        AntitheticPaths<RT, TAN, MIL> S;
         RT z[4];
         if (steps >= 4) {                                // a path takes whole blocks of four normals
             uint64_t blk = 0;
@@ -240,7 +243,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_paths(AdjLaunch<RT> A) {
                     threefry2x64(blk, ctr1, key, v0, v1);
                     normals4<RT>(v0, v1, z);
 #pragma unroll
-                    for (int e = 0; e < 4; e++) S.step(z[e], sh, h, rh1, sg, hs2, mil);
+                    for (int e = 0; e < 4; e++) S.step(z[e], sh, h, rh1, sg, hs2);
                 }
                 S.payoff(type, K, sum);
             }
@@ -255,7 +258,7 @@ __global__ void __launch_bounds__(kAdjThreads) k_adj_paths(AdjLaunch<RT> A) {
                         threefry2x64(q >> 2, ctr1, key, v0, v1);
                         normals4<RT>(v0, v1, z);
                     }
-                    S.step(e == 0 ? z[0] : (e == 1 ? z[1] : (e == 2 ? z[2] : z[3])), sh, h, rh1, sg, hs2, mil);
+                    S.step(e == 0 ? z[0] : (e == 1 ? z[1] : (e == 2 ? z[2] : z[3])), sh, h, rh1, sg, hs2);
                 }
                 S.payoff(type, K, sum);
             }
@@ -366,8 +369,8 @@ uint32_t adj_tile(const AdjLaunch<RT>& A, uint64_t rows_m, uint64_t ctas, uint64
     return (uint32_t)(t < 1 ? 1 : (t < cap ? t : cap));
 }
 
-template <class RT, int MODE>
-cudaError_t launch_paths(AdjLaunch<RT> A, uint64_t m0, uint64_t m1, cudaStream_t stream) {
+template <class RT, int MODE, bool MIL>
+cudaError_t launch_paths_m(AdjLaunch<RT> A, uint64_t m0, uint64_t m1, cudaStream_t stream) {
     if (m0 >= m1) return cudaSuccess;
     A.m0 = m0;
     A.m1 = m1;
@@ -375,17 +378,22 @@ cudaError_t launch_paths(AdjLaunch<RT> A, uint64_t m0, uint64_t m1, cudaStream_t
     const uint64_t per = A.tile;
     const size_t sh = MODE == ADJ_PULL ? (size_t)2 * A.q_max * sizeof(double) : per * (kAdjThreads / 32) * sizeof(double);
     if (sh > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_adj_paths<RT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
+        cudaError_t e = cudaFuncSetAttribute(k_adj_paths<RT, MODE, MIL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh);
         if (e != cudaSuccess) return e;
     }
     for (uint64_t a = m0; a < m1; a += per * 65535) {     // at most 65,535 rows of tiles per launch
         A.m0 = a;
         A.m1 = m1 - a < per * 65535 ? m1 : a + per * 65535;
         const dim3 grid(A.n_chunks, (uint32_t)((A.m1 - a + per - 1) / per));
-        k_adj_paths<RT, MODE><<<grid, kAdjThreads, sh, stream>>>(A);
+        k_adj_paths<RT, MODE, MIL><<<grid, kAdjThreads, sh, stream>>>(A);
         count_launch();
     }
     return cudaGetLastError();
+}
+
+template <class RT, int MODE>
+cudaError_t launch_paths(const AdjLaunch<RT>& A, uint64_t m0, uint64_t m1, cudaStream_t stream) {
+    return A.milstein ? launch_paths_m<RT, MODE, true>(A, m0, m1, stream) : launch_paths_m<RT, MODE, false>(A, m0, m1, stream);
 }
 
 template <class RT>
