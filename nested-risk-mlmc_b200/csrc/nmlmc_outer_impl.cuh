@@ -13,6 +13,8 @@
 // stream (key = (seed, level<<56 | index), counter = (block, phase tag)), which makes each
 // inner sample addressable, and a level call runs breadth-first:
 //
+// (a level call of few outer samples runs as k_small instead, a model's at small fixed counts as
+// k_fixed, both below)
 //   k_outer      one thread per outer sample: outer draws (Y, or R_tau row + constant)
 //   k_phase      pilot round r: every outer sample still refining, fine and coarse, as
 //                uniform-size segments; one thread per chunk of inner samples, block-segmented
@@ -1034,8 +1036,8 @@ __device__ __forceinline__ uint32_t pilots_taken(uint32_t cnt, const CountParams
 // nothing and touches no slot), the counts of items that hit the maximum / stayed at the base
 // count, and the trace record.
 template <class RT, int KIND, class S, int STRIDE = kTile>
-__device__ __forceinline__ void final_item(const DevLevel<RT>& D, uint32_t item, RT mean_big, RT phi_small,
-                                           bool fine_big, double* mom, uint32_t& n_max, uint32_t& n_base,
+__device__ __forceinline__ void final_item(const DevLevel<RT>& D, uint64_t item, uint32_t cf, uint32_t cc, RT mean_big,
+                                           RT phi_small, bool fine_big, double* mom, uint32_t& n_max, uint32_t& n_base,
                                            TraceRec* trace) {
     RT phi_big = (RT)phi_of<KIND, S, RT>(mean_big, 1.f);
     RT f_phi, c_phi;
@@ -1055,13 +1057,12 @@ __device__ __forceinline__ void final_item(const DevLevel<RT>& D, uint32_t item,
             for (int q = 0; q < 4; q++) { p = xmul(p, dphi); mom[(4 + q) * STRIDE] += (double)p; }
         }
     }
-    const uint32_t cf = D.B.cnt_f[item];
     n_max += (cf == (uint32_t)D.L.cf.max_count) ? 1u : 0u;
     n_base += (cf == (uint32_t)D.L.cf.base_count) ? 1u : 0u;
     if (trace) {
         TraceRec tr;
         tr.count_f = cf;
-        tr.count_c = D.L.fine_only ? 0 : D.B.cnt_c[item];
+        tr.count_c = D.L.fine_only ? 0 : cc;
         tr.phi_f = (double)f_phi;
         tr.phi_c = (double)c_phi;
         tr.mean_big = (double)mean_big;
@@ -1110,6 +1111,38 @@ __device__ __forceinline__ void level_finish(const OuterBuffers& B, int slots) {
     if (t == 0) {
         B.counters[CNT_DONE] = 0;
         level_stamp(B.stamps, 1);
+    }
+}
+
+// A CTA's threads' work, moments (mom[q kTile], q = 0..7) and counts, and the warps' sm_acc entries,
+// into its partial-sum slot (added to it, or stored).  All kTile threads call it.
+__device__ __forceinline__ void cta_sums(const OuterBuffers& B, double wsum, uint32_t n_max, uint32_t n_base, const double* mom,
+                                         double (*sm_acc)[16], bool add) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    for (int m = 16; m > 0; m >>= 1) {
+        wsum += __shfl_down_sync(0xffffffffu, wsum, m);
+        n_max += __shfl_down_sync(0xffffffffu, n_max, m);
+        n_base += __shfl_down_sync(0xffffffffu, n_base, m);
+    }
+    double mv[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        mv[q] = mom[q * kTile];
+        for (int m = 16; m > 0; m >>= 1) mv[q] += __shfl_down_sync(0xffffffffu, mv[q], m);
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int q = 0; q < 8; q++) sm_acc[warp][q] += mv[q];
+        sm_acc[warp][8] += wsum;
+        sm_acc[warp][10] += (double)n_max;
+        sm_acc[warp][11] += (double)n_base;
+    }
+    __syncthreads();
+    if (t < 16) {
+        double v = 0;
+        for (int w = 0; w < kWarps; w++) v += sm_acc[w][t];
+        double* to = B.block_sums + (size_t)blockIdx.x * 16 + t;
+        *to = add ? *to + v : v;
     }
 }
 
@@ -1254,8 +1287,8 @@ __global__ void __launch_bounds__(kTile, MINB) k_phase(DevLevel<RT> D, SegSet SS
                     const bool surv = leader && pilot_decide<RT, PREC>(D, g, item, start, a1, a2);
                     warp_append(surv, item, counters + g.next_slot, g.next_list, lane);
                 } else if (leader) {
-                    final_item<RT, KIND, S>(D, item, inner_mean<RT, PREC>(start, a1, g.count), (RT)ind, fine_big, mom,
-                                   n_max, n_base, trace);
+                    final_item<RT, KIND, S>(D, item, D.B.cnt_f[item], D.B.cnt_c[item], inner_mean<RT, PREC>(start, a1, g.count),
+                                            (RT)ind, fine_big, mom, n_max, n_base, trace);
                 }
                 if (t == 0) sm_ticket = next;
                 __syncthreads();
@@ -1344,8 +1377,9 @@ __global__ void __launch_bounds__(kTile, MINB) k_phase(DevLevel<RT> D, SegSet SS
                         if (pilot_decide<RT, PREC>(D, g, item, start, tot1, tot2))
                             g.next_list[atomicAdd(&counters[g.next_slot], 1u)] = item;
                     } else {
-                        final_item<RT, KIND, S>(D, item, inner_mean<RT, PREC>(start, tot1, g.count), (RT)tind, fine_big, mom,
-                                       n_max, n_base, trace);
+                        final_item<RT, KIND, S>(D, item, D.B.cnt_f[item], D.B.cnt_c[item],
+                                                inner_mean<RT, PREC>(start, tot1, g.count), (RT)tind, fine_big, mom, n_max,
+                                                n_base, trace);
                     }
                     sm_ticket = next;
                 }
@@ -1354,31 +1388,7 @@ __global__ void __launch_bounds__(kTile, MINB) k_phase(DevLevel<RT> D, SegSet SS
             }
         }
     }
-    // this thread's work, moments and counts -> per-warp sums -> this CTA's partial-sum slot
-    for (int m = 16; m > 0; m >>= 1) {
-        wsum += __shfl_down_sync(0xffffffffu, wsum, m);
-        n_max += __shfl_down_sync(0xffffffffu, n_max, m);
-        n_base += __shfl_down_sync(0xffffffffu, n_base, m);
-    }
-    double mv[8];
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-        mv[q] = mom[q * kTile];
-        for (int m = 16; m > 0; m >>= 1) mv[q] += __shfl_down_sync(0xffffffffu, mv[q], m);
-    }
-    if (lane == 0) {
-#pragma unroll
-        for (int q = 0; q < 8; q++) sm_acc[warp][q] += mv[q];
-        sm_acc[warp][8] += wsum;
-        sm_acc[warp][10] += (double)n_max;
-        sm_acc[warp][11] += (double)n_base;
-    }
-    __syncthreads();
-    if (t < 16) {
-        double v = 0;
-        for (int w = 0; w < kWarps; w++) v += sm_acc[w][t];
-        D.B.block_sums[(size_t)blockIdx.x * 16 + t] += v;
-    }
+    cta_sums(D.B, wsum, n_max, n_base, mom, sm_acc, true);
     if (SS.reduce) level_finish<kTile>(D.B, D.B.slots);
 }
 
@@ -1739,12 +1749,9 @@ __global__ void __launch_bounds__(kSmallThreads) k_small(DevLevel<RT> D, uint32_
         Acc<PREC> a1, a2;
         float ind;
         w.phase(PH_FINAL, big, false, gs, small, (float)gs / (float)nch, a1, a2, ind);
-        if (lane == 0) {
-            D.B.cnt_f[item] = cf;
-            D.B.cnt_c[item] = cc;
-            final_item<RT, KIND, NoSampler, kSmallWarps>(D, item, inner_mean<RT, PREC>(w.start, a1, big), (RT)ind, fine_big,
-                                                         sm_mom + warp, n_max, n_base, trace);
-        }
+        if (lane == 0)
+            final_item<RT, KIND, NoSampler, kSmallWarps>(D, item, cf, cc, inner_mean<RT, PREC>(w.start, a1, big), (RT)ind,
+                                                         fine_big, sm_mom + warp, n_max, n_base, trace);
         __syncwarp();
     }
     double ws = w.work;
@@ -1926,6 +1933,100 @@ static cudaError_t run_batch(DevLevel<RT>& D, uint32_t nb, TraceRec* trace, cuda
     return cudaSuccess;
 }
 
+// ---- models at small fixed counts: a thread per outer sample ---------------------------------
+// Level 0 (and every level without pilots) of a model at up to kFixedChunks chunks per outer
+// sample: the thread draws its outer sample and its chunks, merges them in k_phase's order (pairs,
+// then pairs of pairs) and adds its phi — no outer draws and counts written and read back (12 bytes
+// per sample each way), no tickets and no barriers per tile.  Bound by the ALU pipe of the counter
+// generator (9 blocks per level-0 sample of 32): 12e6 samples at level 0 892 -> 855 us, 33,000 48 -> 36
+// us, 4e6 at level 1 (64 and 32) 613 -> 545 us against the launch sequence.
+constexpr uint32_t kFixedChunks = 4;
+
+template <class RT, int KIND, int PREC>
+__global__ void __launch_bounds__(kTile, PREC == PREC_FP32 ? 4 : 2) k_fixed(DevLevel<RT> D, TraceRec* trace) {
+    __shared__ double sm_mom[8 * kTile];
+    __shared__ double sm_acc[kWarps][16];
+    const OuterLevel<RT>& L = D.L;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const uint64_t gid = (uint64_t)blockIdx.x * kTile + t;
+    if (gid == 0) level_stamp(D.B.stamps, 0);
+    double* mom = sm_mom + t;
+#pragma unroll
+    for (int q = 0; q < 8; q++) mom[q * kTile] = 0;
+    if (lane < 16) sm_acc[warp][lane] = 0;
+    __syncwarp();
+    const uint32_t C = L.chunk, cf = (uint32_t)L.cf.max_count, cc = (uint32_t)L.cc.max_count;
+    const bool fine_big = L.fine_only || cf > cc;
+    const uint32_t big = fine_big ? cf : cc, small = L.fine_only ? big : (fine_big ? cc : cf);
+    const uint32_t nch = big / C, gs = small / C;
+    const float coeff = (float)gs / (float)nch;
+    const RT start = -L.mp.max_loss;
+    double wsum = 0;
+    uint32_t n_max = 0, n_base = 0;
+    if (gid == 0) sm_acc[0][9] = (double)L.M * (double)big;
+    for (uint64_t i = gid; i < L.M; i += (uint64_t)gridDim.x * kTile) {
+        const TfKey key = tf_key(L.seed, outer_stream_id(L.ell, L.first_index + i));
+        const RT Y = outer_normal_at<PREC, RT>(key, PH_OUTER, 0);
+        Acc<PREC> a1, one, two;
+        one.zero();
+        two.zero();
+        float ind = 0.f;
+        for (uint32_t j = 0; j < nch; j++) {
+            a1.zero();
+            if constexpr (KIND == KIND_SHIFT_MODEL) {
+#pragma unroll 2
+                for (uint32_t b = 0; b < C / 4; b++) {
+                    uint64_t v0, v1;
+                    threefry2x64((uint64_t)(j * (C / 4) + b), PH_FINAL, key, v0, v1);
+                    RT d[4];
+                    shift_values<PREC, RT>(v0, v1, Y, d);
+                    a1.add2(d[0], d[1]);
+                    a1.add2(d[2], d[3]);
+                }
+            } else {
+#pragma unroll 2
+                for (uint32_t b = 0; b < C / 2; b++) {
+                    uint64_t v0, v1;
+                    threefry2x64((uint64_t)(j * (C / 2) + b), PH_FINAL, key, v0, v1);
+                    RT d[2];
+                    ref_values<PREC, RT>(v0, v1, Y, L.mp.stau, L.mp.s1tau, d);
+                    a1.add2(d[0], d[1]);
+                }
+            }
+            // the butterfly of k_phase, in chunk order
+            if (gs == 1) ind += phi_of<KIND, NoSampler, RT>(inner_mean<RT, PREC>(start, a1, small), coeff);
+            if (!(j & 1)) { one = a1; continue; }
+            one.merge(a1);
+            a1 = one;
+            if (gs == 2) ind += phi_of<KIND, NoSampler, RT>(inner_mean<RT, PREC>(start, a1, small), coeff);
+            if (!(j & 2)) { two = a1; continue; }
+            two.merge(a1);
+            a1 = two;
+        }
+        const Acc<PREC>& all = nch == 1 ? one : nch == 2 ? two : a1;
+        wsum += (double)big;
+        final_item<RT, KIND, NoSampler>(D, i, cf, cc, inner_mean<RT, PREC>(start, all, big), (RT)ind, fine_big, mom, n_max,
+                                        n_base, trace);
+    }
+    __syncthreads();
+    cta_sums(D.B, wsum, n_max, n_base, mom, sm_acc, false);
+    level_finish<kTile>(D.B, gridDim.x);
+}
+
+template <class RT, int KIND, int PREC>
+static int fixed_grid(int cap) {
+    static int g = 0;
+    if (g == 0) {
+        int dev = 0, sms = 148, per_sm = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fixed<RT, KIND, PREC>, kTile, 0) != cudaSuccess || per_sm < 1)
+            per_sm = 1;
+        g = per_sm * sms;
+    }
+    return g < cap ? g : cap;
+}
+
 template <class RT, int KIND, int PREC, class S = NoSampler>
 cudaError_t sample_level_t(const OuterLevel<RT>& L, OuterBuffers& B, TraceRec* trace,
                                   cudaStream_t stream) {
@@ -1938,6 +2039,18 @@ cudaError_t sample_level_t(const OuterLevel<RT>& L, OuterBuffers& B, TraceRec* t
             const int grid = (int)(ctas < (uint64_t)B.grid ? ctas : (uint64_t)B.grid);
             const size_t rows = is_portfolio_kind(KIND) ? kSmallWarps * (size_t)L.ot.Q * sizeof(float2) : 0;
             k_small<RT, KIND, PREC><<<grid, kSmallThreads, rows, stream>>>(D, (uint32_t)L.M, trace);
+            count_launch();
+            return cudaGetLastError();
+        }
+    }
+    if constexpr (KIND == KIND_REF_MODEL || KIND == KIND_SHIFT_MODEL) {
+        const uint64_t maxc = (L.fine_only || L.cf.max_count >= L.cc.max_count) ? L.cf.max_count : L.cc.max_count;
+        if (!L.adaptive_f && !L.adaptive_c && maxc / L.chunk <= kFixedChunks) {
+            const uint64_t ctas = (L.M + kTile - 1) / kTile;
+            const int grid = fixed_grid<RT, KIND, PREC>((int)(ctas < (uint64_t)B.grid ? ctas : (uint64_t)B.grid));
+            if (B.prof_mark) B.prof_mark(B.prof_user, 0, stream);
+            k_fixed<RT, KIND, PREC><<<grid, kTile, 0, stream>>>(D, trace);
+            if (B.prof_mark) B.prof_mark(B.prof_user, 1, stream);
             count_launch();
             return cudaGetLastError();
         }
