@@ -131,12 +131,14 @@ __device__ __forceinline__ F2 option_loss_fast2(const FastOption& o, F2 R, F2 ln
 
 // The same loss from an alias column: m d1 as above, m s = 1 / (m inv_s) from the SFU estimate
 // (within one ulp of the record's m s, the only difference from option_loss_fast; one ulp of s
-// moves Phi(d2) by less than 2e-8).
+// moves Phi(d2) by less than 2e-8).  The two Phi share their instructions
+// (f32x2): 4 to 6 % of a large-portfolio level, whose loop waits for its gathers with few registers to
+// spare; on the records of uniform sub-sampling it does not pay (20 stocks, level 6: 504 -> 517 us).
 __device__ __forceinline__ float column_loss_fast(const FastColumn& c, float R, float lnR) {
     const float d1 = (lnR + c.c1) * c.inv_s;
     const float d2 = d1 - rcp_sfu(c.inv_s);
-    const float n1 = norm_cdf_fast(d1), n2 = norm_cdf_fast(d2);
-    const float v = fmaf(c.wR * R, n1, fmaf(c.wK, n2, c.wV0));
+    const F2 n = norm_cdf_fast2(f2(d1, d2));
+    const float v = fmaf(c.wR * R, f2_lo(n), fmaf(c.wK, f2_hi(n), c.wV0));
     return fmaf(c.cv, R, v);
 }
 #endif

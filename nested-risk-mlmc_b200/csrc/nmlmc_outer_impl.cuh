@@ -338,12 +338,18 @@ __device__ __forceinline__ FastOption load_record_l1(const FastOption* p) {
     o.stock = __float_as_uint(st);
     return o;
 }
+template <bool L1 = false>
 __device__ __forceinline__ FastColumn load_column(const FastColumn* p) {
     FastColumn c;
     float thr, link;
-    asm("ld.global.nc.L1::no_allocate.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-        : "=f"(c.c1), "=f"(c.inv_s), "=f"(c.wR), "=f"(c.wK), "=f"(c.wV0), "=f"(c.cv), "=f"(thr), "=f"(link)
-        : "l"(p));
+    if (L1)
+        asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+            : "=f"(c.c1), "=f"(c.inv_s), "=f"(c.wR), "=f"(c.wK), "=f"(c.wV0), "=f"(c.cv), "=f"(thr), "=f"(link)
+            : "l"(p));
+    else
+        asm("ld.global.nc.L1::no_allocate.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+            : "=f"(c.c1), "=f"(c.inv_s), "=f"(c.wR), "=f"(c.wK), "=f"(c.wV0), "=f"(c.cv), "=f"(thr), "=f"(link)
+            : "l"(p));
     c.thr = __float_as_uint(thr);
     c.link = __float_as_uint(link);
     return c;
@@ -354,8 +360,16 @@ __device__ __forceinline__ FastColumn load_column(const FastColumn* p) {
 // says so).
 // PF_COLUMN_PIPE: the alias columns with the next four samples' gathers issued before the current
 // four are evaluated (the 128-register variant).
-enum PfMode : int { PF_UNIFORM = 0, PF_ALIAS = 1, PF_COLUMN = 2, PF_COLUMN_PIPE = 3, PF_UNIFORM_L1 = 4 };
+// Each way is an instantiation of its own of the phase kernel, with its own registers and code
+// (PF_GENERIC: the reference-arithmetic table, and every other kind).
+enum PfMode : int { PF_GENERIC = -1, PF_UNIFORM = 0, PF_ALIAS = 1, PF_COLUMN = 2, PF_COLUMN_PIPE = 3, PF_UNIFORM_L1 = 4,
+                    PF_COLUMN_L1 = 5 };
+constexpr bool is_column(int mode) { return mode == PF_COLUMN || mode == PF_COLUMN_PIPE || mode == PF_COLUMN_L1; }
 constexpr uint64_t kL1TableBytes = 1ull << 20;   // uniform draws from tables up to 1 MB read through L1
+// Alias columns of up to 8192 options (256 KB) are read through L1: gathers past it of so few lines
+// queue at their L2 slices.  20 stocks, level 6, 20,001 outer samples at 4096 inner, through L1 and past
+// it: 1000 options 513 and 1498 us, 4000 560 and 765, 6000 612 and 688, 10,000 615 and 588.
+__host__ __device__ __forceinline__ bool columns_in_l1(const OptionTable<float>& ot) { return ot.P <= 8192; }
 
 // Loss of the option drawn by the 64-bit value v: column j = floor(v P / 2^64), alias coin
 // (v P mod 2^64) >> 32, the option kept when coin < threshold and its alias otherwise (the same
@@ -364,9 +378,9 @@ template <int MODE>
 __device__ __forceinline__ float pf_sample_loss(uint64_t v, const OptionTable<float>& ot, const float2* Rrow) {
     uint32_t j, coin;
     draw_column(v, ot.P, j, coin);
-    if (MODE == PF_COLUMN) {
-        FastColumn c = load_column(ot.fast_col + j);
-        if (coin >= c.thr) c = load_column(ot.fast_col + (c.link >> 8));
+    if (is_column(MODE)) {
+        FastColumn c = load_column<MODE == PF_COLUMN_L1>(ot.fast_col + j);
+        if (coin >= c.thr) c = load_column<MODE == PF_COLUMN_L1>(ot.fast_col + (c.link >> 8));
         const float2 r = Rrow[c.link & 0xffu];
         return column_loss_fast(c, r.x, r.y);
     }
@@ -382,6 +396,7 @@ __device__ __forceinline__ float pf_sample_loss(uint64_t v, const OptionTable<fl
 
 // Four samples of the alias-column path: the Threefry blocks blk, blk + 1 and the four column
 // gathers they select (issued together, not waited for).
+template <bool L1>
 __device__ __forceinline__ void column_issue(const TfKey& key, uint32_t tag, uint64_t blk, const OptionTable<float>& ot,
                                              FastColumn (&c)[4], uint32_t (&coin)[4]) {
     uint64_t v[4];
@@ -391,18 +406,18 @@ __device__ __forceinline__ void column_issue(const TfKey& key, uint32_t tag, uin
     for (int q = 0; q < 4; q++) {
         uint32_t j;
         draw_column(v[q], ot.P, j, coin[q]);
-        c[q] = load_column(ot.fast_col + j);
+        c[q] = load_column<L1>(ot.fast_col + j);
     }
 }
 
 // The rest of those four samples: the alias-column gathers of the draws whose coin asks for them,
 // then the four losses, added to the sums in sample order (pairs into the compensated sum).
-template <int PREC, bool S2>
+template <int PREC, bool S2, int MODE>
 __device__ __forceinline__ void column_finish(FastColumn (&c)[4], const uint32_t (&coin)[4], const OptionTable<float>& ot,
                                               const float2* Rrow, float shift, Acc<PREC>& a1, Acc<PREC>& a2) {
 #pragma unroll
     for (int q = 0; q < 4; q++)
-        if (coin[q] >= c[q].thr) c[q] = load_column(ot.fast_col + (c[q].link >> 8));
+        if (coin[q] >= c[q].thr) c[q] = load_column<MODE == PF_COLUMN_L1>(ot.fast_col + (c[q].link >> 8));
     float x[4];
 #pragma unroll
     for (int q = 0; q < 4; q++) {
@@ -426,26 +441,26 @@ template <int PREC, uint32_t C, bool S2, int MODE>
 __device__ __forceinline__ void pf_chunk_fast(const TfKey& key, uint32_t tag, uint64_t b0,
                                               const OptionTable<float>& ot, const float2* Rrow, float shift,
                                               Acc<PREC>& a1, Acc<PREC>& a2) {
-    if constexpr (MODE == PF_COLUMN) {
+    if constexpr (is_column(MODE) && MODE != PF_COLUMN_PIPE) {
 #pragma unroll 1
         for (uint32_t b = 0; b < C / 2; b += 2) {
             FastColumn c[4];
             uint32_t coin[4];
-            column_issue(key, tag, b0 + b, ot, c, coin);
-            column_finish<PREC, S2>(c, coin, ot, Rrow, shift, a1, a2);
+            column_issue<MODE == PF_COLUMN_L1>(key, tag, b0 + b, ot, c, coin);
+            column_finish<PREC, S2, MODE>(c, coin, ot, Rrow, shift, a1, a2);
         }
     } else if constexpr (MODE == PF_COLUMN_PIPE) {
         constexpr uint32_t G = C / 4;           // groups of four samples
         FastColumn ca[4], cb[4];
         uint32_t ka[4], kb[4];
-        column_issue(key, tag, b0, ot, ca, ka);
+        column_issue<false>(key, tag, b0, ot, ca, ka);
 #pragma unroll 1
         for (uint32_t g = 0; g < G; g += 2) {
-            if (g + 1 < G) column_issue(key, tag, b0 + 2 * (g + 1), ot, cb, kb);
-            column_finish<PREC, S2>(ca, ka, ot, Rrow, shift, a1, a2);
+            if (g + 1 < G) column_issue<false>(key, tag, b0 + 2 * (g + 1), ot, cb, kb);
+            column_finish<PREC, S2, MODE>(ca, ka, ot, Rrow, shift, a1, a2);
             if (g + 1 < G) {
-                if (g + 2 < G) column_issue(key, tag, b0 + 2 * (g + 2), ot, ca, ka);
-                column_finish<PREC, S2>(cb, kb, ot, Rrow, shift, a1, a2);
+                if (g + 2 < G) column_issue<false>(key, tag, b0 + 2 * (g + 2), ot, ca, ka);
+                column_finish<PREC, S2, MODE>(cb, kb, ot, Rrow, shift, a1, a2);
             }
         }
     } else {
@@ -759,7 +774,7 @@ __device__ __forceinline__ void pf_paths_sorted(const DevLevel<float>& D, const 
     }
 }
 
-template <class RT, int KIND, int PREC, uint32_t C, bool S2, class S, bool PIPE>
+template <class RT, int KIND, int PREC, uint32_t C, bool S2, class S, int PM>
 __device__ __forceinline__ void eval_chunk_c(const DevLevel<RT>& D, uint32_t item, uint32_t tag,
                                              uint64_t s0, uint64_t count, float shift, const float2* srow,
                                              Acc<PREC>& a1, Acc<PREC>& a2, double& work, bool own) {
@@ -821,7 +836,7 @@ __device__ __forceinline__ void eval_chunk_c(const DevLevel<RT>& D, uint32_t ite
             a1.add2(X[0], X[1]);
         }
         work += (double)C;
-    } else if (KIND == KIND_PORTFOLIO && PREC == PREC_FP32 && L.ot.fast_s) {
+    } else if constexpr (KIND == KIND_PORTFOLIO && PREC == PREC_FP32 && PM != PF_GENERIC) {
         // portfolio, FP32: packed records scaled by 1 / (sampling probability), the SFU
         // Black-Scholes (nmlmc_bs.cuh); X = loss_j / phat_j.  srow: the outer sample's R_tau row
         // staged in shared memory, else read from the batch buffer.
@@ -829,20 +844,8 @@ __device__ __forceinline__ void eval_chunk_c(const DevLevel<RT>& D, uint32_t ite
             const OptionTable<float>& ot = L.ot;
             const float2* grow = reinterpret_cast<const float2*>(D.B.Rt) + (size_t)item * ot.Q;
             const uint64_t b0 = s0 >> 1;
-            if (ot.fast_col) {
-                constexpr int CM = PIPE ? PF_COLUMN_PIPE : PF_COLUMN;
-                if (srow) pf_chunk_fast<PREC, C, S2, CM>(key, tag, b0, ot, srow, shift, a1, a2);
-                else pf_chunk_fast<PREC, C, S2, CM>(key, tag, b0, ot, grow, shift, a1, a2);
-            } else if (ot.subsample == SUB_UNIFORM && (uint64_t)ot.P * sizeof(FastOption) <= kL1TableBytes) {
-                if (srow) pf_chunk_fast<PREC, C, S2, PF_UNIFORM_L1>(key, tag, b0, ot, srow, shift, a1, a2);
-                else pf_chunk_fast<PREC, C, S2, PF_UNIFORM_L1>(key, tag, b0, ot, grow, shift, a1, a2);
-            } else if (ot.subsample == SUB_UNIFORM) {
-                if (srow) pf_chunk_fast<PREC, C, S2, PF_UNIFORM>(key, tag, b0, ot, srow, shift, a1, a2);
-                else pf_chunk_fast<PREC, C, S2, PF_UNIFORM>(key, tag, b0, ot, grow, shift, a1, a2);
-            } else {
-                if (srow) pf_chunk_fast<PREC, C, S2, PF_ALIAS>(key, tag, b0, ot, srow, shift, a1, a2);
-                else pf_chunk_fast<PREC, C, S2, PF_ALIAS>(key, tag, b0, ot, grow, shift, a1, a2);
-            }
+            if (srow) pf_chunk_fast<PREC, C, S2, PM>(key, tag, b0, ot, srow, shift, a1, a2);
+            else pf_chunk_fast<PREC, C, S2, PM>(key, tag, b0, ot, grow, shift, a1, a2);
         }
         work += (double)C;
     } else if constexpr (KIND == KIND_PF_PATHS && PREC == PREC_FP32 && C <= kPathSortChunk) {
@@ -903,17 +906,17 @@ __device__ __forceinline__ void eval_chunk_c(const DevLevel<RT>& D, uint32_t ite
     }
 }
 
-template <class RT, int KIND, int PREC, bool S2, class S, bool PIPE>
+template <class RT, int KIND, int PREC, bool S2, class S, int PM>
 __device__ __forceinline__ void eval_chunk_s(const DevLevel<RT>& D, uint32_t item, uint32_t tag,
                                              uint64_t s0, uint64_t count, uint32_t C, float shift,
                                              const float2* srow, Acc<PREC>& a1, Acc<PREC>& a2, double& work,
                                              bool own) {
     switch (C) {
-    case 64: eval_chunk_c<RT, KIND, PREC, 64, S2, S, PIPE>(D, item, tag, s0, count, shift, srow, a1, a2, work, own); break;
-    case 32: eval_chunk_c<RT, KIND, PREC, 32, S2, S, PIPE>(D, item, tag, s0, count, shift, srow, a1, a2, work, own); break;
-    case 16: eval_chunk_c<RT, KIND, PREC, 16, S2, S, PIPE>(D, item, tag, s0, count, shift, srow, a1, a2, work, own); break;
-    case 8: eval_chunk_c<RT, KIND, PREC, 8, S2, S, PIPE>(D, item, tag, s0, count, shift, srow, a1, a2, work, own); break;
-    default: eval_chunk_c<RT, KIND, PREC, 4, S2, S, PIPE>(D, item, tag, s0, count, shift, srow, a1, a2, work, own); break;
+    case 64: eval_chunk_c<RT, KIND, PREC, 64, S2, S, PM>(D, item, tag, s0, count, shift, srow, a1, a2, work, own); break;
+    case 32: eval_chunk_c<RT, KIND, PREC, 32, S2, S, PM>(D, item, tag, s0, count, shift, srow, a1, a2, work, own); break;
+    case 16: eval_chunk_c<RT, KIND, PREC, 16, S2, S, PM>(D, item, tag, s0, count, shift, srow, a1, a2, work, own); break;
+    case 8: eval_chunk_c<RT, KIND, PREC, 8, S2, S, PM>(D, item, tag, s0, count, shift, srow, a1, a2, work, own); break;
+    default: eval_chunk_c<RT, KIND, PREC, 4, S2, S, PM>(D, item, tag, s0, count, shift, srow, a1, a2, work, own); break;
     }
 }
 
@@ -924,16 +927,16 @@ __device__ __forceinline__ void eval_chunk_s(const DevLevel<RT>& D, uint32_t ite
 // threshold that the adaptive rule compares with the spread), so the one-pass variance
 // s2 - s1^2 / n does not cancel where the decision is close; the final phase accumulates d.
 // `srow`: the outer sample's R_tau row in shared memory, or nullptr (FP32 portfolio path).
-// PIPE: the pipelined alias-column loop (the 128-register variant of the phase kernel).
+// PM: how the FP32 portfolio path draws its options (PfMode).
 // own: this thread's chunk is real (false for threads past the end of a segment's last tile,
 // which take part only in the warp-cooperative samples of the FP32 path-simulated kernel).
-template <class RT, int KIND, int PREC, class S, bool PIPE>
+template <class RT, int KIND, int PREC, class S, int PM>
 __device__ __forceinline__ void eval_chunk(const DevLevel<RT>& D, uint32_t item, uint32_t tag,
                                            uint64_t s0, uint64_t count, uint32_t C, bool want_s2, RT start,
                                            const float2* srow, Acc<PREC>& a1, Acc<PREC>& a2, double& work,
                                            bool own = true) {
-    if (want_s2) eval_chunk_s<RT, KIND, PREC, true, S, PIPE>(D, item, tag, s0, count, C, (float)start, srow, a1, a2, work, own);
-    else eval_chunk_s<RT, KIND, PREC, false, S, PIPE>(D, item, tag, s0, count, C, 0.f, srow, a1, a2, work, own);
+    if (want_s2) eval_chunk_s<RT, KIND, PREC, true, S, PM>(D, item, tag, s0, count, C, (float)start, srow, a1, a2, work, own);
+    else eval_chunk_s<RT, KIND, PREC, false, S, PM>(D, item, tag, s0, count, C, 0.f, srow, a1, a2, work, own);
 }
 
 // ---- segments of uniform chunk count ------------------------------------------------------
@@ -1154,7 +1157,7 @@ __device__ __forceinline__ void cta_sums(const OuterBuffers& B, double wsum, uin
 // 2: 128 with the pipelined alias-column loop, 3: 80, 4: 64) — the register/occupancy variants the
 // autotuner chooses between.  The variants run the same arithmetic in the same order, so their
 // results are identical.
-template <class RT, int KIND, int PREC, int MINB, class S = NoSampler>
+template <class RT, int KIND, int PREC, int MINB, class S = NoSampler, int PM = PF_GENERIC>
 __global__ void __launch_bounds__(kTile, MINB) k_phase(DevLevel<RT> D, SegSet SS, TraceRec* trace) {
     __shared__ Acc<PREC> sm_a1[kWarps];
     __shared__ Acc<PREC> sm_a2[kWarps];
@@ -1167,8 +1170,7 @@ __global__ void __launch_bounds__(kTile, MINB) k_phase(DevLevel<RT> D, SegSet SS
     // R_tau rows of the FP32 portfolio path can be staged (kRowItems rows of Q stocks)
     const uint32_t Qs = D.L.ot.Q;
     const float2* Rt2 = reinterpret_cast<const float2*>(D.B.Rt);
-    const bool can_stage = KIND == KIND_PORTFOLIO && PREC == PREC_FP32 && D.L.ot.fast_s != nullptr &&
-                           Qs <= kMaxStagedStocks;
+    const bool can_stage = KIND == KIND_PORTFOLIO && PREC == PREC_FP32 && PM != PF_GENERIC && Qs <= kMaxStagedStocks;
     const uint32_t C = D.L.chunk;
     uint32_t* counters = D.B.counters;
     double wsum = 0;                                     // work of this thread's chunks
@@ -1237,7 +1239,7 @@ __global__ void __launch_bounds__(kTile, MINB) k_phase(DevLevel<RT> D, SegSet SS
                 // the FP32 path-simulated kernel evaluates deep samples warp-wide: all lanes call
                 constexpr bool kCoopKind = KIND == KIND_PF_PATHS && PREC == PREC_FP32;
                 if (valid || (kCoopKind && C <= kPathSortChunk))
-                    eval_chunk<RT, KIND, PREC, S, MINB == 2>(D, item, g.tag, (uint64_t)j * C, g.count, C, pilot, start,
+                    eval_chunk<RT, KIND, PREC, S, PM>(D, item, g.tag, (uint64_t)j * C, g.count, C, pilot, start,
                                                              srow, a1, a2, wsum, valid);
                 const float coeff = (float)gs / (float)nch;     // 1 / groups (a power of two)
                 float ind = 0.f;
@@ -1329,7 +1331,7 @@ __global__ void __launch_bounds__(kTile, MINB) k_phase(DevLevel<RT> D, SegSet SS
                     Acc<PREC> a1, a2;
                     a1.zero();
                     a2.zero();
-                    eval_chunk<RT, KIND, PREC, S, MINB == 2>(D, item, g.tag, (uint64_t)j * C, g.count, C, pilot, start, srow, a1, a2, wsum);
+                    eval_chunk<RT, KIND, PREC, S, PM>(D, item, g.tag, (uint64_t)j * C, g.count, C, pilot, start, srow, a1, a2, wsum);
                     float ind = 0.f;
                     if (!pilot && gs == 1) ind = phi_of<KIND, S, RT>(inner_mean<RT, PREC>(start, a1, csmall), coeff);
                     for (uint32_t m = 1; m < 32; m <<= 1) {
@@ -1587,7 +1589,9 @@ struct SmallWarp {
             if (PREC == PREC_FP32 && ot.fast_s) {
                 if constexpr (sizeof(RT) == 4) {
                     const float2* r = reinterpret_cast<const float2*>(row);
-                    if (ot.fast_col) {
+                    if (ot.fast_col && columns_in_l1(ot)) {
+                        for (int q = 0; q < 2; q++) d[q] = pf_sample_loss<PF_COLUMN_L1>(v[q], ot, r);
+                    } else if (ot.fast_col) {
                         for (int q = 0; q < 2; q++) d[q] = pf_sample_loss<PF_COLUMN>(v[q], ot, r);
                     } else if (ot.subsample == SUB_UNIFORM) {
                         for (int q = 0; q < 2; q++) d[q] = pf_sample_loss<PF_UNIFORM_L1>(v[q], ot, r);
@@ -1783,7 +1787,7 @@ constexpr size_t phase_dyn_smem() {
     return PREC != PREC_FP32 ? 0 : KIND == KIND_PORTFOLIO ? kRowSmemBytes : KIND == KIND_PF_PATHS ? kPathSortSmemBytes : 0;
 }
 
-template <class RT, int KIND, int PREC, int MINB, class S = NoSampler>
+template <class RT, int KIND, int PREC, int MINB, class S, int PM>
 static int phase_grid(int cap) {
     static int g = 0;
     if (g == 0) {
@@ -1791,8 +1795,8 @@ static int phase_grid(int cap) {
         constexpr size_t dyn = phase_dyn_smem<KIND, PREC>();
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (dyn) cudaFuncSetAttribute(k_phase<RT, KIND, PREC, MINB, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_phase<RT, KIND, PREC, MINB, S>, kTile, dyn) != cudaSuccess ||
+        if (dyn) cudaFuncSetAttribute(k_phase<RT, KIND, PREC, MINB, S, PM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_phase<RT, KIND, PREC, MINB, S, PM>, kTile, dyn) != cudaSuccess ||
             per_sm < 1)
             per_sm = 1;
         g = per_sm * sms;
@@ -1800,30 +1804,58 @@ static int phase_grid(int cap) {
     return g < cap ? g : cap;
 }
 
-template <class RT, int KIND, int PREC, int MINB, class S = NoSampler>
+template <class RT, int KIND, int PREC, int MINB, class S = NoSampler, int PM = PF_GENERIC>
 static void launch_phase_v(const DevLevel<RT>& D, const SegSet& SS, TraceRec* trace, cudaStream_t stream) {
     if (D.B.prof_mark) D.B.prof_mark(D.B.prof_user, 0, stream);
-    const int grid = phase_grid<RT, KIND, PREC, MINB, S>(D.B.slots);
-    k_phase<RT, KIND, PREC, MINB, S><<<grid, kTile, phase_dyn_smem<KIND, PREC>(), stream>>>(D, SS, trace);
+    const int grid = phase_grid<RT, KIND, PREC, MINB, S, PM>(D.B.slots);
+    // staged rows of the portfolio's own length: what they leave is L1 for the option table
+    size_t dyn = phase_dyn_smem<KIND, PREC>();
+    if (KIND == KIND_PORTFOLIO && PREC == PREC_FP32)
+        dyn = PM == PF_GENERIC || D.L.ot.Q > kMaxStagedStocks ? 0 : (size_t)kRowItems * D.L.ot.Q * sizeof(float2);
+    k_phase<RT, KIND, PREC, MINB, S, PM><<<grid, kTile, dyn, stream>>>(D, SS, trace);
     if (D.B.prof_mark) D.B.prof_mark(D.B.prof_user, 1, stream);
     count_launch();
 }
 
-// The FP32 path has three register/occupancy variants (OuterLevel::variant 0, 1, 2 -> 1, 3, 4
-// resident CTAs per SM guaranteed), and the portfolio a fourth (3 -> 2 CTAs per SM, 128 registers,
-// the pipelined alias-column loop; other kinds run variant 0 for it); the parity precisions run
-// variant 0, the FP32 kernel of path-simulated portfolios two CTAs per SM (128 registers: the
-// class-ordered loop spills at 80, and runs 7 % faster at two CTAs without spills than at three
-// with them; the FP64 path states and exponentials leave one CTA per SM at the compiler's choice).
+// Register/occupancy variants of the FP32 path (OuterLevel::variant): 0, 1, 2 -> 1, 3, 4 resident
+// CTAs per SM guaranteed (up to 255, 80, 64 registers), and 3 for the alias columns: the pipelined loop
+// at two CTAs (128 registers); elsewhere 3 runs as 1.
+template <class RT, int KIND, int PREC, class S, int PM>
+static void launch_variant(const DevLevel<RT>& D, const SegSet& SS, TraceRec* trace, cudaStream_t stream) {
+    if constexpr (is_column(PM))
+        if (D.L.variant == 3) return launch_phase_v<RT, KIND, PREC, 2, S, PF_COLUMN_PIPE>(D, SS, trace, stream);
+    if (D.L.variant == 0) return launch_phase_v<RT, KIND, PREC, 1, S, PM>(D, SS, trace, stream);
+    if (D.L.variant == 2) return launch_phase_v<RT, KIND, PREC, 4, S, PM>(D, SS, trace, stream);
+    launch_phase_v<RT, KIND, PREC, 3, S, PM>(D, SS, trace, stream);
+}
+
+// Portfolios in the parity precisions, and the FP32 kernel of path-simulated ones, run at two CTAs
+// per SM (128 registers): the path kernel's class-ordered loop spills at 80 and runs 7 % faster at two
+// CTAs without spills than at three with them; FP64 portfolio level 3, 20,000 outer samples: 783 us
+// at one, 632 at two.  The models in the parity precisions do so where the first pilots have a wave
+// of tiles for it (FP64 level 3: 2e6 outer samples 2.67 ms at one CTA, 1.90 at two; 20,000: 110 and 119
+// us).
 template <class RT, int KIND, int PREC, class S = NoSampler>
 static void launch_phase(const DevLevel<RT>& D, const SegSet& SS, TraceRec* trace, cudaStream_t stream) {
-    if constexpr (PREC == PREC_FP32 && KIND != KIND_USER && KIND != KIND_PF_PATHS) {
-        if (D.L.variant == 1) return launch_phase_v<RT, KIND, PREC, 3>(D, SS, trace, stream);
-        if (D.L.variant == 2) return launch_phase_v<RT, KIND, PREC, 4>(D, SS, trace, stream);
-        if constexpr (KIND == KIND_PORTFOLIO)
-            if (D.L.variant == 3) return launch_phase_v<RT, KIND, PREC, 2>(D, SS, trace, stream);
+    if constexpr (KIND == KIND_PORTFOLIO && PREC == PREC_FP32) {
+        const OptionTable<RT>& ot = D.L.ot;
+        if (!ot.fast_s) return launch_phase_v<RT, KIND, PREC, 2, S>(D, SS, trace, stream);
+        if (ot.fast_col) {
+            if (columns_in_l1(ot)) return launch_variant<RT, KIND, PREC, S, PF_COLUMN_L1>(D, SS, trace, stream);
+            return launch_variant<RT, KIND, PREC, S, PF_COLUMN>(D, SS, trace, stream);
+        }
+        if (ot.subsample != SUB_UNIFORM) return launch_variant<RT, KIND, PREC, S, PF_ALIAS>(D, SS, trace, stream);
+        if ((uint64_t)ot.P * sizeof(FastOption) <= kL1TableBytes) return launch_variant<RT, KIND, PREC, S, PF_UNIFORM_L1>(D, SS, trace, stream);
+        return launch_variant<RT, KIND, PREC, S, PF_UNIFORM>(D, SS, trace, stream);
+    } else if constexpr (PREC == PREC_FP32 && !is_portfolio_kind(KIND) && KIND != KIND_USER) {
+        launch_variant<RT, KIND, PREC, S, PF_GENERIC>(D, SS, trace, stream);
+    } else if constexpr (is_portfolio_kind(KIND)) {
+        launch_phase_v<RT, KIND, PREC, 2, S>(D, SS, trace, stream);
+    } else {
+        if constexpr (KIND != KIND_USER)
+            if (D.L.M >= 32768) return launch_phase_v<RT, KIND, PREC, 2, S>(D, SS, trace, stream);
+        launch_phase_v<RT, KIND, PREC, 1, S>(D, SS, trace, stream);
     }
-    launch_phase_v<RT, KIND, PREC, (KIND == KIND_PF_PATHS && PREC == PREC_FP32) ? 2 : 1, S>(D, SS, trace, stream);
 }
 
 static inline uint32_t ilog2_u64(uint64_t v) {
