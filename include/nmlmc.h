@@ -176,7 +176,9 @@ typedef struct nmlmc_level_result {
     uint64_t M;
     uint64_t inner_stats[6];   /* inner samples, decisions, hit max, hit base, #randu, #randn */
     double seconds;            /* device time of the level: CUDA events around a single call;
-                                  inside a round's graph, %globaltimer stamps at its boundaries */
+                                  inside a round's graph, %globaltimer stamps at its begin and end
+                                  (levels that ran side by side: the round's time in proportion
+                                  to their inner samples) */
 } nmlmc_level_result;
 
 typedef struct nmlmc_portfolio {
@@ -295,8 +297,9 @@ int nmlmc_reset_streams(nmlmc_ctx* ctx);
 int nmlmc_sample(nmlmc_ctx* ctx, uint32_t ell, uint64_t M, nmlmc_level_result* out);
 /* Several levels in one submission.  OUTER layout: the levels' launch sequences are captured
  * into one CUDA graph (kept and updated in place while the topology repeats), each level summing
- * into its own slot, one device->host copy and one synchronisation for the round; levels run one
- * after another inside the graph.  Up to 64 levels; with tracing or phase profiling armed, or on
+ * into its own slot of pinned host memory, one synchronisation for the round; levels run side by
+ * side where their outer samples fit the batch buffers together, one after another otherwise.  Up to
+ * 64 levels; with tracing or phase profiling armed, or on
  * the CORE layout, the levels run as consecutive nmlmc_sample calls. */
 int nmlmc_sample_levels(nmlmc_ctx* ctx, uint32_t n, const uint32_t* ells, const uint64_t* Ms,
                         nmlmc_level_result* outs);

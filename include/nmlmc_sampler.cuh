@@ -158,7 +158,7 @@ public:
             release();
             return NMLMC_ERR_NOMEM;
         }
-        if (cudaMemset(B_.counters, 0, 256 * 4) != cudaSuccess) return NMLMC_ERR_CUDA;
+        if (cudaMemsetAsync(B_.counters, 0, 256 * 4, stream_) != cudaSuccess) return NMLMC_ERR_CUDA;
         memset(next_, 0, sizeof next_);
         ready_ = true;
         return NMLMC_OK;

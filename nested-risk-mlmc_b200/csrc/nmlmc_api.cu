@@ -88,8 +88,7 @@ RT h_norm_cdf_inv(RT p) {
            (((((b[0] * r + b[1]) * r + b[2]) * r + b[3]) * r + b[4]) * r + 1);
 }
 
-// Levels of a round that run side by side (their own counters and partial sums in the batch
-// buffers, a side stream each).
+// Levels of a round that run side by side (counters, partial sums and a side stream each).
 constexpr uint32_t kSideLevels = 16;
 constexpr uint32_t kCounterSlots = 256;      // counters of one level
 
@@ -188,7 +187,9 @@ struct nmlmc_ctx {
     double* h_pin = nullptr;          // 32 doubles
     // one-submission level rounds (nmlmc_sample_levels on the OUTER layout)
     double* h_lev = nullptr;          // pinned [kMaxSubmit][16] sums, then [kMaxSubmit][2] stamps
-    cudaStream_t side[kSideLevels] = {};   // capture streams of levels that run side by side
+    uint32_t* side_counters = nullptr;     // counters and partial sums of levels 1, 2, ... that run
+    double* side_sums = nullptr;           // beside level 0 of a round
+    cudaStream_t side[kSideLevels] = {};   // their capture streams
     cudaEvent_t side_ev[kSideLevels] = {}; // [0] the fork, [i] the end of level i
     std::vector<GraphSlot> graphs;    // executable graphs of recent submissions, by topology
     uint64_t graph_clock = 0;
@@ -477,6 +478,7 @@ int build_dev_portfolio(nmlmc_ctx* c, DevPortfolio<RT>& d) {
             dev_malloc(&d.lvl_w, kPathLevels * sizeof(RT)) != cudaSuccess ||
             dev_malloc(&d.lvl_wf, kPathLevels * sizeof(float)) != cudaSuccess)
             return set_err(NMLMC_ERR_NOMEM);
+        NM_CUDA(cudaStreamSynchronize(nullptr), "uploads");      // the tables it reads: c->stream does not wait for them
         NM_CUDA(launch_ref_records(t, d.ref, d.lvl_w, d.lvl_wf, c->stream), "option constants");
     }
     t.ref = d.ref;
@@ -532,6 +534,7 @@ int build_dev_portfolio(nmlmc_ctx* c, DevPortfolio<RT>& d) {
             }
         }
     }
+    NM_CUDA(cudaStreamSynchronize(nullptr), "uploads");          // before c->stream reads the tables
     return NMLMC_OK;
 }
 
@@ -588,7 +591,7 @@ int alloc_core(nmlmc_ctx* c) {
         dfree(c->d_states); dfree(c->d_states_next); dfree(c->d_core_part); dfree(c->d_core_counts);
         return set_err(NMLMC_ERR_NOMEM);
     }
-    NM_CUDA(cudaMemset(c->d_core_counts, 0, nc), "memset");
+    NM_CUDA(cudaMemsetAsync(c->d_core_counts, 0, nc, c->stream), "memset");
     c->states_cores = cores;
     return NMLMC_OK;
 }
@@ -648,15 +651,16 @@ int alloc_outer(nmlmc_ctx* c, uint64_t want) {
               dev_malloc(&B.cnt_c, cap * sizeof(uint32_t)) == cudaSuccess &&
               dev_malloc(&B.lists, 4 * cap * sizeof(uint32_t)) == cudaSuccess &&
               dev_malloc(&B.class_items, cap * sizeof(uint32_t)) == cudaSuccess &&
-              dev_malloc(&B.counters, kSideLevels * kCounterSlots * sizeof(uint32_t)) == cudaSuccess &&
-              dev_malloc(&B.block_sums, (size_t)kSideLevels * B.grid * 16 * sizeof(double)) == cudaSuccess &&
+              dev_malloc(&B.counters, kCounterSlots * sizeof(uint32_t)) == cudaSuccess &&
+              dev_malloc(&B.block_sums, (size_t)B.grid * 16 * sizeof(double)) == cudaSuccess &&
               dev_malloc(&B.level_acc, kMaxSubmit * 16 * sizeof(double)) == cudaSuccess;
     c->ob_alloc = true;                   // free_outer releases a partial set too
     if (!ok) {
         free_outer(c);
         return set_err(NMLMC_ERR_NOMEM);
     }
-    cudaMemset(B.counters, 0, kSideLevels * kCounterSlots * sizeof(uint32_t));
+    // on the context's stream, which does not wait for the default stream
+    NM_CUDA(cudaMemsetAsync(B.counters, 0, kCounterSlots * sizeof(uint32_t), c->stream), "memset");
     return NMLMC_OK;
 }
 
@@ -972,7 +976,8 @@ void shard_range(const nmlmc_ctx* c, uint64_t Mtotal, uint64_t& lo, uint64_t& M)
 
 // The batch buffers of a round's level `i` that runs beside the others: outer samples [off, off + M)
 // of every per-sample array, counters and partial sums of its own.
-OuterBuffers side_buffers(const OuterBuffers& ob, uint32_t i, uint64_t off, uint64_t M) {
+OuterBuffers side_buffers(const nmlmc_ctx* c, uint32_t i, uint64_t off, uint64_t M) {
+    const OuterBuffers& ob = c->ob;
     OuterBuffers B = ob;
     B.cap = M;
     B.Yv = static_cast<double*>(ob.Yv) + off;
@@ -981,12 +986,23 @@ OuterBuffers side_buffers(const OuterBuffers& ob, uint32_t i, uint64_t off, uint
     B.cnt_c += off;
     B.lists += 4 * off;
     B.class_items += off;
-    B.counters += (size_t)i * kCounterSlots;
-    B.block_sums += (size_t)i * ob.grid * 16;
+    if (i) {
+        B.counters = c->side_counters + (size_t)(i - 1) * kCounterSlots;
+        B.block_sums = c->side_sums + (size_t)(i - 1) * ob.grid * 16;
+    }
     return B;
 }
 
-int ensure_side_streams(nmlmc_ctx* c, uint32_t n) {
+int ensure_side(nmlmc_ctx* c, uint32_t n) {
+    if (!c->side_sums) {
+        const size_t nc = (kSideLevels - 1) * kCounterSlots * sizeof(uint32_t);
+        if (!c->side_counters && dev_malloc(&c->side_counters, nc) != cudaSuccess) return set_err(NMLMC_ERR_NOMEM);
+        NM_CUDA(cudaMemsetAsync(c->side_counters, 0, nc, c->stream), "memset");
+        if (dev_malloc(&c->side_sums, (size_t)(kSideLevels - 1) * c->ob.grid * 16 * sizeof(double)) != cudaSuccess) {
+            c->side_sums = nullptr;
+            return set_err(NMLMC_ERR_NOMEM);
+        }
+    }
     for (uint32_t i = 0; i < n; i++) {
         if (!c->side[i]) NM_CUDA(cudaStreamCreateWithFlags(&c->side[i], cudaStreamNonBlocking), "side stream");
         if (!c->side_ev[i]) NM_CUDA(cudaEventCreateWithFlags(&c->side_ev[i], cudaEventDisableTiming), "side event");
@@ -1038,7 +1054,7 @@ int sample_outer_levels(nmlmc_ctx* c, uint32_t n, const uint32_t* ells, const ui
     const bool side = n > 1 && n <= kSideLevels && total <= ob.cap;
     key.push_back(side);
     if (side) {
-        const int rc = ensure_side_streams(c, n);
+        const int rc = ensure_side(c, n);
         if (rc) return rc;
     }
     // the executable graph of a recent round with the same levels is reused if it runs no level as
@@ -1059,7 +1075,7 @@ int sample_outer_levels(nmlmc_ctx* c, uint32_t n, const uint32_t* ells, const ui
         const uint64_t M = Ms[i];
         OuterLevel<RT>& L = levels[i];
         L.no_small = !(small >> i & 1);
-        OuterBuffers B = side ? side_buffers(ob, i, off, M) : ob;
+        OuterBuffers B = side ? side_buffers(c, i, off, M) : ob;
         off += M;
         const cudaStream_t st = side && i ? c->side[i] : c->stream;
         if (st != c->stream) err = cudaStreamWaitEvent(st, c->side_ev[0], 0);
@@ -1192,6 +1208,7 @@ int nmlmc_destroy(nmlmc_ctx* c) {
     free_outer(c);
     for (cudaEvent_t e : c->pev) cudaEventDestroy(e);
     drop_graphs(c);
+    dfree(c->side_counters); dfree(c->side_sums);
     for (cudaStream_t st : c->side)
         if (st) cudaStreamDestroy(st);
     for (cudaEvent_t e : c->side_ev)
@@ -1246,7 +1263,7 @@ int nmlmc_reset_streams(nmlmc_ctx* c) {
         int rc = alloc_core(c);
         if (rc) return rc;
         // init_samplers: both random_state(seed, core) from counter {0,0}, no cached normal
-        NM_CUDA(cudaMemset(c->d_states, 0, (size_t)c->cfg.cores * 2 * sizeof(CoreStream)), "reset streams");
+        NM_CUDA(cudaMemsetAsync(c->d_states, 0, (size_t)c->cfg.cores * 2 * sizeof(CoreStream), c->stream), "reset streams");
     }
     return NMLMC_OK;
 }
@@ -1633,8 +1650,9 @@ int nmlmc_get_sampler_state(nmlmc_ctx* c, void* buf, size_t cap, size_t* size) {
         int rc = alloc_core(c);
         if (rc) return rc;
         NM_CUDA(cudaStreamSynchronize(c->stream), "sync");
-        NM_CUDA(cudaMemcpy(static_cast<char*>(buf) + sizeof h, c->d_states, core_bytes, cudaMemcpyDeviceToHost),
+        NM_CUDA(cudaMemcpyAsync(static_cast<char*>(buf) + sizeof h, c->d_states, core_bytes, cudaMemcpyDeviceToHost, c->stream),
                 "sampler state d2h");
+        NM_CUDA(cudaStreamSynchronize(c->stream), "sampler state d2h");
     }
     return NMLMC_OK;
 }
@@ -1659,8 +1677,9 @@ int nmlmc_set_sampler_state(nmlmc_ctx* c, const void* buf, size_t size) {
         int rc = alloc_core(c);
         if (rc) return rc;
         NM_CUDA(cudaStreamSynchronize(c->stream), "sync");
-        NM_CUDA(cudaMemcpy(c->d_states, static_cast<const char*>(buf) + sizeof h, core_bytes, cudaMemcpyHostToDevice),
+        NM_CUDA(cudaMemcpyAsync(c->d_states, static_cast<const char*>(buf) + sizeof h, core_bytes, cudaMemcpyHostToDevice, c->stream),
                 "sampler state h2d");
+        NM_CUDA(cudaStreamSynchronize(c->stream), "sampler state h2d");
     }
     return NMLMC_OK;
 }
