@@ -98,15 +98,17 @@ struct OuterBuffers {
 // work, in units of one FP32 normal with 96 per phase for the sums and the decision (a phase of 32
 // samples keeps 8 of 32 lanes busy), stays below what the launch sequence costs whatever its size —
 // about 50 us for one phase, 105 to 200 us with pilots.  Measured on both sides of the lines (one
-// kernel, sequence): model level 0, 6200 samples 47.8 and 46.4 us; level 5, 12,500: 102 and 121 us;
-// reference model level 3, 2600: 76 and 117 us; FP64 level 3, 6200: 90 and 89 us; importance
-// portfolio level 3, 10,400: 143 and 224 us.  Larger counts than 4096 (one phase: 2048) leave a
-// single warp too long alone: model level 8, 12,000: 212 and 184 us.
+// kernel, sequence; the models' level 0 has since become k_fixed): model level 0, 6200 samples 47.8
+// and 46.4 us; level 5, 12,500: 102 and 121 us; reference model level 3, 2600: 76 and 117 us; FP64
+// level 3, 6200: 90 and 89 us; importance portfolio level 3, 10,400: 143 and 224 us.  Larger counts
+// than 4096 (one phase: 2048) leave a single warp too long alone: model level 8, 12,000: 212 and
+// 184 us.  An N0 that is no power of two stays with the sequence, whose tiles hold a power of two of
+// chunks per outer sample.
 constexpr uint32_t kSmallMaxChunk = 32, kSmallMaxStocks = 256;
 template <class RT>
 bool level_is_small(const OuterLevel<RT>& L, int kind, int prec, const OuterBuffers& B) {
     if (kind == KIND_USER || (is_portfolio_kind(kind) && (L.ot.mixed || L.ot.Q > kSmallMaxStocks))) return false;
-    if (B.prof_mark || L.chunk < 4 || L.chunk > kSmallMaxChunk || L.M > B.cap) return false;
+    if (B.prof_mark || L.chunk < 4 || L.chunk > kSmallMaxChunk || L.M > B.cap || (L.N0 & (L.N0 - 1))) return false;
     const uint64_t maxc = (L.fine_only || L.cf.max_count >= L.cc.max_count) ? L.cf.max_count : L.cc.max_count;
     const bool pilots = L.adaptive_f || L.adaptive_c;
     if (maxc > (pilots ? 4096u : 2048u)) return false;

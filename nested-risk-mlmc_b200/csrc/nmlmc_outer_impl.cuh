@@ -2077,7 +2077,7 @@ cudaError_t sample_level_t(const OuterLevel<RT>& L, OuterBuffers& B, TraceRec* t
     }
     if constexpr (KIND == KIND_REF_MODEL || KIND == KIND_SHIFT_MODEL) {
         const uint64_t maxc = (L.fine_only || L.cf.max_count >= L.cc.max_count) ? L.cf.max_count : L.cc.max_count;
-        if (!L.adaptive_f && !L.adaptive_c && maxc / L.chunk <= kFixedChunks) {
+        if (!L.adaptive_f && !L.adaptive_c && maxc / L.chunk <= kFixedChunks && !(L.N0 & (L.N0 - 1))) {
             const uint64_t ctas = (L.M + kTile - 1) / kTile;
             const int grid = fixed_grid<RT, KIND, PREC>((int)(ctas < (uint64_t)B.grid ? ctas : (uint64_t)B.grid));
             if (B.prof_mark) B.prof_mark(B.prof_user, 0, stream);

@@ -56,3 +56,17 @@ def test_small_calls_draw_the_same_samples(nm, case):
             np.testing.assert_allclose(got["diffsums"][k], (d ** (k + 1)).sum() if ell else 0, rtol=tol, atol=tol)
         assert got["stats"][1] == m and got["stats"][0] == got["work"]
         at += m
+
+
+# tiles of the launch sequence hold a power of two of chunks: an N0 of three chunks keeps to it
+@pytest.mark.parametrize("prec,r,ell,M,pieces", [("FP32", 1.5, 0, 5_000, (200, 33)), ("FP32", 1.5, 3, 40_000, (300, 7)),
+                                                 ("FP64", 0.0, 2, 20_000, (50,))])
+def test_counts_of_three_chunks_take_the_sequence(nm, prec, r, ell, M, pieces):
+    big = _sampler(nm, "shift", prec, 96, 2, r).sample(ell, M, trace=True)["trace"]
+    s, at = _sampler(nm, "shift", prec, 96, 2, r), 0
+    for m in pieces:
+        n0 = nm.kernel_launches()
+        got = s.sample(ell, m, trace=True)["trace"]
+        assert nm.kernel_launches() - n0 > 1
+        assert got.tobytes() == big[at:at + m].tobytes()
+        at += m
