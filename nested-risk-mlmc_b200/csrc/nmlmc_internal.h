@@ -81,6 +81,7 @@ struct OuterBuffers {
     double* block_sums;      // per-CTA partial moments [grid][16]
     double* level_acc;       // the level's result [16] (device or pinned host memory), written by its last
                              // kernel: the sums of block_sums, entry 12 the path-limit flag
+                             // (path-simulated portfolios, 0 otherwise)
     int grid;                // CTA slots of block_sums
     int slots;               // slots the current level uses (set per level)
     uint64_t* stamps;        // optional: %globaltimer at the level's begin and end [2] (as level_acc)
@@ -119,7 +120,7 @@ bool level_is_small(const OuterLevel<RT>& L, int kind, int prec, const OuterBuff
 
 // Device counter slot (OuterBuffers::counters) that the batched kernels set when a
 // path-simulated inner sample would exceed kMaxPathSteps (the call then fails with
-// NMLMC_ERR_LIMIT); the host clears it.
+// NMLMC_ERR_LIMIT); k_outer clears it on a level's first batch.
 constexpr uint32_t kCounterPathLimit = 240;
 
 // Records a failed status for nmlmc_last_error() (this thread) and returns it.

@@ -1088,9 +1088,10 @@ __device__ __forceinline__ void level_stamp(uint64_t* stamps, int slot) {
 // End of a level's last kernel, called by all T threads of every CTA after its partial sums are
 // written: the CTA that arrives last adds the partials of all `slots` CTAs to the level's 16 sums
 // (thread t sum t % 16 of slots t / 16, t / 16 + T / 16, ..., then the groups in order: a fixed
-// order) and stores them, with the path-limit flag in entry 12, where the caller reads them — in
-// the host's pinned memory, so a call needs neither a reduction kernel (7 us) nor a copy back.
-template <int T>
+// order) and stores them where the caller reads them — in the host's pinned memory, so a call needs
+// neither a reduction kernel (7 us) nor a copy back.  LIMIT: entry 12 is the path-limit flag, which
+// the path-simulated kind's k_outer has cleared; no other kind clears or sets it, and its entry is 0.
+template <int T, bool LIMIT = false>
 __device__ __forceinline__ void level_finish(const OuterBuffers& B, int slots) {
     __shared__ double red[T / 16][17];
     __shared__ uint32_t arrived;
@@ -1108,7 +1109,7 @@ __device__ __forceinline__ void level_finish(const OuterBuffers& B, int slots) {
     if (t < 16) {
         double s = 0;
         for (int k = 0; k < T / 16; k++) s += red[k][t];
-        if (t == 12) s = (double)__ldcg(B.counters + CNT_ERR);
+        if (t == 12) s = LIMIT ? (double)__ldcg(B.counters + CNT_ERR) : 0.0;
         B.level_acc[t] = s;
     }
     if (t == 0) {
@@ -1391,7 +1392,7 @@ __global__ void __launch_bounds__(kTile, MINB) k_phase(DevLevel<RT> D, SegSet SS
         }
     }
     cta_sums(D.B, wsum, n_max, n_base, mom, sm_acc, true);
-    if (SS.reduce) level_finish<kTile>(D.B, D.B.slots);
+    if (SS.reduce) level_finish<kTile, KIND == KIND_PF_PATHS>(D.B, D.B.slots);
 }
 
 // ---- outer draws ---------------------------------------------------------------------------
@@ -1425,7 +1426,7 @@ __global__ void __launch_bounds__(kTile) k_outer(DevLevel<RT> D, uint32_t nb, in
     if (first) {
         for (uint32_t k = gid; k < (uint32_t)D.B.slots * 16; k += gsz) D.B.block_sums[k] = 0;
         if (gid == 0) {
-            D.B.counters[CNT_ERR] = 0;
+            D.B.counters[CNT_ERR] = 0;           // once per level: its end reports every batch
             level_stamp(D.B.stamps, 0);
         }
     }

@@ -131,3 +131,44 @@ def test_outer_paths_beyond_the_step_limit_fail(nm, prec_name):
     with pytest.raises(nm.NmlmcError) as err:
         s.sample(1, 64)
     assert err.value.status == nm.ERR_LIMIT
+
+
+@pytest.mark.parametrize("prec_name", ["fp32", "ref32", "fp64"])
+def test_a_step_limit_failure_is_not_seen_by_later_calls(nm, prec_name):
+    """After ERR_LIMIT the same context samples other problems as a fresh one does, by every route
+    of a level: one kernel (few outer samples, fixed counts) and the launch sequence."""
+    import nmlmc
+    case = CASES[0]
+    pf = O.synthetic_portfolio(**case["pf"])
+    prec = dict(fp32=nm.PREC_FP32, ref32=nm.PREC_REF32, fp64=nm.PREC_FP64)[prec_name]
+
+    def sampler():
+        s = nmlmc.Sampler(N0=32, beta=2, adaptive_r=1.5, precision=prec, streams=nmlmc.STREAMS_OUTER, seed=4)
+        s.set_autotune(0)
+        return s
+
+    def fail(s):
+        s.set_portfolio(pf, max_loss=0.3, subsample=nm.SUB_RANDOM,
+                        methods=dict(method=[2] * len(pf["w"]), dt_h0inv=(1 << 24) + 1))
+        with pytest.raises(nm.NmlmcError) as err:
+            s.sample(1, 64)
+        assert err.value.status == nm.ERR_LIMIT
+        s.reset_streams()
+
+    def model(s):
+        s.set_model(nm.MODEL_SHIFT, 0.0, 1.0)
+
+    def portfolio(s):
+        s.set_portfolio(pf, max_loss=0.3, subsample=nm.SUB_RANDOM)
+
+    # few outer samples, a fixed count at more of them, pilots (the sequence)
+    for problem, ell, M in ((model, 0, 100), (model, 0, 40_000), (model, 3, 100), (model, 3, 40_000),
+                            (portfolio, 2, 50), (portfolio, 2, 40_000)):
+        s, ref = sampler(), sampler()
+        fail(s)
+        problem(s)
+        problem(ref)
+        got, want = s.sample(ell, M), ref.sample(ell, M)
+        np.testing.assert_array_equal(got["fsums"], want["fsums"])
+        np.testing.assert_array_equal(got["diffsums"], want["diffsums"])
+        assert got["work"] == want["work"]
