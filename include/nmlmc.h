@@ -157,7 +157,8 @@ typedef struct nmlmc_ctx nmlmc_ctx;
 
 typedef struct nmlmc_config {
     uint32_t cores;            /* virtual cores of the CORE layout (0 -> 2048)                  */
-    uint32_t N0;               /* inner samples at level 0                                      */
+    uint32_t N0;               /* inner samples at level 0 (OUTER layout: a power of two from 4,
+                                  or a multiple of 32)                                          */
     uint32_t beta;             /* inner refinement factor (power of two)                         */
     double adaptive_r;         /* adaptive exponent r; adaptive iff 1 < r < 2 (or <= 2, below)   */
     int32_t antithetic;        /* antithetic coarse estimator                                   */
@@ -310,7 +311,8 @@ int nmlmc_sample_levels(nmlmc_ctx* ctx, uint32_t n, const uint32_t* ells, const 
  * CTAs per SM, with the next inner samples' table gathers issued before the current ones are
  * evaluated; other kinds run variant 0 for it) and a chunk length (inner
  * samples per thread; power of two in [4, 64] dividing N0; a level's items of n inner samples
- * take n / chunk threads, so it also sets the outer samples per warp).  With autotuning on, the
+ * take n / chunk threads, so it also sets the outer samples per warp; an N0 that is no power of two
+ * runs one variant, with chunks of about that length times its odd factor).  With autotuning on, the
  * first nmlmc_sample / nmlmc_sample_levels call of a level with enough work times the
  * candidates on a probe of the level's own parameters whose outer stream indices start at 2^55
  * (no result changes) and keeps the fastest for that level in the context.  Mode 1 (the

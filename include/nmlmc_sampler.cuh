@@ -129,7 +129,7 @@ public:
     ~batched_sampler() { release(); }
 
     // N0, beta, adaptive_r, antithetic as nested_sampler_params (nested_sampler.hpp:14-34; the
-    // batched path needs the antithetic estimator and N0 a power-of-two multiple of its chunk),
+    // batched path needs the antithetic estimator and N0 a power of two from 4 or a multiple of 32),
     // adaptive_incl_r2 admits r = 2; seed: the streams' key; workspace_bytes:
     // SAMPLER::GetWorkspaceSize(data).  Returns an NMLMC_* status.
     int init(uint32_t N0, uint32_t beta, double adaptive_r, bool antithetic, bool adaptive_incl_r2,
@@ -139,7 +139,7 @@ public:
         if (N0 == 0 || beta < 2 || (beta & (beta - 1)) || !antithetic || chunk < 4 || (chunk & (chunk - 1)) ||
             N0 % chunk || batch == 0 || batch > (1ull << 31))
             return NMLMC_ERR_ARG;
-        N0_ = N0; beta_ = beta; r_ = adaptive_r; incl_r2_ = adaptive_incl_r2; seed_ = seed; chunk_ = chunk;
+        N0_ = N0; beta_ = beta; r_ = adaptive_r; incl_r2_ = adaptive_incl_r2; seed_ = seed; chunk_ = phase_chunk(N0, chunk);
         stream_ = stream;
         int dev = 0, sms = 148;
         if (cudaGetDevice(&dev) != cudaSuccess) return NMLMC_ERR_CUDA;

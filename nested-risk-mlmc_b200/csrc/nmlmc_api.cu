@@ -810,7 +810,7 @@ OuterLevel<RT> outer_level_params(const nmlmc_ctx* c, uint32_t ell, uint64_t M, 
     L.antithetic = c->cfg.antithetic != 0;
     L.N0 = c->cfg.N0;
     const PhaseChoice pc = phase_choice(c, ell);
-    L.chunk = pc.chunk;
+    L.chunk = phase_chunk(L.N0, pc.chunk);
     L.variant = pc.variant;
     L.adaptive_r = (RT)c->cfg.adaptive_r;
     L.cf = count_params(c->cfg, ell);
@@ -845,7 +845,7 @@ constexpr double kProbeMs = 20.0;       // device time of one tuning probe
 template <class RT>
 cudaError_t time_phase_config(nmlmc_ctx* c, uint32_t ell, uint64_t Mp, const PhaseChoice& pc, double& ms_out) {
     OuterLevel<RT> L = outer_level_params<RT>(c, ell, Mp, kProbeIndex);
-    L.chunk = pc.chunk;
+    L.chunk = phase_chunk(L.N0, pc.chunk);
     L.variant = pc.variant;
     OuterBuffers B = c->ob;
     B.prof_mark = nullptr;
@@ -1234,8 +1234,8 @@ int nmlmc_configure(nmlmc_ctx* c, const nmlmc_config* cfg) {
     if (k.streams != NMLMC_STREAMS_CORE && k.streams != NMLMC_STREAMS_OUTER) return set_err(NMLMC_ERR_ARG);
     if (k.streams == NMLMC_STREAMS_CORE && k.precision == NMLMC_PREC_FP32) return set_err(NMLMC_ERR_ARG);
     if (k.streams == NMLMC_STREAMS_OUTER) {
-        // chunks of min(N0, 32) samples must tile every count N0 * 2^k; the breadth-first path
-        // implements the antithetic estimator
+        // min(N0, 32) samples, a power of two from 4, must divide N0 (phase_chunk); the breadth-first
+        // path implements the antithetic estimator
         const uint32_t ch = k.N0 >= 32 ? 32 : k.N0;
         if ((k.N0 % ch) != 0 || (ch & (ch - 1)) != 0 || ch < 4 || !k.antithetic) return set_err(NMLMC_ERR_ARG);
         if (k.batch > (1ull << 31)) return set_err(NMLMC_ERR_ARG);

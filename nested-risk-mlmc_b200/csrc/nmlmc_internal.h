@@ -57,7 +57,7 @@ struct OuterLevel {
     uint64_t first_index;   // stream index of the first outer sample (OUTER layout key)
     uint64_t seed;
     bool fine_only, antithetic, adaptive_f, adaptive_c;
-    uint32_t N0, chunk;     // chunk = inner samples per thread (power of two dividing all counts)
+    uint32_t N0, chunk;     // chunk = inner samples per thread (phase_chunk: a power of two of them in each count)
     uint32_t variant;       // phase-kernel register/occupancy variant (FP32 path: 0, 1, 2)
     bool no_small;          // run the launch sequence whatever the size (level_is_small)
     RT adaptive_r;
@@ -95,6 +95,18 @@ struct OuterBuffers {
     void* prof_user;
 };
 
+// Inner samples per thread of the batched phases for a chosen chunk length (a power of two from 4
+// dividing N0).  A tile of threads holds a power of two of chunks per outer sample, so the odd factor
+// of an N0 that is no power of two goes into the chunk, about as long as the chosen one: N0 = 96 takes
+// 4 chunks of 24 for 32.
+inline uint32_t phase_chunk(uint32_t N0, uint32_t chunk) {
+    uint32_t odd = N0;
+    while (odd && !(odd & 1)) odd >>= 1;
+    if (odd <= 1) return chunk;
+    for (uint32_t f = 1; f < odd && chunk > 4; f <<= 1) chunk >>= 1;
+    return chunk * odd;
+}
+
 // Whether a level call runs as one kernel, a warp per outer sample (k_small): while its warps'
 // work, in units of one FP32 normal with 96 per phase for the sums and the decision (a phase of 32
 // samples keeps 8 of 32 lanes busy), stays below what the launch sequence costs whatever its size —
@@ -103,8 +115,7 @@ struct OuterBuffers {
 // and 46.4 us; level 5, 12,500: 102 and 121 us; reference model level 3, 2600: 76 and 117 us; FP64
 // level 3, 6200: 90 and 89 us; importance portfolio level 3, 10,400: 143 and 224 us.  Larger counts
 // than 4096 (one phase: 2048) leave a single warp too long alone: model level 8, 12,000: 212 and
-// 184 us.  An N0 that is no power of two stays with the sequence, whose tiles hold a power of two of
-// chunks per outer sample.
+// 184 us.  An N0 that is no power of two stays with the sequence: its chunks are none either.
 constexpr uint32_t kSmallMaxChunk = 32, kSmallMaxStocks = 256;
 template <class RT>
 bool level_is_small(const OuterLevel<RT>& L, int kind, int prec, const OuterBuffers& B) {

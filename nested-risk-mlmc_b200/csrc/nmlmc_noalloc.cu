@@ -161,7 +161,7 @@ extern "C" int nmlmc_sample_level_noalloc(int32_t kind, double tau, double max_l
         if (precision == NMLMC_PREC_FP32) {
             OuterLevel<float> L{};
             L.ell = ell; L.M = M; L.first_index = first_index; L.seed = seed;
-            L.fine_only = ell == 0; L.antithetic = true; L.N0 = N0; L.chunk = chunk;
+            L.fine_only = ell == 0; L.antithetic = true; L.N0 = N0; L.chunk = phase_chunk(N0, chunk);
             L.adaptive_r = (float)adaptive_r; L.cf = cf; L.cc = cc;
             L.adaptive_f = adaptive && cf.max_count > 2 * cf.base_count;
             L.adaptive_c = !L.fine_only && adaptive && cc.max_count > 2 * cc.base_count;
@@ -171,7 +171,7 @@ extern "C" int nmlmc_sample_level_noalloc(int32_t kind, double tau, double max_l
         } else {
             OuterLevel<double> L{};
             L.ell = ell; L.M = M; L.first_index = first_index; L.seed = seed;
-            L.fine_only = ell == 0; L.antithetic = true; L.N0 = N0; L.chunk = chunk;
+            L.fine_only = ell == 0; L.antithetic = true; L.N0 = N0; L.chunk = phase_chunk(N0, chunk);
             L.adaptive_r = adaptive_r; L.cf = cf; L.cc = cc;
             L.adaptive_f = adaptive && cf.max_count > 2 * cf.base_count;
             L.adaptive_c = !L.fine_only && adaptive && cc.max_count > 2 * cc.base_count;

@@ -361,10 +361,14 @@ __device__ __forceinline__ FastColumn load_column(const FastColumn* p) {
 // PF_COLUMN_PIPE: the alias columns with the next four samples' gathers issued before the current
 // four are evaluated (the 128-register variant).
 // Each way is an instantiation of its own of the phase kernel, with its own registers and code
-// (PF_GENERIC: the reference-arithmetic table, and every other kind).
-enum PfMode : int { PF_GENERIC = -1, PF_UNIFORM = 0, PF_ALIAS = 1, PF_COLUMN = 2, PF_COLUMN_PIPE = 3, PF_UNIFORM_L1 = 4,
-                    PF_COLUMN_L1 = 5 };
+// (PF_GENERIC: the reference-arithmetic table, and every other kind).  PF_ANY and PF_ANY_PACKED are
+// PF_GENERIC and the packed records for chunks that are no power of two (phase_chunk): their length
+// is a run-time value, and one instantiation serves every way to draw.
+enum PfMode : int { PF_ANY = -2, PF_GENERIC = -1, PF_UNIFORM = 0, PF_ALIAS = 1, PF_COLUMN = 2, PF_COLUMN_PIPE = 3,
+                    PF_UNIFORM_L1 = 4, PF_COLUMN_L1 = 5, PF_ANY_PACKED = 6 };
 constexpr bool is_column(int mode) { return mode == PF_COLUMN || mode == PF_COLUMN_PIPE || mode == PF_COLUMN_L1; }
+constexpr bool is_packed(int mode) { return mode >= 0; }
+constexpr bool any_chunk(int mode) { return mode == PF_ANY || mode == PF_ANY_PACKED; }
 constexpr uint64_t kL1TableBytes = 1ull << 20;   // uniform draws from tables up to 1 MB read through L1
 // Alias columns of up to 8192 options (256 KB) are read through L1: gathers past it of so few lines
 // queue at their L2 slices.  20 stocks, level 6, 20,001 outer samples at 4096 inner, through L1 and past
@@ -376,6 +380,10 @@ __host__ __device__ __forceinline__ bool columns_in_l1(const OptionTable<float>&
 // option in every mode); Rrow holds (R, ln R) per stock of this outer sample.
 template <int MODE>
 __device__ __forceinline__ float pf_sample_loss(uint64_t v, const OptionTable<float>& ot, const float2* Rrow) {
+    if constexpr (MODE == PF_ANY_PACKED) {
+        if (ot.fast_col) return pf_sample_loss<PF_COLUMN>(v, ot, Rrow);
+        return ot.subsample == SUB_UNIFORM ? pf_sample_loss<PF_UNIFORM>(v, ot, Rrow) : pf_sample_loss<PF_ALIAS>(v, ot, Rrow);
+    }
     uint32_t j, coin;
     draw_column(v, ot.P, j, coin);
     if (is_column(MODE)) {
@@ -437,10 +445,12 @@ __device__ __forceinline__ void column_finish(FastColumn (&c)[4], const uint32_t
 // two at a time, spills included).  PF_COLUMN_PIPE keeps two such groups, A and B: B's blocks and
 // column gathers are issued before A's alias gathers and losses, so B's round trip runs while A is
 // evaluated.  Every mode adds the samples to the sums in the same order.
-template <int PREC, uint32_t C, bool S2, int MODE>
+// CT: C at compile time (0: a run-time length Cr).
+template <int PREC, uint32_t CT, bool S2, int MODE>
 __device__ __forceinline__ void pf_chunk_fast(const TfKey& key, uint32_t tag, uint64_t b0,
                                               const OptionTable<float>& ot, const float2* Rrow, float shift,
-                                              Acc<PREC>& a1, Acc<PREC>& a2) {
+                                              Acc<PREC>& a1, Acc<PREC>& a2, uint32_t Cr) {
+    const uint32_t C = CT ? CT : Cr;
     if constexpr (is_column(MODE) && MODE != PF_COLUMN_PIPE) {
 #pragma unroll 1
         for (uint32_t b = 0; b < C / 2; b += 2) {
@@ -450,7 +460,7 @@ __device__ __forceinline__ void pf_chunk_fast(const TfKey& key, uint32_t tag, ui
             column_finish<PREC, S2, MODE>(c, coin, ot, Rrow, shift, a1, a2);
         }
     } else if constexpr (MODE == PF_COLUMN_PIPE) {
-        constexpr uint32_t G = C / 4;           // groups of four samples
+        constexpr uint32_t G = CT / 4;          // groups of four samples
         FastColumn ca[4], cb[4];
         uint32_t ka[4], kb[4];
         column_issue<false>(key, tag, b0, ot, ca, ka);
@@ -533,8 +543,9 @@ __device__ __forceinline__ void* user_ws(const OuterBuffers& B, uint32_t item) {
 // ---- one chunk: inner samples [s0, s0 + C) of phase `tag` of outer sample `item` ----------
 // The chunk's share of sample_inner's sums (nested_sampler.hpp:131-161; model::sampler::
 // sample_inner, model_sampler.cpp:66-79, or the portfolio's inner value above).
-// C (inner samples per chunk) is a compile-time constant so the independent Threefry blocks of a
-// chunk can be interleaved (two at a time) for instruction-level parallelism.
+// CT = C (inner samples per chunk) is a compile-time constant so the independent Threefry blocks of
+// a chunk can be interleaved (two at a time) for instruction-level parallelism; CT = 0 takes the
+// run-time length Cr (chunks that are no power of two, multiples of 4).
 // ---- path-simulated portfolio, FP32 -------------------------------------------------------
 // The Unbiased level of the inner sample with path namespace ns (sample_inner_unbiased,
 // portfolio_sampler.cpp:521-537), the level of the double-precision formula, and its steps.
@@ -774,11 +785,13 @@ __device__ __forceinline__ void pf_paths_sorted(const DevLevel<float>& D, const 
     }
 }
 
-template <class RT, int KIND, int PREC, uint32_t C, bool S2, class S, int PM>
+template <class RT, int KIND, int PREC, uint32_t CT, bool S2, class S, int PM>
 __device__ __forceinline__ void eval_chunk_c(const DevLevel<RT>& D, uint32_t item, uint32_t tag,
-                                             uint64_t s0, uint64_t count, float shift, const float2* srow,
+                                             uint64_t s0, uint64_t count, uint32_t Cr, float shift, const float2* srow,
                                              Acc<PREC>& a1, Acc<PREC>& a2, double& work, bool own) {
-    if (!own && !(KIND == KIND_PF_PATHS && PREC == PREC_FP32 && C <= kPathSortChunk)) return;
+    constexpr bool kSorted = KIND == KIND_PF_PATHS && PREC == PREC_FP32 && CT != 0 && CT <= kPathSortChunk;
+    if (!own && !kSorted) return;
+    const uint32_t C = CT ? CT : Cr;
     const OuterLevel<RT>& L = D.L;
     const TfKey key = tf_key(L.seed, outer_stream_id(L.ell, L.first_index + item));
     const RT* Yv = reinterpret_cast<const RT*>(D.B.Yv);
@@ -836,7 +849,7 @@ __device__ __forceinline__ void eval_chunk_c(const DevLevel<RT>& D, uint32_t ite
             a1.add2(X[0], X[1]);
         }
         work += (double)C;
-    } else if constexpr (KIND == KIND_PORTFOLIO && PREC == PREC_FP32 && PM != PF_GENERIC) {
+    } else if constexpr (KIND == KIND_PORTFOLIO && PREC == PREC_FP32 && is_packed(PM)) {
         // portfolio, FP32: packed records scaled by 1 / (sampling probability), the SFU
         // Black-Scholes (nmlmc_bs.cuh); X = loss_j / phat_j.  srow: the outer sample's R_tau row
         // staged in shared memory, else read from the batch buffer.
@@ -844,14 +857,14 @@ __device__ __forceinline__ void eval_chunk_c(const DevLevel<RT>& D, uint32_t ite
             const OptionTable<float>& ot = L.ot;
             const float2* grow = reinterpret_cast<const float2*>(D.B.Rt) + (size_t)item * ot.Q;
             const uint64_t b0 = s0 >> 1;
-            if (srow) pf_chunk_fast<PREC, C, S2, PM>(key, tag, b0, ot, srow, shift, a1, a2);
-            else pf_chunk_fast<PREC, C, S2, PM>(key, tag, b0, ot, grow, shift, a1, a2);
+            if (srow) pf_chunk_fast<PREC, CT, S2, PM>(key, tag, b0, ot, srow, shift, a1, a2, Cr);
+            else pf_chunk_fast<PREC, CT, S2, PM>(key, tag, b0, ot, grow, shift, a1, a2, Cr);
         }
         work += (double)C;
-    } else if constexpr (KIND == KIND_PF_PATHS && PREC == PREC_FP32 && C <= kPathSortChunk) {
+    } else if constexpr (kSorted) {
         if constexpr (sizeof(RT) == 4) {
             const float* Rrow = reinterpret_cast<const float*>(D.B.Rt) + (size_t)item * L.ot.Q * 2;
-            pf_paths_sorted<C, S2, PREC>(D, key, tag, s0, Rrow, shift, a1, a2, work, own);
+            pf_paths_sorted<CT, S2, PREC>(D, key, tag, s0, Rrow, shift, a1, a2, work, own);
         }
     } else {                                     // portfolio: one 64-bit value per inner sample
         const OptionTable<RT>& ot = L.ot;
@@ -911,12 +924,16 @@ __device__ __forceinline__ void eval_chunk_s(const DevLevel<RT>& D, uint32_t ite
                                              uint64_t s0, uint64_t count, uint32_t C, float shift,
                                              const float2* srow, Acc<PREC>& a1, Acc<PREC>& a2, double& work,
                                              bool own) {
+    if constexpr (any_chunk(PM)) {
+        eval_chunk_c<RT, KIND, PREC, 0, S2, S, PM>(D, item, tag, s0, count, C, shift, srow, a1, a2, work, own);
+        return;
+    }
     switch (C) {
-    case 64: eval_chunk_c<RT, KIND, PREC, 64, S2, S, PM>(D, item, tag, s0, count, shift, srow, a1, a2, work, own); break;
-    case 32: eval_chunk_c<RT, KIND, PREC, 32, S2, S, PM>(D, item, tag, s0, count, shift, srow, a1, a2, work, own); break;
-    case 16: eval_chunk_c<RT, KIND, PREC, 16, S2, S, PM>(D, item, tag, s0, count, shift, srow, a1, a2, work, own); break;
-    case 8: eval_chunk_c<RT, KIND, PREC, 8, S2, S, PM>(D, item, tag, s0, count, shift, srow, a1, a2, work, own); break;
-    default: eval_chunk_c<RT, KIND, PREC, 4, S2, S, PM>(D, item, tag, s0, count, shift, srow, a1, a2, work, own); break;
+    case 64: eval_chunk_c<RT, KIND, PREC, 64, S2, S, PM>(D, item, tag, s0, count, C, shift, srow, a1, a2, work, own); break;
+    case 32: eval_chunk_c<RT, KIND, PREC, 32, S2, S, PM>(D, item, tag, s0, count, C, shift, srow, a1, a2, work, own); break;
+    case 16: eval_chunk_c<RT, KIND, PREC, 16, S2, S, PM>(D, item, tag, s0, count, C, shift, srow, a1, a2, work, own); break;
+    case 8: eval_chunk_c<RT, KIND, PREC, 8, S2, S, PM>(D, item, tag, s0, count, C, shift, srow, a1, a2, work, own); break;
+    default: eval_chunk_c<RT, KIND, PREC, 4, S2, S, PM>(D, item, tag, s0, count, C, shift, srow, a1, a2, work, own); break;
     }
 }
 
@@ -1171,7 +1188,7 @@ __global__ void __launch_bounds__(kTile, MINB) k_phase(DevLevel<RT> D, SegSet SS
     // R_tau rows of the FP32 portfolio path can be staged (kRowItems rows of Q stocks)
     const uint32_t Qs = D.L.ot.Q;
     const float2* Rt2 = reinterpret_cast<const float2*>(D.B.Rt);
-    const bool can_stage = KIND == KIND_PORTFOLIO && PREC == PREC_FP32 && PM != PF_GENERIC && Qs <= kMaxStagedStocks;
+    const bool can_stage = KIND == KIND_PORTFOLIO && PREC == PREC_FP32 && is_packed(PM) && Qs <= kMaxStagedStocks;
     const uint32_t C = D.L.chunk;
     uint32_t* counters = D.B.counters;
     double wsum = 0;                                     // work of this thread's chunks
@@ -1812,7 +1829,7 @@ static void launch_phase_v(const DevLevel<RT>& D, const SegSet& SS, TraceRec* tr
     // staged rows of the portfolio's own length: what they leave is L1 for the option table
     size_t dyn = phase_dyn_smem<KIND, PREC>();
     if (KIND == KIND_PORTFOLIO && PREC == PREC_FP32)
-        dyn = PM == PF_GENERIC || D.L.ot.Q > kMaxStagedStocks ? 0 : (size_t)kRowItems * D.L.ot.Q * sizeof(float2);
+        dyn = !is_packed(PM) || D.L.ot.Q > kMaxStagedStocks ? 0 : (size_t)kRowItems * D.L.ot.Q * sizeof(float2);
     k_phase<RT, KIND, PREC, MINB, S, PM><<<grid, kTile, dyn, stream>>>(D, SS, trace);
     if (D.B.prof_mark) D.B.prof_mark(D.B.prof_user, 1, stream);
     count_launch();
@@ -1836,8 +1853,15 @@ static void launch_variant(const DevLevel<RT>& D, const SegSet& SS, TraceRec* tr
 // at one, 632 at two.  The models in the parity precisions do so where the first pilots have a wave
 // of tiles for it (FP64 level 3: 2e6 outer samples 2.67 ms at one CTA, 1.90 at two; 20,000: 110 and 119
 // us).
+// Chunks that are no power of two (N0 neither) run their one instantiation at the compiler's choice
+// of registers.
 template <class RT, int KIND, int PREC, class S = NoSampler>
 static void launch_phase(const DevLevel<RT>& D, const SegSet& SS, TraceRec* trace, cudaStream_t stream) {
+    if (D.L.chunk & (D.L.chunk - 1)) {
+        if constexpr (KIND == KIND_PORTFOLIO && PREC == PREC_FP32)
+            if (D.L.ot.fast_s) return launch_phase_v<RT, KIND, PREC, 1, S, PF_ANY_PACKED>(D, SS, trace, stream);
+        return launch_phase_v<RT, KIND, PREC, 1, S, PF_ANY>(D, SS, trace, stream);
+    }
     if constexpr (KIND == KIND_PORTFOLIO && PREC == PREC_FP32) {
         const OptionTable<RT>& ot = D.L.ot;
         if (!ot.fast_s) return launch_phase_v<RT, KIND, PREC, 2, S>(D, SS, trace, stream);
@@ -1876,6 +1900,7 @@ static cudaError_t run_batch(DevLevel<RT>& D, uint32_t nb, TraceRec* trace, cuda
     if (og > grid) og = grid;
     if (og < 1) og = 1;
     const uint64_t maxc = (L.fine_only || L.cf.max_count >= L.cc.max_count) ? L.cf.max_count : L.cc.max_count;
+    if (maxc % C || ((maxc / C) & (maxc / C - 1))) return cudaErrorInvalidValue;      // phase_chunk
     if (first) {
         // CTAs of the phase launches: at most two tiles (fine and coarse) per 256 chunks of the
         // largest count, so a small call neither starts nor sums hundreds of idle CTAs
