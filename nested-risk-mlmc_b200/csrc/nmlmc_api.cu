@@ -1304,8 +1304,7 @@ static int set_portfolio_impl(nmlmc_ctx* c, const nmlmc_portfolio* p, const nmlm
     const int32_t* method = pm ? pm->method : nullptr;
     if (pm && (pm->dt_h0inv == 0 || pm->dt_beta < 2 || !(pm->dt_prob_expo < 0)))
         return set_err(NMLMC_ERR_ARG);                     // portfolio_sampler.cpp:525
-    HostPortfolio& h = c->pf;
-    h = HostPortfolio{};
+    HostPortfolio h;             // the context's is replaced when every check has passed
     h.Q = p->Q;
     h.P = p->P;
     h.S0.assign(p->S0, p->S0 + p->Q);
@@ -1353,6 +1352,7 @@ static int set_portfolio_impl(nmlmc_ctx* c, const nmlmc_portfolio* p, const nmlm
         if (out_start) out_start[h.order[k]] = h.start[k];
         if (out_delta) out_delta[h.order[k]] = h.delta_est[k];
     }
+    c->pf = std::move(h);
     c->kind = KIND_PORTFOLIO;
     c->pf_prec = -1;
     reset_phase(c);
@@ -1949,8 +1949,7 @@ static int portfolio_from_ref(const portfolio_data* d) {
     if (d->options[1].size + d->options[2].size &&
         (d->dt_h0inv == 0 || d->dt_beta < 2 || !(d->dt_prob_expo < 0)))
         return NMLMC_ERR_ARG;                                            // portfolio_sampler.cpp:525
-    HostPortfolio& h = g_ctx->pf;
-    h = HostPortfolio{};
+    HostPortfolio h;             // the context's is replaced when every check has passed
     h.Q = (uint32_t)s.size;
     h.P = (uint32_t)P;
     for (size_t i = 0; i < s.size; i++) {
@@ -1979,6 +1978,7 @@ static int portfolio_from_ref(const portfolio_data* d) {
     h.use_coarse_delta_cv = d->use_coarse_delta_cv ? 1 : 0;
     h.use_antithetic_risk = d->use_antithetic_risk ? 1 : 0;
     h.use_milstein = d->use_milstein ? 1 : 0;
+    g_ctx->pf = std::move(h);
     g_ctx->kind = KIND_PORTFOLIO;
     g_ctx->pf_prec = -1;
     return ensure_portfolio(g_ctx);

@@ -70,3 +70,29 @@ def test_non_finite_inputs_are_rejected(nm):
         s.set_portfolio(pf, max_loss=float("nan"))
     s.set_portfolio(pf, max_loss=1.0)                    # the valid portfolio is accepted
     assert s.sample(1, 100)["M"] == 100
+
+
+@pytest.mark.parametrize("bad", ["stock", "type", "prob", "method"])
+def test_a_rejected_portfolio_leaves_the_context_as_it_was(nm, bad):
+    """nmlmc_set_portfolio checks everything before it replaces the portfolio in place."""
+    pf, other = O.synthetic_portfolio(9, 120, 3), O.synthetic_portfolio(2, 30, 4)
+    methods = None
+    if bad == "stock":
+        other["stock_ind"] = np.array(other["stock_ind"]) + 5
+    elif bad == "type":
+        other["type"] = np.zeros_like(other["type"])
+    elif bad == "prob":
+        other["prob"] = np.linspace(1.0, 2.0, 30)               # not falling
+    else:
+        methods = dict(method=[3] * 30)
+    s, ref = _model(nm), _model(nm)
+    for x in (s, ref):
+        x.set_portfolio(pf, max_loss=1.0)
+    with pytest.raises(nm.NmlmcError) as e:
+        s.set_portfolio(other, max_loss=5.0, methods=methods)
+    assert e.value.status == nm.ERR_ARG
+    for ell, M in ((0, 300), (3, 200)):
+        a, b = s.sample(ell, M), ref.sample(ell, M)
+        np.testing.assert_array_equal(a["fsums"], b["fsums"])
+        np.testing.assert_array_equal(a["stats"], b["stats"])
+    np.testing.assert_array_equal(s.full_loss(0, 0, 50), ref.full_loss(0, 0, 50))
