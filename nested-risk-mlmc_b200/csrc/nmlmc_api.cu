@@ -241,7 +241,12 @@ cudaError_t dev_malloc(T** p, size_t bytes) {
         return cudaErrorMemoryAllocation;
     }
     if (k > 0) g_fail_alloc.store(k - 1);
-    return cudaMalloc(p, bytes);
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) {
+        *p = nullptr;
+        cudaGetLastError();                       // reported here, not by the next launch's check
+    }
+    return e;
 }
 
 int set_err(int e) {
@@ -279,6 +284,19 @@ void dfree(T*& p) {
     p = nullptr;
 }
 
+// Allocation of a context's own buffers.  The block that nmlmc_path_adjoint keeps between calls
+// makes room where it is in the way.
+template <class T>
+cudaError_t ctx_malloc(nmlmc_ctx* c, T** p, size_t bytes) {
+    cudaError_t e = dev_malloc(p, bytes);
+    if (e != cudaSuccess && c->adj_mem) {
+        dfree(c->adj_mem);
+        c->adj_bytes = 0;
+        e = dev_malloc(p, bytes);
+    }
+    return e;
+}
+
 template <class RT>
 void free_dev_portfolio(DevPortfolio<RT>& d) {
     dfree(d.strike); dfree(d.maturity); dfree(d.start); dfree(d.w); dfree(d.prob); dfree(d.W_est);
@@ -288,10 +306,10 @@ void free_dev_portfolio(DevPortfolio<RT>& d) {
 }
 
 template <class T>
-int upload(T*& d, const std::vector<T>& h) {
+int upload(nmlmc_ctx* c, T*& d, const std::vector<T>& h) {
     dfree(d);
     size_t n = h.size() ? h.size() : 1;
-    if (dev_malloc(&d, n * sizeof(T)) != cudaSuccess) return set_err(NMLMC_ERR_NOMEM);
+    if (ctx_malloc(c, &d, n * sizeof(T)) != cudaSuccess) return set_err(NMLMC_ERR_NOMEM);
     if (!h.empty()) NM_CUDA(cudaMemcpy(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice), "upload");
     return NMLMC_OK;
 }
@@ -389,11 +407,11 @@ int build_dev_portfolio(nmlmc_ctx* c, DevPortfolio<RT>& d) {
         cprob[m] += prob[j];
     }
     int rc;
-    if ((rc = upload(d.strike, K)) || (rc = upload(d.maturity, T)) || (rc = upload(d.start, start)) ||
-        (rc = upload(d.w, w)) || (rc = upload(d.prob, prob)) || (rc = upload(d.W_est, West)) ||
-        (rc = upload(d.cdf, cdf)) || (rc = upload(d.S0, S0)) || (rc = upload(d.mu, mu)) ||
-        (rc = upload(d.sigma, sg)) || (rc = upload(d.delta_coalesce, delta)) ||
-        (rc = upload(d.stock_ind, h.stock_ind)) || (rc = upload(d.type, h.type)))
+    if ((rc = upload(c, d.strike, K)) || (rc = upload(c, d.maturity, T)) || (rc = upload(c, d.start, start)) ||
+        (rc = upload(c, d.w, w)) || (rc = upload(c, d.prob, prob)) || (rc = upload(c, d.W_est, West)) ||
+        (rc = upload(c, d.cdf, cdf)) || (rc = upload(c, d.S0, S0)) || (rc = upload(c, d.mu, mu)) ||
+        (rc = upload(c, d.sigma, sg)) || (rc = upload(c, d.delta_coalesce, delta)) ||
+        (rc = upload(c, d.stock_ind, h.stock_ind)) || (rc = upload(c, d.type, h.type)))
         return rc;
     OptionTable<RT>& t = d.table;
     t.strike = d.strike; t.maturity = d.maturity; t.start = d.start; t.w = d.w; t.prob = d.prob;
@@ -428,7 +446,7 @@ int build_dev_portfolio(nmlmc_ctx* c, DevPortfolio<RT>& d) {
                 guide.push_back(i ? i - 1 : 0);
             }
         }
-        if ((rc = upload(d.guide, guide))) return rc;
+        if ((rc = upload(c, d.guide, guide))) return rc;
         t.guide = d.guide;
     }
     t.fast = nullptr;
@@ -444,7 +462,7 @@ int build_dev_portfolio(nmlmc_ctx* c, DevPortfolio<RT>& d) {
         build_alias(P, pr, tab, phat);
         std::vector<RT> ph(P);
         for (uint32_t j = 0; j < P; j++) ph[j] = (RT)phat[j];
-        if ((rc = upload(d.alias, tab)) || (rc = upload(d.phat, ph))) return rc;
+        if ((rc = upload(c, d.alias, tab)) || (rc = upload(c, d.phat, ph))) return rc;
         t.alias = d.alias;
         t.phat = d.phat;
     }
@@ -469,14 +487,14 @@ int build_dev_portfolio(nmlmc_ctx* c, DevPortfolio<RT>& d) {
                 po[j] = PathOption{S0[s], sg[s], K[j], T[j], w[j], West[j],
                                    h.subsample == SUB_RANDOM ? (float)phat[j] : t.inv_count_prob, s << 1 | (h.type[j] > 0 ? 1u : 0u)};
             }
-            if ((rc = upload(d.path, po))) return rc;
+            if ((rc = upload(c, d.path, po))) return rc;
             t.path = d.path;
         }
     }
     if (reference) {
-        if (dev_malloc(&d.ref, P * sizeof(RefOption<RT>)) != cudaSuccess ||
-            dev_malloc(&d.lvl_w, kPathLevels * sizeof(RT)) != cudaSuccess ||
-            dev_malloc(&d.lvl_wf, kPathLevels * sizeof(float)) != cudaSuccess)
+        if (ctx_malloc(c, &d.ref, P * sizeof(RefOption<RT>)) != cudaSuccess ||
+            ctx_malloc(c, &d.lvl_w, kPathLevels * sizeof(RT)) != cudaSuccess ||
+            ctx_malloc(c, &d.lvl_wf, kPathLevels * sizeof(float)) != cudaSuccess)
             return set_err(NMLMC_ERR_NOMEM);
         NM_CUDA(cudaStreamSynchronize(nullptr), "uploads");      // the tables it reads: c->stream does not wait for them
         NM_CUDA(launch_ref_records(t, d.ref, d.lvl_w, d.lvl_wf, c->stream), "option constants");
@@ -512,7 +530,7 @@ int build_dev_portfolio(nmlmc_ctx* c, DevPortfolio<RT>& d) {
             // full-loss records: the loss L(Y) itself, no control variate
             std::vector<FastOption> fo(P);
             for (uint32_t j = 0; j < P; j++) fo[j] = record(j, 1.0, false);
-            if ((rc = upload(d.fast, fo))) return rc;
+            if ((rc = upload(c, d.fast, fo))) return rc;
             t.fast = d.fast;
             if (h.subsample != SUB_NONE) {
                 // sampler records: the inner value X = loss_j / phat_j folded into the weights
@@ -520,7 +538,7 @@ int build_dev_portfolio(nmlmc_ctx* c, DevPortfolio<RT>& d) {
                     const double sc = h.subsample == SUB_UNIFORM ? (double)P : (phat[j] > 0 ? 1.0 / phat[j] : 0.0);
                     fo[j] = record(j, sc, h.use_delta_cv != 0);
                 }
-                if ((rc = upload(d.fast_s, fo))) return rc;
+                if ((rc = upload(c, d.fast_s, fo))) return rc;
                 t.fast_s = d.fast_s;
                 if (h.subsample == SUB_RANDOM && Q <= kColumnMaxStocks && P < kColumnMaxOptions) {
                     std::vector<FastColumn> col(P);
@@ -528,7 +546,7 @@ int build_dev_portfolio(nmlmc_ctx* c, DevPortfolio<RT>& d) {
                         const FastOption& o = fo[j];
                         col[j] = FastColumn{o.c1, o.inv_s, o.wR, o.wK, o.wV0, o.cv, tab[j].x, (tab[j].y << 8) | o.stock};
                     }
-                    if ((rc = upload(d.fast_col, col))) return rc;
+                    if ((rc = upload(c, d.fast_col, col))) return rc;
                     t.fast_col = d.fast_col;
                 }
             }
@@ -584,10 +602,10 @@ int alloc_core(nmlmc_ctx* c) {
     dfree(c->d_states); dfree(c->d_states_next); dfree(c->d_core_part); dfree(c->d_core_counts);
     c->states_cores = 0;
     const size_t nc = core_counts(cores) * sizeof(uint32_t);
-    if (dev_malloc(&c->d_states, (size_t)cores * 2 * sizeof(CoreStream)) != cudaSuccess ||
-        dev_malloc(&c->d_states_next, (size_t)cores * 2 * sizeof(CoreStream)) != cudaSuccess ||
-        dev_malloc(&c->d_core_part, core_part_words(cores) * sizeof(uint64_t)) != cudaSuccess ||
-        dev_malloc(&c->d_core_counts, nc) != cudaSuccess) {
+    if (ctx_malloc(c, &c->d_states, (size_t)cores * 2 * sizeof(CoreStream)) != cudaSuccess ||
+        ctx_malloc(c, &c->d_states_next, (size_t)cores * 2 * sizeof(CoreStream)) != cudaSuccess ||
+        ctx_malloc(c, &c->d_core_part, core_part_words(cores) * sizeof(uint64_t)) != cudaSuccess ||
+        ctx_malloc(c, &c->d_core_counts, nc) != cudaSuccess) {
         dfree(c->d_states); dfree(c->d_states_next); dfree(c->d_core_part); dfree(c->d_core_counts);
         return set_err(NMLMC_ERR_NOMEM);
     }
@@ -645,15 +663,15 @@ int alloc_outer(nmlmc_ctx* c, uint64_t want) {
     B.cap = cap;
     B.Q = Q;
     B.grid = sms * 4;            // partial-sum slots; the phase kernel runs its resident CTAs (<= grid)
-    bool ok = dev_malloc(&B.Yv, cap * sizeof(double)) == cudaSuccess &&
-              dev_malloc(&B.Rt, (Q ? cap * Q : 1) * sizeof(double)) == cudaSuccess &&
-              dev_malloc(&B.cnt_f, cap * sizeof(uint32_t)) == cudaSuccess &&
-              dev_malloc(&B.cnt_c, cap * sizeof(uint32_t)) == cudaSuccess &&
-              dev_malloc(&B.lists, 4 * cap * sizeof(uint32_t)) == cudaSuccess &&
-              dev_malloc(&B.class_items, cap * sizeof(uint32_t)) == cudaSuccess &&
-              dev_malloc(&B.counters, kCounterSlots * sizeof(uint32_t)) == cudaSuccess &&
-              dev_malloc(&B.block_sums, (size_t)B.grid * 16 * sizeof(double)) == cudaSuccess &&
-              dev_malloc(&B.level_acc, kMaxSubmit * 16 * sizeof(double)) == cudaSuccess;
+    bool ok = ctx_malloc(c, &B.Yv, cap * sizeof(double)) == cudaSuccess &&
+              ctx_malloc(c, &B.Rt, (Q ? cap * Q : 1) * sizeof(double)) == cudaSuccess &&
+              ctx_malloc(c, &B.cnt_f, cap * sizeof(uint32_t)) == cudaSuccess &&
+              ctx_malloc(c, &B.cnt_c, cap * sizeof(uint32_t)) == cudaSuccess &&
+              ctx_malloc(c, &B.lists, 4 * cap * sizeof(uint32_t)) == cudaSuccess &&
+              ctx_malloc(c, &B.class_items, cap * sizeof(uint32_t)) == cudaSuccess &&
+              ctx_malloc(c, &B.counters, kCounterSlots * sizeof(uint32_t)) == cudaSuccess &&
+              ctx_malloc(c, &B.block_sums, (size_t)B.grid * 16 * sizeof(double)) == cudaSuccess &&
+              ctx_malloc(c, &B.level_acc, kMaxSubmit * 16 * sizeof(double)) == cudaSuccess;
     c->ob_alloc = true;                   // free_outer releases a partial set too
     if (!ok) {
         free_outer(c);
@@ -684,7 +702,7 @@ int ensure_trace(nmlmc_ctx* c, uint64_t M) {
     if (M > c->trace_cap) return set_err(NMLMC_ERR_ARG);
     if (c->d_trace_cap < M) {
         dfree(c->d_trace);
-        if (dev_malloc(&c->d_trace, M * sizeof(TraceRec)) != cudaSuccess) return set_err(NMLMC_ERR_NOMEM);
+        if (ctx_malloc(c, &c->d_trace, M * sizeof(TraceRec)) != cudaSuccess) return set_err(NMLMC_ERR_NOMEM);
         c->d_trace_cap = M;
     }
     return NMLMC_OK;
@@ -996,9 +1014,9 @@ OuterBuffers side_buffers(const nmlmc_ctx* c, uint32_t i, uint64_t off, uint64_t
 int ensure_side(nmlmc_ctx* c, uint32_t n) {
     if (!c->side_sums) {
         const size_t nc = (kSideLevels - 1) * kCounterSlots * sizeof(uint32_t);
-        if (!c->side_counters && dev_malloc(&c->side_counters, nc) != cudaSuccess) return set_err(NMLMC_ERR_NOMEM);
+        if (!c->side_counters && ctx_malloc(c, &c->side_counters, nc) != cudaSuccess) return set_err(NMLMC_ERR_NOMEM);
         NM_CUDA(cudaMemsetAsync(c->side_counters, 0, nc, c->stream), "memset");
-        if (dev_malloc(&c->side_sums, (size_t)(kSideLevels - 1) * c->ob.grid * 16 * sizeof(double)) != cudaSuccess) {
+        if (ctx_malloc(c, &c->side_sums, (size_t)(kSideLevels - 1) * c->ob.grid * 16 * sizeof(double)) != cudaSuccess) {
             c->side_sums = nullptr;
             return set_err(NMLMC_ERR_NOMEM);
         }
@@ -1376,19 +1394,16 @@ int nmlmc_set_portfolio_methods(nmlmc_ctx* c, const nmlmc_portfolio* p, const nm
 namespace {
 
 // Device memory of nmlmc_path_adjoint calls: one block per context, kept between calls up to
-// kAdjKeepBytes (allocating and freeing two dozen buffers took 2 ms of each call) and released
-// with the context.  The derivatives kept between the two passes take at most kAdjStoreBytes of it.
+// kAdjKeepBytes (allocating and freeing two dozen buffers took 2 ms of each call) and released with
+// the context, or when another allocation of the context needs the room (ctx_malloc).  The derivatives
+// kept between the two passes take at most kAdjStoreBytes of it.
 constexpr size_t kAdjKeepBytes = 5ull << 28, kAdjStoreBytes = 1ull << 30;
 
 int adj_reserve(nmlmc_ctx* c, size_t bytes) {
     if (c->adj_bytes >= bytes) return NMLMC_OK;
     dfree(c->adj_mem);
     c->adj_bytes = 0;
-    if (dev_malloc(&c->adj_mem, bytes) != cudaSuccess) {
-        cudaGetLastError();
-        c->adj_mem = nullptr;
-        return NMLMC_ERR_NOMEM;
-    }
+    if (dev_malloc(&c->adj_mem, bytes) != cudaSuccess) return NMLMC_ERR_NOMEM;
     c->adj_bytes = bytes;
     return NMLMC_OK;
 }

@@ -96,3 +96,43 @@ def test_a_rejected_portfolio_leaves_the_context_as_it_was(nm, bad):
         np.testing.assert_array_equal(a["fsums"], b["fsums"])
         np.testing.assert_array_equal(a["stats"], b["stats"])
     np.testing.assert_array_equal(s.full_loss(0, 0, 50), ref.full_loss(0, 0, 50))
+
+
+def _small_batch(nm):
+    g = np.random.default_rng(4)
+    P, Q = 300, 4
+    pf = dict(S0=np.full(Q, 100.0), mu=np.full(Q, 0.05), sigma=0.1 + 0.3 * g.random(Q),
+              stock_ind=g.integers(0, Q, P).astype(np.uint32), type=np.where(g.random(P) < 0.5, 1, -1).astype(np.int32),
+              strike=100.0 * (0.8 + 0.4 * g.random(P)), maturity=0.25 + 1.75 * g.random(P), w=g.standard_normal(P))
+    return nm.make_batch([pf], [1.0], r=0.05, rho=0.2, tau=1 / 52)
+
+
+@pytest.mark.parametrize("what", ["buffers", "cores", "portfolio", "trace"])
+def test_the_adjoints_kept_block_is_given_back_to_other_allocations(nm, what):
+    """A context keeps its last nmlmc_path_adjoint's device block; an allocation that fails with it
+    in place is tried again without it."""
+    lib = nm.lib()
+
+    def call(s):
+        if what == "cores":
+            s.configure(precision=nm.PREC_REF32, streams=nm.STREAMS_CORE, cores=64)
+            s.set_model(nm.MODEL_SHIFT, 0.0, 1.0)
+        if what == "portfolio":
+            s.set_portfolio(O.synthetic_portfolio(4, 100, 3), max_loss=1.0)
+        return s.sample(2, 500, trace=what == "trace")
+
+    want = call(_model(nm))
+    s = _model(nm)
+    if what == "trace":
+        s.sample(2, 500)                        # its buffers are there: the trace's allocation is next
+        s.reset_streams()
+    adj = s.path_adjoint(_small_batch(nm), ell=2, pairs=1, M=64, seed=3)
+    try:
+        lib.nmlmc_inject_alloc_failure(0)
+        got = call(s)
+    finally:
+        lib.nmlmc_inject_alloc_failure(-1)
+    np.testing.assert_array_equal(got["fsums"], want["fsums"])
+    np.testing.assert_array_equal(got["diffsums"], want["diffsums"])
+    again = s.path_adjoint(_small_batch(nm), ell=2, pairs=1, M=64, seed=3)
+    np.testing.assert_allclose(again["grad_w_EL"], adj["grad_w_EL"], rtol=1e-12, atol=1e-11)
