@@ -1011,21 +1011,26 @@ OuterBuffers side_buffers(const nmlmc_ctx* c, uint32_t i, uint64_t off, uint64_t
     return B;
 }
 
-int ensure_side(nmlmc_ctx* c, uint32_t n) {
-    if (!c->side_sums) {
-        const size_t nc = (kSideLevels - 1) * kCounterSlots * sizeof(uint32_t);
-        if (!c->side_counters && ctx_malloc(c, &c->side_counters, nc) != cudaSuccess) return set_err(NMLMC_ERR_NOMEM);
-        NM_CUDA(cudaMemsetAsync(c->side_counters, 0, nc, c->stream), "memset");
-        if (ctx_malloc(c, &c->side_sums, (size_t)(kSideLevels - 1) * c->ob.grid * 16 * sizeof(double)) != cudaSuccess) {
-            c->side_sums = nullptr;
-            return set_err(NMLMC_ERR_NOMEM);
+// Buffers, streams and events for `n` levels side by side.  False where they cannot be had: the
+// levels then run one after another.
+bool ensure_side(nmlmc_ctx* c, uint32_t n) {
+    const size_t nc = (kSideLevels - 1) * kCounterSlots * sizeof(uint32_t);
+    bool ok = true;
+    if (!c->side_counters) {
+        ok = ctx_malloc(c, &c->side_counters, nc) == cudaSuccess;
+        if (ok && cudaMemsetAsync(c->side_counters, 0, nc, c->stream) != cudaSuccess) {
+            dfree(c->side_counters);
+            ok = false;
         }
     }
-    for (uint32_t i = 0; i < n; i++) {
-        if (!c->side[i]) NM_CUDA(cudaStreamCreateWithFlags(&c->side[i], cudaStreamNonBlocking), "side stream");
-        if (!c->side_ev[i]) NM_CUDA(cudaEventCreateWithFlags(&c->side_ev[i], cudaEventDisableTiming), "side event");
+    if (ok && !c->side_sums)
+        ok = ctx_malloc(c, &c->side_sums, (size_t)(kSideLevels - 1) * c->ob.grid * 16 * sizeof(double)) == cudaSuccess;
+    for (uint32_t i = 0; i < n && ok; i++) {
+        if (!c->side[i]) ok = cudaStreamCreateWithFlags(&c->side[i], cudaStreamNonBlocking) == cudaSuccess;
+        if (ok && !c->side_ev[i]) ok = cudaEventCreateWithFlags(&c->side_ev[i], cudaEventDisableTiming) == cudaSuccess;
     }
-    return NMLMC_OK;
+    if (!ok) cudaGetLastError();
+    return ok;
 }
 
 // All levels of one MLMC round in one submission: the level sequences are captured from the
@@ -1069,12 +1074,8 @@ int sample_outer_levels(nmlmc_ctx* c, uint32_t n, const uint32_t* ells, const ui
     // ms).  Larger rounds fill it level by level.
     uint64_t total = 0;
     for (uint64_t m : Ms) total += m;
-    const bool side = n > 1 && n <= kSideLevels && total <= ob.cap;
+    const bool side = n > 1 && n <= kSideLevels && total <= ob.cap && ensure_side(c, n);
     key.push_back(side);
-    if (side) {
-        const int rc = ensure_side(c, n);
-        if (rc) return rc;
-    }
     // the executable graph of a recent round with the same levels is reused if it runs no level as
     // one kernel that is too large for it now, and at most one small level as a sequence (60 us more,
     // an instantiation costs 100 us)

@@ -136,3 +136,25 @@ def test_the_adjoints_kept_block_is_given_back_to_other_allocations(nm, what):
     np.testing.assert_array_equal(got["diffsums"], want["diffsums"])
     again = s.path_adjoint(_small_batch(nm), ell=2, pairs=1, M=64, seed=3)
     np.testing.assert_allclose(again["grad_w_EL"], adj["grad_w_EL"], rtol=1e-12, atol=1e-11)
+
+
+@pytest.mark.parametrize("after", [0, 1])
+def test_a_round_without_room_to_overlap_runs_its_levels_in_turn(nm, after):
+    """The counters and partial sums of levels that run side by side are optional."""
+    lib = nm.lib()
+    s, ref = _model(nm), _model(nm)
+    s.sample(0, 10)                             # the batch buffers: only the side buffers are left to allocate
+    ref.sample(0, 10)
+    want = [ref.sample(e, m) for e, m in ((0, 4000), (2, 1000), (5, 300))]
+    try:
+        lib.nmlmc_inject_alloc_failure(after)
+        got = s.sample_levels([0, 2, 5], [4000, 1000, 300])
+    finally:
+        lib.nmlmc_inject_alloc_failure(-1)
+    for x, y in zip(got, want):
+        np.testing.assert_array_equal(x["fsums"], y["fsums"])
+        np.testing.assert_array_equal(x["diffsums"], y["diffsums"])
+        np.testing.assert_array_equal(x["stats"], y["stats"])
+    a, b = s.sample_levels([0, 5], [100, 100]), [ref.sample(0, 100), ref.sample(5, 100)]      # with room again
+    for x, y in zip(a, b):
+        np.testing.assert_array_equal(x["fsums"], y["fsums"])
