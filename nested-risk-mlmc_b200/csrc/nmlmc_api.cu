@@ -702,6 +702,7 @@ int ensure_trace(nmlmc_ctx* c, uint64_t M) {
     if (M > c->trace_cap) return set_err(NMLMC_ERR_ARG);
     if (c->d_trace_cap < M) {
         dfree(c->d_trace);
+        c->d_trace_cap = 0;
         if (ctx_malloc(c, &c->d_trace, M * sizeof(TraceRec)) != cudaSuccess) return set_err(NMLMC_ERR_NOMEM);
         c->d_trace_cap = M;
     }

@@ -158,3 +158,19 @@ def test_a_round_without_room_to_overlap_runs_its_levels_in_turn(nm, after):
     a, b = s.sample_levels([0, 5], [100, 100]), [ref.sample(0, 100), ref.sample(5, 100)]      # with room again
     for x, y in zip(a, b):
         np.testing.assert_array_equal(x["fsums"], y["fsums"])
+
+
+def test_a_trace_buffer_that_cannot_grow_can_be_used_again(nm):
+    lib = nm.lib()
+    s, ref = _model(nm), _model(nm)
+    want = ref.sample(2, 300, trace=True)
+    s.sample(1, 500, trace=True)
+    try:
+        lib.nmlmc_inject_alloc_failure(0)
+        with pytest.raises(nm.NmlmcError) as e:
+            s.sample(2, 900, trace=True)
+        assert e.value.status == nm.ERR_NOMEM
+    finally:
+        lib.nmlmc_inject_alloc_failure(-1)
+    got = s.sample(2, 300, trace=True)
+    assert got["trace"].tobytes() == want["trace"].tobytes()
