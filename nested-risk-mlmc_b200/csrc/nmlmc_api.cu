@@ -740,7 +740,6 @@ int sample_core(nmlmc_ctx* c, uint32_t ell, uint64_t M, nmlmc_level_result* out)
     out->M = M;
     memcpy(out->inner_stats, c->h_pin + 10, 6 * sizeof(uint64_t));
     out->seconds = ms * 1e-3;
-    c->trace_host = nullptr;
     if (c->h_pin[9] != 0) return set_err(NMLMC_ERR_LIMIT);   // a sample exceeded kMaxPathSteps
     return NMLMC_OK;
 }
@@ -982,7 +981,6 @@ int sample_outer(nmlmc_ctx* c, uint32_t ell, uint64_t Mtotal, nmlmc_level_result
     cudaEventElapsedTime(&ms, c->ev0, c->ev1);
     fill_outer_result(c, c->h_pin, M, ms * 1e-3, out);
     c->next_outer[ell] += Mtotal;
-    c->trace_host = nullptr;
     return NMLMC_OK;
 }
 
@@ -1562,6 +1560,10 @@ int nmlmc_set_trace(nmlmc_ctx* c, nmlmc_trace_rec* host_buf, uint64_t cap) {
 
 int nmlmc_sample(nmlmc_ctx* c, uint32_t ell, uint64_t M, nmlmc_level_result* out) {
     if (!c || !out) return set_err(NMLMC_ERR_ARG);
+    struct Disarm {                               // the armed buffer is this call's, however it ends
+        nmlmc_ctx* c;
+        ~Disarm() { c->trace_host = nullptr; }
+    } disarm{c};
     if (!c->configured || c->kind < 0) return set_err(NMLMC_ERR_STATE);
     if (ell >= NMLMC_MAX_LEVELS) return set_err(NMLMC_ERR_ARG);
     memset(out, 0, sizeof(*out));

@@ -174,3 +174,28 @@ def test_a_trace_buffer_that_cannot_grow_can_be_used_again(nm):
         lib.nmlmc_inject_alloc_failure(-1)
     got = s.sample(2, 300, trace=True)
     assert got["trace"].tobytes() == want["trace"].tobytes()
+
+
+def test_an_armed_trace_buffer_is_used_by_one_call(nm):
+    """A call that fails, or draws nothing, disarms the buffer too: the next one does not write it."""
+    s = _model(nm)
+    buf = np.zeros(50, nm.TRACE_DTYPE)
+
+    def arm():
+        assert nm.lib().nmlmc_set_trace(s.h, buf.ctypes.data, 50) == nm.OK
+
+    arm()
+    assert s.sample(2, 0)["M"] == 0
+    s.sample(2, 40)
+    arm()
+    with pytest.raises(nm.NmlmcError):
+        s.sample(40, 10)                         # no such level
+    s.sample(2, 40)
+    arm()
+    with pytest.raises(nm.NmlmcError):
+        s.sample(2, 60)                          # more samples than the buffer holds
+    assert s.sample(2, 60)["M"] == 60
+    assert not buf.view(np.uint8).any()
+    arm()
+    s.sample(2, 40)
+    assert buf["count_f"][:40].all() and not buf["count_f"][40:].any()
