@@ -307,16 +307,18 @@ int nmlmc_sample_levels(nmlmc_ctx* ctx, uint32_t n, const uint32_t* ells, const 
 /* ---- phase-kernel autotuner (batched FP32 path) ----------------------------------------------
  * No counterpart in the reference (its CUDA build has one fixed launch shape).  The phase kernel
  * of the OUTER layout has three register/occupancy variants (0: up to 255 registers per thread,
- * 1: three resident CTAs of 256 threads per SM guaranteed, 2: four), for portfolios a fourth (3: two
- * CTAs per SM, with the next inner samples' table gathers issued before the current ones are
- * evaluated; other kinds run variant 0 for it) and a chunk length (inner
+ * 1: three resident CTAs of 256 threads per SM guaranteed, 2: four), for portfolios with importance
+ * sub-sampling from alias columns a fourth (3: two CTAs per SM, with the next inner samples' table
+ * gathers issued before the current ones are evaluated; elsewhere 3 runs as 1) and a chunk length (inner
  * samples per thread; power of two in [4, 64] dividing N0; a level's items of n inner samples
  * take n / chunk threads, so it also sets the outer samples per warp; an N0 that is no power of two
  * runs one variant, with chunks of about that length times its odd factor).  With autotuning on, the
  * first nmlmc_sample / nmlmc_sample_levels call of a level with enough work times the
  * candidates on a probe of the level's own parameters whose outer stream indices start at 2^55
  * (no result changes) and keeps the fastest for that level in the context.  Mode 1 (the
- * default) tunes the variant only; the variants give identical results.  Mode 2 also tries half
+ * default) tunes the variant only; the variants give identical results.  A level that one kernel
+ * serves whatever the variant (a model's at small fixed counts) is tuned without a probe
+ * (probe_ms 0).  Mode 2 also tries half
  * and double the chunk length; another chunk length regroups the FP32 compensated inner sums
  * (last-bit differences of inner means), so pin the configuration to make such runs reproducible
  * across processes.  Changing the model, portfolio or configuration drops the tuned (not the

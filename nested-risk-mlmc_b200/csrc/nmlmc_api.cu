@@ -849,9 +849,9 @@ OuterLevel<RT> outer_level_params(const nmlmc_ctx* c, uint32_t ell, uint64_t M, 
 // parameters on about 20 ms of work (probe_size), from outer samples whose
 // stream indices start at 2^55, far from any real index, so the probe changes no result — and
 // keeps the fastest for the level:
-//   1. the register/occupancy variants 0, 1, 2 (and 3 for the portfolio) at the default chunk
-//      length, another than the
-//      default taken only if > 3 % faster;
+//   1. the register/occupancy variants 0, 1, 2 (and 3 for alias columns) at the default chunk
+//      length, another than the default taken only if > 3 % faster.  A level that has one (k_fixed
+//      among them) takes it without a probe;
 //   2. (mode 2, or an explicit nmlmc_autotune_level) half and double the chunk length at the
 //      best variant, taken only if > 3 % faster.
 // The variants compute identically, so mode 1 never changes a result; the chunk length changes
@@ -865,6 +865,7 @@ cudaError_t time_phase_config(nmlmc_ctx* c, uint32_t ell, uint64_t Mp, const Pha
     OuterLevel<RT> L = outer_level_params<RT>(c, ell, Mp, kProbeIndex);
     L.chunk = phase_chunk(L.N0, pc.chunk);
     L.variant = pc.variant;
+    L.no_small = true;                      // the launch sequence, whose kernels the candidates change
     OuterBuffers B = c->ob;
     B.prof_mark = nullptr;
     B.stamps = nullptr;
@@ -905,20 +906,35 @@ cudaError_t probe_size(nmlmc_ctx* c, uint32_t ell, uint64_t& Mp) {
     }
 }
 
+// Variants of the level's phase kernel at its default chunk length (launch_phase): one where a
+// single instantiation serves it, three with the pipelined loop's alias columns as a fourth.
+template <class RT>
+uint32_t phase_variants(const nmlmc_ctx* c, uint32_t ell) {
+    OuterLevel<RT> L = outer_level_params<RT>(c, ell, 0, 0);
+    L.chunk = phase_chunk(L.N0, default_phase(c).chunk);
+    if ((L.chunk & (L.chunk - 1)) || level_is_fixed(L, c->kind)) return 1;
+    if (c->kind != KIND_PORTFOLIO) return 3;
+    return !L.ot.fast_s ? 1 : L.ot.fast_col ? 4 : 3;
+}
+
 template <class RT>
 int tune_level(nmlmc_ctx* c, uint32_t ell, bool chunks) {
     NvtxRange nv("nmlmc autotune level");
+    PhaseChoice best = default_phase(c);
+    best.state = 1;
+    const uint32_t n_var = phase_variants<RT>(c, ell);
+    if (n_var == 1 && !chunks) {                  // nothing to choose from
+        c->phase[ell] = best;
+        return NMLMC_OK;
+    }
     uint64_t Mp = 0;
     NM_CUDA(probe_size<RT>(c, ell, Mp), "autotune probe size");
     // the default stays unless another candidate is more than 3 % faster on the probe (near-ties
     // on a short probe are noise)
-    PhaseChoice best = default_phase(c);
-    best.state = 1;
     double best_ms;
     NM_CUDA(time_phase_config<RT>(c, ell, Mp, best, best_ms), "autotune probe");
     const uint32_t v0 = best.variant;
-    const uint32_t n_var = c->kind == KIND_PORTFOLIO ? 4u : 3u;   // variant 3: portfolio only
-    for (uint32_t v = 0; v < n_var; v++) {
+    for (uint32_t v = 0; n_var > 1 && v < n_var; v++) {
         if (v == v0) continue;
         PhaseChoice pc = best;
         pc.variant = v;

@@ -129,6 +129,16 @@ bool level_is_small(const OuterLevel<RT>& L, int kind, int prec, const OuterBuff
     return L.M * per * unit <= (pilots ? 6000000ull : is_portfolio_kind(kind) ? 1300000ull : 800000ull);
 }
 
+// Whether a level runs as k_fixed, a thread per outer sample: a model without pilots at up to
+// kFixedChunks chunks per outer sample, however many outer samples.
+constexpr uint32_t kFixedChunks = 4;
+template <class RT>
+bool level_is_fixed(const OuterLevel<RT>& L, int kind) {
+    if (kind != KIND_REF_MODEL && kind != KIND_SHIFT_MODEL) return false;
+    const uint64_t maxc = (L.fine_only || L.cf.max_count >= L.cc.max_count) ? L.cf.max_count : L.cc.max_count;
+    return !L.adaptive_f && !L.adaptive_c && maxc / L.chunk <= kFixedChunks && !(L.N0 & (L.N0 - 1));
+}
+
 // Device counter slot (OuterBuffers::counters) that the batched kernels set when a
 // path-simulated inner sample would exceed kMaxPathSteps (the call then fails with
 // NMLMC_ERR_LIMIT); k_outer clears it on a level's first batch.

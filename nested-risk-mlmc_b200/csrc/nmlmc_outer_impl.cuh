@@ -1998,7 +1998,6 @@ static cudaError_t run_batch(DevLevel<RT>& D, uint32_t nb, TraceRec* trace, cuda
 // per sample each way), no tickets and no barriers per tile.  Bound by the ALU pipe of the counter
 // generator (9 blocks per level-0 sample of 32): 12e6 samples at level 0 892 -> 855 us, 33,000 48 -> 36
 // us, 4e6 at level 1 (64 and 32) 613 -> 545 us against the launch sequence.
-constexpr uint32_t kFixedChunks = 4;
 
 template <class RT, int KIND, int PREC>
 __global__ void __launch_bounds__(kTile, PREC == PREC_FP32 ? 4 : 2) k_fixed(DevLevel<RT> D, TraceRec* trace) {
@@ -2102,8 +2101,7 @@ cudaError_t sample_level_t(const OuterLevel<RT>& L, OuterBuffers& B, TraceRec* t
         }
     }
     if constexpr (KIND == KIND_REF_MODEL || KIND == KIND_SHIFT_MODEL) {
-        const uint64_t maxc = (L.fine_only || L.cf.max_count >= L.cc.max_count) ? L.cf.max_count : L.cc.max_count;
-        if (!L.adaptive_f && !L.adaptive_c && maxc / L.chunk <= kFixedChunks && !(L.N0 & (L.N0 - 1))) {
+        if (level_is_fixed(L, KIND)) {
             const uint64_t ctas = (L.M + kTile - 1) / kTile;
             const int grid = fixed_grid<RT, KIND, PREC>((int)(ctas < (uint64_t)B.grid ? ctas : (uint64_t)B.grid));
             if (B.prof_mark) B.prof_mark(B.prof_user, 0, stream);

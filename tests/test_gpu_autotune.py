@@ -132,3 +132,32 @@ def test_invalid_and_unpinned_configurations(nm):
     f64.set_model(nm.MODEL_SHIFT, 0.0, 1.0)
     with pytest.raises(nm.NmlmcError):
         f64.autotune_level(2, 1 << 15)           # tuning is for the FP32 path
+
+
+def _launches(nm, f):
+    n0 = nm.kernel_launches()
+    f()
+    return nm.kernel_launches() - n0
+
+
+def test_a_level_without_variants_is_not_probed(nm):
+    """A model level at small fixed counts runs as one kernel that no variant changes: its first call
+    launches that kernel alone; the level counts as tuned."""
+    s = _model(nm)
+    assert _launches(nm, lambda: s.sample(0, 1 << 19)) == 1
+    assert s.phase_config(0) == dict(variant=1, chunk=32, state=nm.PHASE_TUNED, probe_ms=0.0)
+    want = _model(nm, autotune=0)
+    want.sample(0, 1 << 19)
+    _same(s.sample(0, 5000), want.sample(0, 5000))
+
+
+def test_probes_run_the_kernels_the_variants_change(nm):
+    """With a batch of 1024 outer samples a probe is one batch, and a small one: it runs as the launch
+    sequence all the same, once per candidate and warm-up.  The pipelined variant exists for alias
+    columns only."""
+    for imp, variants in ((True, 4), (False, 3)):
+        s = nm.Sampler(N0=64, beta=2, adaptive_r=0.0, precision=nm.PREC_FP32, streams=nm.STREAMS_OUTER, seed=5, batch=1024)
+        s.set_portfolio(O.synthetic_portfolio(6, 400, 9, prob="w" if imp else "uniform"), max_loss=1.0,
+                        subsample=nm.SUB_RANDOM if imp else nm.SUB_UNIFORM)
+        # probe size, then every variant and two other chunk lengths; two runs of k_outer and k_phase each
+        assert _launches(nm, lambda: s.autotune_level(1, 1 << 16)) == (1 + variants + 2) * 2 * 2
