@@ -179,7 +179,7 @@ typedef struct nmlmc_level_result {
     double seconds;            /* device time of the level: CUDA events around a single call;
                                   inside a round's graph, %globaltimer stamps at its begin and end
                                   (levels that ran side by side: the round's time in proportion
-                                  to their inner samples) */
+                                  to theirs) */
 } nmlmc_level_result;
 
 typedef struct nmlmc_portfolio {

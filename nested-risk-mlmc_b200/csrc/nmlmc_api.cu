@@ -1169,18 +1169,18 @@ int sample_outer_levels(nmlmc_ctx* c, uint32_t n, const uint32_t* ells, const ui
     c->graph_launches++;
     NM_CUDA(cudaStreamSynchronize(c->stream), "sync");
     // device time of every level: between its own stamps, or, side by side, the round's time shared in
-    // proportion to the inner samples, so that the levels' times add up to it
-    double inner = 0;
+    // proportion to those, so that the levels' times add up to it
+    double own = 0;
     uint64_t t0 = ~0ull, t1 = 0;
     for (uint32_t i = 0; i < n; i++) {
         if (!Ms[i]) continue;
-        inner += c->h_lev[16 * (size_t)i + 9];
+        own += (double)(h_st[2 * i + 1] - h_st[2 * i]);
         t0 = std::min(t0, h_st[2 * i]);
         t1 = std::max(t1, h_st[2 * i + 1]);
     }
+    const double share = side && own > 0 ? (double)(t1 - t0) / own : 1.0;
     for (uint32_t i = 0; i < n; i++) {
-        const double sec = 1e-9 * (side ? (inner > 0 ? (double)(t1 - t0) * c->h_lev[16 * (size_t)i + 9] / inner : 0.0)
-                                        : (double)(h_st[2 * i + 1] - h_st[2 * i]));
+        const double sec = 1e-9 * share * (double)(h_st[2 * i + 1] - h_st[2 * i]);
         fill_outer_result(c, c->h_lev + 16 * (size_t)i, Ms[i], sec, &outs[i]);
         c->next_outer[ells[i]] += Mtot[i];
     }

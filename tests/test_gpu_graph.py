@@ -52,3 +52,15 @@ def test_levels_submission_portfolio(nm):
     for x, y in zip(ra, rb):
         np.testing.assert_array_equal(x["fsums"], y["fsums"])
         np.testing.assert_array_equal(x["diffsums"], y["diffsums"])
+
+
+def test_level_times_of_a_round_side_by_side_are_measured(nm):
+    """Levels that run side by side share the round's time by their own device times: a deep level of
+    few inner samples, a chain of pilots, takes microseconds whatever its neighbour draws."""
+    _, s = _pair(nm, nm.PREC_FP32)
+    s.sample_levels([0, 7], [60_000, 3])
+    r0, r7 = s.sample_levels([0, 7], [60_000, 3])
+    assert r0["stats"][0] > 50 * r7["stats"][0]
+    assert r7["seconds"] > 2e-6 and r0["seconds"] > 2e-6
+    one = s.sample_levels([0, 7], [0, 3])                 # a level without outer samples takes none
+    assert one[0]["seconds"] == 0 and one[1]["seconds"] > 2e-6
