@@ -92,7 +92,7 @@ RT h_norm_cdf_inv(RT p) {
 constexpr uint32_t kSideLevels = 16;
 constexpr uint32_t kCounterSlots = 256;      // counters of one level
 
-// Levels one nmlmc_sample_levels submission may hold (accumulator slots of the OUTER buffers).
+// Levels one nmlmc_sample_levels submission may hold (result slots in the pinned buffer).
 constexpr uint32_t kMaxSubmit = 64;
 
 // Portfolio as handed to the sampler, kept on the host in double (the values are the real_t
@@ -671,7 +671,7 @@ int alloc_outer(nmlmc_ctx* c, uint64_t want) {
               ctx_malloc(c, &B.class_items, cap * sizeof(uint32_t)) == cudaSuccess &&
               ctx_malloc(c, &B.counters, kCounterSlots * sizeof(uint32_t)) == cudaSuccess &&
               ctx_malloc(c, &B.block_sums, (size_t)B.grid * 16 * sizeof(double)) == cudaSuccess &&
-              ctx_malloc(c, &B.level_acc, kMaxSubmit * 16 * sizeof(double)) == cudaSuccess;
+              ctx_malloc(c, &B.level_acc, 16 * sizeof(double)) == cudaSuccess;
     c->ob_alloc = true;                   // free_outer releases a partial set too
     if (!ok) {
         free_outer(c);
@@ -784,13 +784,10 @@ void fill_outer_result(const nmlmc_ctx* c, const double* a, uint64_t M, double s
     out->seconds = seconds;
 }
 
-// Default phase configuration: up to 255 registers for the models (their inner loop is ALU-bound
-// and gains nothing from more warps), four CTAs per SM for the FP32 portfolio (its option-table
-// gathers need the warps to hide L2 latency), chunks of min(N0, 32) inner samples.
-// Defaults of the FP32 path, measured per level of the benchmark runs: the portfolio kernel at
-// 64 registers (variant 2: four CTAs per SM keep more table gathers in flight), the model kinds at
-// 80 (variant 1: fastest or within 0.3 % of it at every level of the adaptive model problem, 3-7 %
-// ahead of variant 0).
+// Default phase configuration: chunks of min(N0, 32) inner samples, and on the FP32 path, measured
+// per level of the benchmark runs, the portfolio kernel at 64 registers (variant 2: four CTAs per SM
+// keep more table gathers in flight) and the model kinds at 80 (variant 1: fastest or within 0.3 % of
+// it at every level of the adaptive model problem, 3-7 % ahead of variant 0).
 PhaseChoice default_phase(const nmlmc_ctx* c) {
     PhaseChoice p;
     p.variant = c->cfg.precision != NMLMC_PREC_FP32 ? 0u : c->kind == KIND_PORTFOLIO ? 2u : 1u;
@@ -1049,8 +1046,8 @@ bool ensure_side(nmlmc_ctx* c, uint32_t n) {
 }
 
 // All levels of one MLMC round in one submission: the level sequences are captured from the
-// stream into a CUDA graph (no host round trip inside: device counters size every phase), each
-// level accumulating into its own slot; one copy of the slots and one synchronisation per round.
+// stream into a CUDA graph (no host round trip inside: device counters size every phase), the last
+// kernel of each level storing its sums in its slot of pinned memory; one synchronisation per round.
 // The executable graph is kept and updated in place (cudaGraphExecUpdate) while later rounds
 // have the same topology (the same levels and batch counts), re-instantiated otherwise.
 template <class RT>
@@ -1410,9 +1407,9 @@ int nmlmc_set_portfolio_methods(nmlmc_ctx* c, const nmlmc_portfolio* p, const nm
 namespace {
 
 // Device memory of nmlmc_path_adjoint calls: one block per context, kept between calls up to
-// kAdjKeepBytes (allocating and freeing two dozen buffers took 2 ms of each call) and released with
-// the context, or when another allocation of the context needs the room (ctx_malloc).  The derivatives
-// kept between the two passes take at most kAdjStoreBytes of it.
+// kAdjKeepBytes, so that a repeated call neither allocates nor frees, and released with the context,
+// or when another allocation of the context needs the room (ctx_malloc).  The derivatives kept
+// between the two passes take at most kAdjStoreBytes of it.
 constexpr size_t kAdjKeepBytes = 5ull << 28, kAdjStoreBytes = 1ull << 30;
 
 int adj_reserve(nmlmc_ctx* c, size_t bytes) {

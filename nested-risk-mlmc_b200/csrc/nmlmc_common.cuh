@@ -45,10 +45,10 @@ constexpr uint64_t kMaxPathSteps = 1ull << 24;
 
 // Black-Scholes constants of one option in the reference's real_t evaluation order (REF32 / FP64
 // tables; k_ref_records): what calc_bs, the discount and the delta control variate of an inner
-// sample recompute from the option alone, evaluated once with the same device functions, so an
-// inner sample's value is unchanged.  It is left with one log, two erfc and the divisions by
-// R-dependent values: three erfc, two logs, two exponentials and four square roots were evaluated
-// before, from ten scattered table reads (now one record).
+// sample need of the option alone, evaluated once with the device functions that the formulas name,
+// so an inner sample's value is that of evaluating them in place.  An inner sample reads one record
+// and is left with one log, two erfc and the divisions by R-dependent values (in place: three erfc,
+// two logs, two exponentials and four square roots from ten scattered reads).
 template <class RT>
 struct __align__(16) RefOption {
     RT strike, v2, v3;    // v2 = (r + sigma^2 / 2) (T - tau), v3 = sigma sqrt(T - tau)
@@ -155,11 +155,6 @@ __device__ __forceinline__ float xpow(float a, float b) { return __double2float_
 __device__ __forceinline__ double xpow(double a, double b) { return pow(a, b); }
 
 __device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-    for (int m = 16; m > 0; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
-    return v;
-}
-__device__ __forceinline__ uint64_t warp_sum_u64(uint64_t v) {
 #pragma unroll
     for (int m = 16; m > 0; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
     return v;

@@ -695,8 +695,8 @@ __device__ __forceinline__ void core_run(const CoreLaunch<RT>& L, uint32_t core,
     }
 }
 
-// Threads per CTA: two virtual cores, so that 2048 cores spread evenly over the SMs (CTAs of eight
-// left 108 SMs with 16 warps and 40 with 8).
+// Threads per CTA: two virtual cores, so that 2048 cores spread evenly over the SMs, 13 or 14 warps
+// on each (CTAs of eight cores put 16 on 108 SMs and 8 on the other 40).
 constexpr int kCoreThreads = 64, kCoreWarps = kCoreThreads / 32;
 // CTAs whose partial sums are added together before the groups are.
 constexpr uint32_t kCoreGroup = 32;
@@ -740,7 +740,7 @@ __device__ __forceinline__ bool core_last(uint32_t* count, uint32_t n) {
 
 // The level's results from the cores' partials, inside the level kernel: the last CTA of a group of
 // kCoreGroup adds the group's, the last group's adds the groups' and stores the 16 words in the
-// host's pinned memory (a one-CTA kernel over all cores took 18 us, two copies back followed).
+// host's pinned memory: no second kernel (18 us for one CTA over 2048 cores) and no copies back.
 __device__ __forceinline__ void core_finish(uint64_t* part, uint32_t* counts, uint64_t* out) {
     const uint32_t groups = (gridDim.x + kCoreGroup - 1) / kCoreGroup, g = blockIdx.x / kCoreGroup;
     const uint32_t first = g * kCoreGroup, n = gridDim.x - first < kCoreGroup ? gridDim.x - first : kCoreGroup;

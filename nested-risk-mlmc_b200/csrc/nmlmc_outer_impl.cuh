@@ -540,12 +540,6 @@ __device__ __forceinline__ void* user_ws(const OuterBuffers& B, uint32_t item) {
     return B.ws_bytes ? static_cast<unsigned char*>(B.user_ws) + (size_t)item * B.ws_bytes : nullptr;
 }
 
-// ---- one chunk: inner samples [s0, s0 + C) of phase `tag` of outer sample `item` ----------
-// The chunk's share of sample_inner's sums (nested_sampler.hpp:131-161; model::sampler::
-// sample_inner, model_sampler.cpp:66-79, or the portfolio's inner value above).
-// CT = C (inner samples per chunk) is a compile-time constant so the independent Threefry blocks of
-// a chunk can be interleaved (two at a time) for instruction-level parallelism; CT = 0 takes the
-// run-time length Cr (chunks that are no power of two, multiples of 4).
 // ---- path-simulated portfolio, FP32 -------------------------------------------------------
 // The Unbiased level of the inner sample with path namespace ns (sample_inner_unbiased,
 // portfolio_sampler.cpp:521-537), the level of the double-precision formula, and its steps.
@@ -785,6 +779,12 @@ __device__ __forceinline__ void pf_paths_sorted(const DevLevel<float>& D, const 
     }
 }
 
+// ---- one chunk: inner samples [s0, s0 + C) of phase `tag` of outer sample `item` ----------
+// The chunk's share of sample_inner's sums (nested_sampler.hpp:131-161; model::sampler::
+// sample_inner, model_sampler.cpp:66-79, or the portfolio's inner value above).
+// CT = C (inner samples per chunk) is a compile-time constant so the independent Threefry blocks of
+// a chunk can be interleaved (two at a time) for instruction-level parallelism; CT = 0 takes the
+// run-time length Cr (chunks that are no power of two, multiples of 4).
 template <class RT, int KIND, int PREC, uint32_t CT, bool S2, class S, int PM>
 __device__ __forceinline__ void eval_chunk_c(const DevLevel<RT>& D, uint32_t item, uint32_t tag,
                                              uint64_t s0, uint64_t count, uint32_t Cr, float shift, const float2* srow,
@@ -1413,10 +1413,6 @@ __global__ void __launch_bounds__(kTile, MINB) k_phase(DevLevel<RT> D, SegSet SS
 }
 
 // ---- outer draws ---------------------------------------------------------------------------
-// sample_outer of the model (Y = randn_sync, model_sampler.cpp:57-59) or of the portfolio (the
-// stocks at tau and the delta-CV constant, portfolio_sampler.cpp:293-311, 606-614) per outer
-// sample, from the OUTER layout's phase-0 draws.  Also clears what the batch's later kernels count
-// in, and (first batch of a level) their partial sums.
 // GBM of stock s at tau and its row entry (R, ln R) on the FP32 path, R alone otherwise.
 template <class RT, int PREC>
 __device__ __forceinline__ RT stock_at_tau(const OptionTable<RT>& ot, uint32_t s, RT W, RT* Rrow) {
@@ -1434,6 +1430,10 @@ __device__ __forceinline__ RT stock_at_tau(const OptionTable<RT>& ot, uint32_t s
     return R;
 }
 
+// sample_outer of the model (Y = randn_sync, model_sampler.cpp:57-59) or of the portfolio (the
+// stocks at tau and the delta-CV constant, portfolio_sampler.cpp:293-311, 606-614) per outer
+// sample, from the OUTER layout's phase-0 draws.  Also clears what the batch's later kernels count
+// in, and (first batch of a level) their partial sums.
 template <class RT, int KIND, int PREC, class S = NoSampler>
 __global__ void __launch_bounds__(kTile) k_outer(DevLevel<RT> D, uint32_t nb, int first) {
     const OuterLevel<RT>& L = D.L;

@@ -31,8 +31,8 @@ __device__ __forceinline__ RT opt_derv_stock(const OptionTable<RT>& ot, uint32_t
 // simulate_stock_dt<with_coarse> (gbm_approx.hpp:18-57) on the three paths S[0..3) of
 // sample_inner_approx, plus (with_coarse) the coupled coarse paths S[3..6) stepping every
 // coarse_step fine steps on the summed increments.  States in double, increments in real_t.  Steps
-// are counted in 32 bits (at most kMaxPathSteps): a 64-bit remainder per step cost as much as the
-// rest of the step.
+// are counted in 32 bits (at most kMaxPathSteps) and the coarse ones by a counter: a 64-bit remainder
+// per step would cost as much as the rest of the step.
 template <class RT, class NZ>
 __device__ void stock_dt(NZ& nz, double* S, uint32_t N, RT mu, RT sigma, RT t, bool milstein,
                          bool with_coarse, uint32_t coarse_step) {
