@@ -1798,8 +1798,6 @@ __global__ void __launch_bounds__(kSmallThreads) k_small(DevLevel<RT> D, uint32_
     level_finish<kSmallThreads>(D.B, gridDim.x);
 }
 
-// Persistent grid of the phase kernel: the CTAs that are resident at once (occupancy x SMs),
-// at most the grid the partial-sum buffer was sized for.
 // Dynamic shared memory of a phase-kernel instantiation: the staged R_tau rows of the FP32
 // portfolio path (set as the kernel's maximum once, before the occupancy query and the first
 // launch).
@@ -1808,27 +1806,30 @@ constexpr size_t phase_dyn_smem() {
     return PREC != PREC_FP32 ? 0 : KIND == KIND_PORTFOLIO ? kRowSmemBytes : KIND == KIND_PF_PATHS ? kPathSortSmemBytes : 0;
 }
 
+// Persistent grid of the phase kernel: the CTAs that are resident at once (occupancy, at most
+// `ctas` per SM, x SMs), at most the grid the partial-sum buffer was sized for.
 template <class RT, int KIND, int PREC, int MINB, class S, int PM>
-static int phase_grid(int cap) {
-    static int g = 0;
-    if (g == 0) {
-        int dev = 0, sms = 148, per_sm = 0;
+static int phase_grid(int cap, int ctas) {
+    static int sms = 148, per_sm = 0;
+    if (per_sm == 0) {
+        int dev = 0, n = 0;
         constexpr size_t dyn = phase_dyn_smem<KIND, PREC>();
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         if (dyn) cudaFuncSetAttribute(k_phase<RT, KIND, PREC, MINB, S, PM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_phase<RT, KIND, PREC, MINB, S, PM>, kTile, dyn) != cudaSuccess ||
-            per_sm < 1)
-            per_sm = 1;
-        g = per_sm * sms;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_phase<RT, KIND, PREC, MINB, S, PM>, kTile, dyn) != cudaSuccess ||
+            n < 1)
+            n = 1;
+        per_sm = n;
     }
+    const int g = (per_sm < ctas ? per_sm : ctas) * sms;
     return g < cap ? g : cap;
 }
 
 template <class RT, int KIND, int PREC, int MINB, class S = NoSampler, int PM = PF_GENERIC>
-static void launch_phase_v(const DevLevel<RT>& D, const SegSet& SS, TraceRec* trace, cudaStream_t stream) {
+static void launch_phase_v(const DevLevel<RT>& D, const SegSet& SS, TraceRec* trace, cudaStream_t stream, int ctas = 8) {
     if (D.B.prof_mark) D.B.prof_mark(D.B.prof_user, 0, stream);
-    const int grid = phase_grid<RT, KIND, PREC, MINB, S, PM>(D.B.slots);
+    const int grid = phase_grid<RT, KIND, PREC, MINB, S, PM>(D.B.slots, ctas);
     // staged rows of the portfolio's own length: what they leave is L1 for the option table
     size_t dyn = phase_dyn_smem<KIND, PREC>();
     if (KIND == KIND_PORTFOLIO && PREC == PREC_FP32)
@@ -1855,7 +1856,9 @@ static void launch_variant(const DevLevel<RT>& D, const SegSet& SS, TraceRec* tr
 // CTAs without spills than at three with them; FP64 portfolio level 3, 20,000 outer samples: 783 us
 // at one, 632 at two.  The models in the parity precisions do so where the first pilots have a wave
 // of tiles for it (FP64 level 3: 2e6 outer samples 2.67 ms at one CTA, 1.90 at two; 20,000: 110 and 119
-// us).
+// us).  Below that the FP64 models run one CTA per SM, although two fit in the registers: a round of
+// few tiles would put two on one SM and leave another idle (reference model, level 12, 1000 outer
+// samples: rounds of one tile per CTA 29 us at two, 21 at one).
 // Chunks that are no power of two (N0 neither) run their one instantiation at the compiler's choice
 // of registers.
 template <class RT, int KIND, int PREC, class S = NoSampler>
@@ -1882,7 +1885,7 @@ static void launch_phase(const DevLevel<RT>& D, const SegSet& SS, TraceRec* trac
     } else {
         if constexpr (KIND != KIND_USER)
             if (D.L.M >= 32768) return launch_phase_v<RT, KIND, PREC, 2, S>(D, SS, trace, stream);
-        launch_phase_v<RT, KIND, PREC, 1, S>(D, SS, trace, stream);
+        launch_phase_v<RT, KIND, PREC, 1, S>(D, SS, trace, stream, PREC == PREC_FP64 && KIND != KIND_USER ? 1 : 8);
     }
 }
 
