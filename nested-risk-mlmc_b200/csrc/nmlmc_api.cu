@@ -859,11 +859,12 @@ constexpr uint64_t kProbeIndex = 1ull << 55;
 constexpr double kProbeMs = 20.0;       // device time of one tuning probe
 
 template <class RT>
-cudaError_t time_phase_config(nmlmc_ctx* c, uint32_t ell, uint64_t Mp, const PhaseChoice& pc, double& ms_out) {
+cudaError_t time_phase_config(nmlmc_ctx* c, uint32_t ell, uint64_t Mp, const PhaseChoice& pc, bool fixed, double& ms_out) {
     OuterLevel<RT> L = outer_level_params<RT>(c, ell, Mp, kProbeIndex);
     L.chunk = phase_chunk(L.N0, pc.chunk);
     L.variant = pc.variant;
-    L.no_small = true;                      // the launch sequence, whose kernels the candidates change
+    L.no_small = true;                      // the launch sequence, whose kernels the candidates change,
+    L.no_fixed = !fixed;                    // unless the call itself runs as k_fixed (chunk candidates)
     OuterBuffers B = c->ob;
     B.prof_mark = nullptr;
     B.stamps = nullptr;
@@ -888,12 +889,12 @@ cudaError_t time_phase_config(nmlmc_ctx* c, uint32_t ell, uint64_t Mp, const Pha
 // tuned call was small.  The work per outer sample ranges from the base count to the maximum count
 // of the level, too wide to predict from the configuration.
 template <class RT>
-cudaError_t probe_size(nmlmc_ctx* c, uint32_t ell, uint64_t& Mp) {
+cudaError_t probe_size(nmlmc_ctx* c, uint32_t ell, bool fixed, uint64_t& Mp) {
     const uint64_t lim = c->ob.cap;
     Mp = lim < 4096 ? lim : 4096;
     for (;;) {
         double ms = 0;
-        cudaError_t e = time_phase_config<RT>(c, ell, Mp, default_phase(c), ms);
+        cudaError_t e = time_phase_config<RT>(c, ell, Mp, default_phase(c), fixed, ms);
         if (e != cudaSuccess) return e;
         if (ms >= kProbeMs || Mp >= lim) return cudaSuccess;
         double grow = ms > 0 ? kProbeMs / ms : 8.0;
@@ -904,40 +905,41 @@ cudaError_t probe_size(nmlmc_ctx* c, uint32_t ell, uint64_t& Mp) {
     }
 }
 
-// Variants of the level's phase kernel at its default chunk length (launch_phase): one where a
-// single instantiation serves it, three with the pipelined loop's alias columns as a fourth.
+// Variants of the phase kernel at the default chunk length (launch_phase): one where a single
+// instantiation serves the level, three with the pipelined loop's alias columns as a fourth.
 template <class RT>
-uint32_t phase_variants(const nmlmc_ctx* c, uint32_t ell) {
-    OuterLevel<RT> L = outer_level_params<RT>(c, ell, 0, 0);
-    L.chunk = phase_chunk(L.N0, default_phase(c).chunk);
-    if ((L.chunk & (L.chunk - 1)) || level_is_fixed(L, c->kind)) return 1;
+uint32_t phase_variants(const nmlmc_ctx* c, const OuterLevel<RT>& L, bool fixed) {
+    if (fixed || (L.chunk & (L.chunk - 1))) return 1;
     if (c->kind != KIND_PORTFOLIO) return 3;
     return !L.ot.fast_s ? 1 : L.ot.fast_col ? 4 : 3;
 }
 
 template <class RT>
-int tune_level(nmlmc_ctx* c, uint32_t ell, bool chunks) {
+int tune_level(nmlmc_ctx* c, uint32_t ell, uint64_t M, bool chunks) {
     NvtxRange nv("nmlmc autotune level");
     PhaseChoice best = default_phase(c);
     best.state = 1;
-    const uint32_t n_var = phase_variants<RT>(c, ell);
+    OuterLevel<RT> L = outer_level_params<RT>(c, ell, M, 0);
+    L.chunk = phase_chunk(L.N0, best.chunk);
+    const bool fixed = level_is_fixed(L, c->kind, c->cfg.precision);
+    const uint32_t n_var = phase_variants<RT>(c, L, fixed);
     if (n_var == 1 && !chunks) {                  // nothing to choose from
         c->phase[ell] = best;
         return NMLMC_OK;
     }
     uint64_t Mp = 0;
-    NM_CUDA(probe_size<RT>(c, ell, Mp), "autotune probe size");
+    NM_CUDA(probe_size<RT>(c, ell, fixed, Mp), "autotune probe size");
     // the default stays unless another candidate is more than 3 % faster on the probe (near-ties
     // on a short probe are noise)
     double best_ms;
-    NM_CUDA(time_phase_config<RT>(c, ell, Mp, best, best_ms), "autotune probe");
+    NM_CUDA(time_phase_config<RT>(c, ell, Mp, best, fixed, best_ms), "autotune probe");
     const uint32_t v0 = best.variant;
     for (uint32_t v = 0; n_var > 1 && v < n_var; v++) {
         if (v == v0) continue;
         PhaseChoice pc = best;
         pc.variant = v;
         double ms;
-        NM_CUDA(time_phase_config<RT>(c, ell, Mp, pc, ms), "autotune probe");
+        NM_CUDA(time_phase_config<RT>(c, ell, Mp, pc, fixed, ms), "autotune probe");
         if (ms < 0.97 * best_ms) { best_ms = ms; best.variant = v; }
     }
     const uint32_t c0 = best.chunk;
@@ -946,7 +948,7 @@ int tune_level(nmlmc_ctx* c, uint32_t ell, bool chunks) {
         PhaseChoice pc = best;
         pc.chunk = ch;
         double ms;
-        NM_CUDA(time_phase_config<RT>(c, ell, Mp, pc, ms), "autotune probe");
+        NM_CUDA(time_phase_config<RT>(c, ell, Mp, pc, fixed, ms), "autotune probe");
         if (ms < 0.97 * best_ms) { best_ms = ms; best.chunk = ch; }
     }
     best.probe_ms = best_ms;
@@ -963,7 +965,7 @@ int ensure_tuned(nmlmc_ctx* c, uint32_t ell, uint64_t M) {
     const uint64_t Mp = M < c->ob.cap ? M : c->ob.cap;
     const CountParams cf = count_params(c->cfg, ell);
     if (Mp < 4096 || (double)Mp * (double)cf.base_count * (double)(ell + 1) < 8.0e6) return NMLMC_OK;
-    return tune_level<RT>(c, ell, c->autotune == 2);
+    return tune_level<RT>(c, ell, M, c->autotune == 2);
 }
 
 template <class RT>
@@ -1080,6 +1082,7 @@ int sample_outer_levels(nmlmc_ctx* c, uint32_t n, const uint32_t* ells, const ui
         key.push_back(ell);
         key.push_back((Ms[i] + ob.cap - 1) / ob.cap);
         if (Ms[i] && level_is_small(levels[i], c->kind, c->cfg.precision, ob)) small |= 1ull << i;
+        key.push_back(level_is_fixed(levels[i], c->kind, c->cfg.precision));
     }
     // Levels whose outer samples fit the batch buffers together run side by side, each a branch of
     // the graph: most of a round's levels are chains of small kernels that leave most of the chip idle
@@ -1785,7 +1788,7 @@ int nmlmc_autotune_level(nmlmc_ctx* c, uint32_t ell, uint64_t M) {
     int rc = ensure_portfolio(c);
     if (rc || (rc = alloc_outer(c, M))) return rc;
     if (c->kind == KIND_PORTFOLIO && c->pf.mixed()) return set_err(NMLMC_ERR_ARG);
-    return tune_level<float>(c, ell, true);
+    return tune_level<float>(c, ell, M, true);
 }
 
 int nmlmc_inject_alloc_failure(int32_t after) {

@@ -59,7 +59,8 @@ struct OuterLevel {
     bool fine_only, antithetic, adaptive_f, adaptive_c;
     uint32_t N0, chunk;     // chunk = inner samples per thread (phase_chunk: a power of two of them in each count)
     uint32_t variant;       // phase-kernel register/occupancy variant (FP32 path: 0, 1, 2)
-    bool no_small;          // run the launch sequence whatever the size (level_is_small)
+    bool no_small;          // not as one kernel for few outer samples, whatever their number (level_is_small)
+    bool no_fixed;          // nor as one for fixed counts (level_is_fixed)
     RT adaptive_r;
     CountParams cf, cc;
     ModelParams<RT> mp;
@@ -130,13 +131,23 @@ bool level_is_small(const OuterLevel<RT>& L, int kind, int prec, const OuterBuff
 }
 
 // Whether a level runs as k_fixed, a thread per outer sample: a model without pilots at up to
-// kFixedChunks chunks per outer sample, however many outer samples.
+// kFixedChunks chunks per outer sample.  One chunk is one thread's work in the launch sequence too;
+// more of them a thread takes one after another, so few outer samples leave the chip idle: at four
+// chunks k_fixed and the sequence take, in us, FP32 reference model 5000 outer samples 32 and 29, 8000
+// 32 and 29 to 34, 33,000 34 and 54; FP64 X = Y + Z 5000 42 and 29, 20,000 42 and 43, 300,000 202 and 212;
+// FP64 reference model 5000 71 and 41, 33,000 73 and 67, 120,000 199 and 173, 300,000 386 and 388.
 constexpr uint32_t kFixedChunks = 4;
 template <class RT>
-bool level_is_fixed(const OuterLevel<RT>& L, int kind) {
+bool level_is_fixed(const OuterLevel<RT>& L, int kind, int prec) {
     if (kind != KIND_REF_MODEL && kind != KIND_SHIFT_MODEL) return false;
+    if (L.no_fixed || L.adaptive_f || L.adaptive_c || (L.N0 & (L.N0 - 1))) return false;
     const uint64_t maxc = (L.fine_only || L.cf.max_count >= L.cc.max_count) ? L.cf.max_count : L.cc.max_count;
-    return !L.adaptive_f && !L.adaptive_c && maxc / L.chunk <= kFixedChunks && !(L.N0 & (L.N0 - 1));
+    const uint64_t nch = maxc / L.chunk;
+    if (nch > kFixedChunks) return false;
+    const uint64_t serial = nch * (kind == KIND_REF_MODEL ? 2 : 1);       // chunks of normals per thread
+    if (nch <= 1) return true;
+    if (prec == PREC_FP32) return serial <= 4 || L.M >= 8192;
+    return L.M >= (serial <= 4 ? 16384u : 262144u);
 }
 
 // Device counter slot (OuterBuffers::counters) that the batched kernels set when a

@@ -2107,7 +2107,7 @@ cudaError_t sample_level_t(const OuterLevel<RT>& L, OuterBuffers& B, TraceRec* t
         }
     }
     if constexpr (KIND == KIND_REF_MODEL || KIND == KIND_SHIFT_MODEL) {
-        if (level_is_fixed(L, KIND)) {
+        if (level_is_fixed(L, KIND, PREC)) {
             const uint64_t ctas = (L.M + kTile - 1) / kTile;
             const int grid = fixed_grid<RT, KIND, PREC>((int)(ctas < (uint64_t)B.grid ? ctas : (uint64_t)B.grid));
             if (B.prof_mark) B.prof_mark(B.prof_user, 0, stream);

@@ -70,3 +70,17 @@ def test_counts_of_three_chunks_take_the_sequence(nm, prec, r, ell, M, pieces):
         assert nm.kernel_launches() - n0 > 1
         assert got.tobytes() == big[at:at + m].tobytes()
         at += m
+
+
+# a model's fixed counts of four chunks: one kernel where the outer samples fill the chip, the sequence
+# below, the same records
+@pytest.mark.parametrize("kind,prec,M,piece", [("ref", "FP32", 9_000, 2_000), ("ref", "FP64", 270_000, 5_000),
+                                               ("shift", "REF32", 17_000, 3_000), ("shift", "FP32", 9_000, 5_000)])
+def test_fixed_counts_take_the_kernel_that_fills_the_chip(nm, kind, prec, M, piece):
+    n0 = nm.kernel_launches()
+    big = _sampler(nm, kind, prec, 32, 4, 0.0).sample(1, M, trace=True)["trace"]
+    assert nm.kernel_launches() - n0 == 1
+    n0 = nm.kernel_launches()
+    got = _sampler(nm, kind, prec, 32, 4, 0.0).sample(1, piece, trace=True)["trace"]
+    assert nm.kernel_launches() - n0 == (1 if (kind, prec) == ("shift", "FP32") else 2)
+    assert got.tobytes() == big[:piece].tobytes()
