@@ -1856,9 +1856,10 @@ static void launch_variant(const DevLevel<RT>& D, const SegSet& SS, TraceRec* tr
 // CTAs without spills than at three with them; FP64 portfolio level 3, 20,000 outer samples: 783 us
 // at one, 632 at two.  The models in the parity precisions do so where the first pilots have a wave
 // of tiles for it (FP64 level 3: 2e6 outer samples 2.67 ms at one CTA, 1.90 at two; 20,000: 110 and 119
-// us).  Below that the FP64 models run one CTA per SM, although two fit in the registers: a round of
-// few tiles would put two on one SM and leave another idle (reference model, level 12, 1000 outer
-// samples: rounds of one tile per CTA 29 us at two, 21 at one).
+// us).  Pilots of fewer than 4096 outer samples run one CTA per SM in the FP64 models, although two fit
+// in the registers: a round of few tiles would put two on one SM and leave another idle.  X = Y + Z,
+// beta 4, at one and two: level 7, 1000 samples 942 and 1025 us, 3000 1124 and 1391, 8000 1666 and 1716; level
+// 6, 3000 423 and 416, 8000 719 and 644; reference model, level 7, 3000 at fixed counts 20.6 and 15.1 ms.
 // Chunks that are no power of two (N0 neither) run their one instantiation at the compiler's choice
 // of registers.
 template <class RT, int KIND, int PREC, class S = NoSampler>
@@ -1885,7 +1886,8 @@ static void launch_phase(const DevLevel<RT>& D, const SegSet& SS, TraceRec* trac
     } else {
         if constexpr (KIND != KIND_USER)
             if (D.L.M >= 32768) return launch_phase_v<RT, KIND, PREC, 2, S>(D, SS, trace, stream);
-        launch_phase_v<RT, KIND, PREC, 1, S>(D, SS, trace, stream, PREC == PREC_FP64 && KIND != KIND_USER ? 1 : 8);
+        const bool few = PREC == PREC_FP64 && KIND != KIND_USER && (D.L.adaptive_f || D.L.adaptive_c) && D.L.M < 4096;
+        launch_phase_v<RT, KIND, PREC, 1, S>(D, SS, trace, stream, few ? 1 : 8);
     }
 }
 
