@@ -1344,10 +1344,6 @@ __global__ void __launch_bounds__(kTile, MINB) k_phase(DevLevel<RT> D, SegSet SS
                 gacc.zero();
                 float tind = 0.f;
                 for (uint32_t tl = 0; tl < tiles_per_item; tl++) {
-                    // the next item is claimed no earlier than the last tile: a CTA that held two long
-                    // items would leave the second waiting while others run dry (reference model to 16,384
-                    // chunks, 3000 outer samples: 950 to 1390 us from call to call, 1065 so)
-                    if (t == 0 && tl + 1 == tiles_per_item) next = atomicAdd(queue, 1u);
                     const uint32_t j = tl * kTile + t;
                     Acc<PREC> a1, a2;
                     a1.zero();
@@ -1366,6 +1362,11 @@ __global__ void __launch_bounds__(kTile, MINB) k_phase(DevLevel<RT> D, SegSet SS
                     if (lane == 0) { sm_a1[warp] = a1; sm_a2[warp] = a2; sm_ind[warp] = ind; }
                     __syncthreads();
                     if (t == 0) {
+                        // the next item is claimed when the last tile's values are there: a CTA that held
+                        // two long items would leave the second waiting while others run dry (reference
+                        // model to 16,384 chunks, 3000 outer samples: 950 to 1390 us from call to call,
+                        // 1065 so)
+                        if (tl + 1 == tiles_per_item) next = atomicAdd(queue, 1u);
                         if (!pilot && gs > 32 && gs < (uint32_t)kTile) {
                             const uint32_t gw = gs / 32;
                             for (uint32_t gq = 0; gq < (uint32_t)kWarps / gw; gq++) {
